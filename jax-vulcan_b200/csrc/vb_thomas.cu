@@ -6,55 +6,19 @@
 //     Inv_j = A'_j^{-1}                                            (solver.py:46,48)
 // Each A'_j is inverted in place by Gauss-Jordan elimination with threshold
 // partial pivoting (pivot_key32) on a register-resident tile (implicit
-// pivoting: no row exchanges),
-// one serial chain of ni pivot steps per layer with one block barrier each.
+// pivoting: no row exchanges), one serial chain of ni pivot steps per layer,
+// in panels (vb_gj_panel.cuh: the kernels that run; variants of the
+// synchronisation below).
 // The forward sweep of the first right-hand side rides along
 // (solver.py:73-88). The stored inverses turn every later solve into
 // matrix-vector products (solver.py:91-111).
 #include <cuda_runtime.h>
 
 #include "vb_common.cuh"
+#include "vb_gj_panel.cuh"
 #include "vb_launch.cuh"
 
 namespace vb {
-
-// High word of |v| (sign cleared): orders |v| up to ties of the low word.
-__device__ __forceinline__ unsigned hi_key(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
-__device__ __forceinline__ unsigned hi_key(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-
-// Pivot choice of every factor kernel. The key of a candidate row is the top
-// 24 bits of |v| (the sign-cleared high word shifted right by 7: the exponent
-// and the leading 13 mantissa bits in FP64, 16 in FP32) above 255 - row, so
-// one 32-bit max reduction over the warp names the pivot row: the largest
-// magnitude to within a relative 2^-13 (FP64) or 2^-16 (FP32), the lowest row
-// among those (threshold partial pivoting with threshold 1 - 2^-13; strict
-// partial pivoting takes the exact maximum, at the price of a second
-// reduction, ballots and shuffles on the pivot chain). A NaN counts as
-// magnitude 0. Rows that may not pivot (pivoted, padding) take key 0, below
-// every candidate (row <= 127, so a candidate's low byte is >= 128).
-template <typename R>
-__device__ __forceinline__ unsigned pivot_key32(R v, int row) {
-  const unsigned mag = isnan(v) ? 0u : (hi_key(v) >> 7);
-  return (mag << 8) | (unsigned)(255 - row);
-}
-__device__ __forceinline__ int pivot_row(unsigned kmax) { return 255 - (int)(kmax & 255u); }
-
-// Correctly rounded reciprocal (the value of 1 / x).
-__device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
-
-// Power of two s with s * m in [1, 2) for a finite m > 0 (1 otherwise).
-__device__ __forceinline__ double pow2_scale(double m) {
-  if (!(m > 0.0) || !isfinite(m)) return 1.0;
-  int e;
-  frexp(m, &e);               // m = f 2^e, f in [0.5, 1)
-  return ldexp(1.0, 1 - e);   // s m = 2 f in [1, 2)
-}
-
-// Two values of the factor's element type handed over in one shared-memory access.
-template <typename R> struct Pair;
-template <> struct Pair<double> { using T = double2; };
-template <> struct Pair<float> { using T = float2; };
 
 // ---------------------------------------------------------------- Gauss-Jordan factor
 // Shared-memory plan of gj_factor_atmosphere (carved in this order, each
@@ -65,70 +29,30 @@ struct GJK {
   static constexpr int NPC = CPW * NW;          // column capacity (warp w holds columns w*CPW + c)
   static constexpr int CPWP = (CPW + 1) & ~1;   // stride of a warp's pivot-row slot (pairs)
   __host__ __device__ static size_t al(size_t x) { return (x + 15) & ~(size_t)15; }
-  static size_t smem_bytes(int n, int ld, bool dpf, int li = 0, bool pipe = false) {
+  static size_t smem_bytes(int n, int ld, bool dpf, int li = 0) {
     const size_t blk = (size_t)n * ld, iblk = (size_t)n * (li ? li : ld);
     return al(iblk * sizeof(R))                       // Ib: the inverse of the layer (natural order, stride li)
            + (dpf ? al(blk * sizeof(double)) : 0)     // Db: the next diagonal block, prefetched
            + al(2 * NPC * sizeof(double))             // rsc: row scales of this and the previous layer (EQ)
-           + al(2 * NPR * sizeof(R))                  // colb: multipliers of the next step (2 parities)
            + al(NPR * sizeof(R))                      // rps: 1 / pivot of each row
            + al(4 * NPR * sizeof(double))             // rsb: the next layer's rhs and sub_d rows (2 parities)
-           + al((pipe ? 2 : 1) * NW * CPWP * sizeof(R))  // prs: pivot-row hand-over, a slot per warp (x2: parity)
+           + al(2 * NW * CPWP * sizeof(R))            // prs: pivot-row hand-over, a slot per warp and parity
            + al(2 * NPR * sizeof(double))             // vecs: right-hand side ping-pong
            + al(NPC * sizeof(int))                    // pivs: pivot row of each step
            + al(NPR * sizeof(int))                    // qs: step of each pivot row
-           + al(2 * sizeof(int))                      // pb: pivot row of the next step (2 parities)
            + 16                                       // mbarrier of the prefetch
-           + (pipe ? al(2 * CPW * NPR * sizeof(R))    // colr: multiplier ring, one slot per column of two panels
-                         + al(2 * CPW * sizeof(int))  // pring: pivot row of each ring slot
-                         + al((2 * CPW + 2) * 8)      // mbarriers: a slot's publication (2 CPW), a panel consumed (2)
-                         + 16                         // abort flag
-                   : 0);
+           + al(2 * CPW * NPR * sizeof(R))            // colr: multiplier ring, one slot per column of two panels
+           + al(2 * CPW * sizeof(int))                // pring: pivot row of each ring slot
+           + al((2 * CPW + 2) * 8)                    // mbarriers: a slot's publication (2 CPW), a panel consumed (2)
+           + 16;                                      // abort flag
   }
 };
 
-// Factor all layers of one atmosphere by Gauss-Jordan inversion of each
-// Schur-updated diagonal block. On entry Din[j] holds D_j (row stride ld); on
-// exit out[j] holds A'_j^{-1}; with rhs != nullptr the first sweep of the
-// right-hand side rhs[nz][ni] is done in place (solver.py:73-88).
-//
-// The reference inverts each block by lu_factor then lu_solve(LU, I)
-// (solver.py:46-48). Here the inverse comes from one serial chain of ni
-// Gauss-Jordan steps instead of three (factor, forward and back
-// substitution). Gauss-Jordan bounds the left residual |X B - I| of the
-// inverse X of the matrix B it eliminates on. With tr set the elimination
-// runs on the transposed block B = A'^T (partial pivoting within a row of
-// A'), so X = A'^{-1} has a small right residual |A' X - I| as the
-// reference's lu_solve(LU, I) columns do: what solves x = X b need (the Ros2
-// step; on the stiff config-0 draw eliminating on A' itself left the block
-// solve's normwise backward error at 4e-12 instead of 7e-15). Without tr it
-// runs on B = A' (partial pivoting within a column, as lu_factor), for
-// callers that solve with X^T (the transposed sweeps of the adjoint), which
-// need |X A' - I| small.
-//  * Tile in registers: lane l holds rows l + 32 r (r < RPL), warp w columns
-//    w*CPW + c (c < CPW) of B. No row exchanges: row p_k is the pivot row
-//    of step k. Pivot rows are not normalised during the elimination (row i
-//    carries the factor piv_i of its own step), so every element update is
-//    one FMA
-//        S[i][:] -= m_i S[p][:],   m_i = S[i][k] / piv_k  (m_p = 0),
-//    column k becomes -m_i (row p: 1), and each row is scaled by 1/piv_i at
-//    the end. The stored result T satisfies B^{-1}[q(i)][p_m] = T[i][m]
-//    (q(i): the step whose pivot row is i), applied (transposed back when
-//    tr) by the scatter into Ib.
-//  * One block barrier per step. During step k the owner warp of column
-//    k+1 updates that column first, takes its argmax (one redux.sync on
-//    the packed pivot_key32: threshold partial pivoting), inverts the
-//    pivot and publishes p_{k+1} with the scaled multipliers; the other warps
-//    update meanwhile. A warp takes its part of the pivot row from the owner
-//    lane through a per-warp shared slot (no block barrier).
-//  * Layer j's Schur update reads Inv_{j-1} from Ib (shared), D_j from Db
-//    (bulk-prefetched during layer j-1) when DPF, else from global memory.
-//  * EQ (transposed orientation): every row of A'_j is scaled by a power of
-//    two bringing its largest magnitude to [1, 2) before the elimination
-//    (row equilibration, exact); the stored inverse is X = (R A'_j)^{-1},
-//    the scales go to rs_out, and A'_j^{-1} = X diag(r).
-//  * li: row stride of Ib and of the stored inverses (ld when 0).
-template <int RPL, int CPW, int NW, bool DPF, typename R, bool EQ = false, bool PIPE = false>
+// The pipelined scalar factor: the elimination of panel_factor_atmosphere (its
+// tile, pivot rule, orientation, row scales and scatter) with the warps of a
+// block handing over every step through a ring of shared-memory slots instead
+// of a block barrier per panel; the same arithmetic in the same order.
+template <int RPL, int CPW, int NW, bool DPF, typename R, bool EQ = false>
 __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, const double* Din, R* out,
                                                      const double* __restrict__ supn,
                                                      const double* __restrict__ subn, double* rhs,
@@ -158,20 +82,18 @@ __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, cons
   R* Ib = reinterpret_cast<R*>(take((size_t)iblk * sizeof(R)));
   double* Db = DPF ? reinterpret_cast<double*>(take((size_t)blk * sizeof(double))) : nullptr;
   double* rsc = reinterpret_cast<double*>(take(2 * NPC * sizeof(double)));
-  R* colb = reinterpret_cast<R*>(take(2 * NPR * sizeof(R)));
   R* rps = reinterpret_cast<R*>(take(NPR * sizeof(R)));
   double* rsb = reinterpret_cast<double*>(take(4 * NPR * sizeof(double)));
-  R* prs = reinterpret_cast<R*>(take((PIPE ? 2 : 1) * NW * G::CPWP * sizeof(R)));
   double* vecs = reinterpret_cast<double*>(take(2 * NPR * sizeof(double)));
   int* pivs = reinterpret_cast<int*>(take(G::NPC * sizeof(int)));
   int* qs = reinterpret_cast<int*>(take(NPR * sizeof(int)));
-  int* pb = reinterpret_cast<int*>(take(2 * sizeof(int)));
   uint64_t* bar = reinterpret_cast<uint64_t*>(take(16));
-  R* colr = PIPE ? reinterpret_cast<R*>(take(2 * CPW * NPR * sizeof(R))) : nullptr;
-  int* pring = PIPE ? reinterpret_cast<int*>(take(2 * CPW * sizeof(int))) : nullptr;
-  uint64_t* fbar = PIPE ? reinterpret_cast<uint64_t*>(take((2 * CPW + 2) * 8)) : nullptr;
-  uint64_t* ebar = PIPE ? fbar + 2 * CPW : nullptr;
-  volatile int* abortp = PIPE ? reinterpret_cast<volatile int*>(take(16)) : nullptr;
+  R* prs = reinterpret_cast<R*>(take(2 * NW * CPWP * sizeof(R)));
+  R* colr = reinterpret_cast<R*>(take(2 * CPW * NPR * sizeof(R)));
+  int* pring = reinterpret_cast<int*>(take(2 * CPW * sizeof(int)));
+  uint64_t* fbar = reinterpret_cast<uint64_t*>(take((2 * CPW + 2) * 8));
+  uint64_t* ebar = fbar + 2 * CPW;
+  volatile int* abortp = reinterpret_cast<volatile int*>(take(16));
   const uint32_t dbytes = (uint32_t)(blk * sizeof(double));
   int st_local = 0;
   // pipeline signals: fbar[s] completes when the owner warp of ring slot s
@@ -188,7 +110,7 @@ __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, cons
   if (rhs)
     for (int i = threadIdx.x; i < n; i += blockDim.x) vecs[i] = rhs[i];
   if (DPF && threadIdx.x == 0) mbar_init(bar, 1);
-  if (PIPE && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     pipe_init();
     *abortp = 0;
   }
@@ -214,7 +136,8 @@ __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, cons
   };
   // multipliers t / piv of step kn into cb (0 on the pivot row), its pivot
   // row into *pbp, pivs[kn], qs[p1] and 1 / piv into rps[p1]
-  auto store_step_rp = [&](const R (&t)[RPL], int p1, R piv, R rp, int kn, R* cb, int* pbp, R (&mo)[RPL]) {
+  auto store_step = [&](const R (&t)[RPL], int p1, R piv, int kn, R* cb, int* pbp, R (&mo)[RPL]) {
+    const R rp = rcp_rn(piv);
     if (piv == R(0)) st_local |= VB_STATUS_ZERO_PIVOT;
 #pragma unroll
     for (int r = 0; r < RPL; ++r) {
@@ -227,19 +150,9 @@ __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, cons
     qs[p1] = kn;
     rps[p1] = rp;
   };
-  auto store_step = [&](const R (&t)[RPL], int p1, R piv, int kn, R* cb, int* pbp, R (&mo)[RPL]) {
-    store_step_rp(t, p1, piv, rcp_rn(piv), kn, cb, pbp, mo);
-  };
-  auto publish = [&](const R (&t)[RPL], unsigned used, int kn, R* cb, int* pbp, R (&mo)[RPL]) {
-    R piv;
-    const int p1 = pivot_of(t, used, piv);
-    store_step(t, p1, piv, kn, cb, pbp, mo);
-    return p1;
-  };
-
   R a[RPL][CPW];
 
-  // PIPE: the same elimination without a block barrier per step. The warp
+  // The elimination without a block barrier per step. The warp
   // that owns column k publishes step k (pivot row, multipliers) into ring
   // slot (panel parity, column in panel) and signals fbar of the slot; the
   // owner of a panel runs its steps back to back from registers while the
@@ -478,104 +391,20 @@ __device__ __forceinline__ void gj_factor_atmosphere(int nz, int n, int ld, cons
       bulk_g2s(Db, Din + (int64_t)(j + 1) * blk, dbytes, bar);
     }
     unsigned used = 0;   // rows lane + 32 r already pivoted
-    if constexpr (PIPE) {
-      eliminate_pipelined(used);
-      __syncthreads();
-      if (*abortp) {
-        // a wait gave up: drain the prefetch in flight, report, return
-        if (threadIdx.x == 0) {
-          if (DPF && j + 1 < nz) mbar_wait(bar, (uint32_t)((j + 1) & 1), WAIT_LIMIT);
-          atomicOr(status, VB_STATUS_WATCHDOG);
-        }
-        return;
-      }
-      if (threadIdx.x == 0) {   // every signal of this layer has completed: restart the phases
-#pragma unroll 1
-        for (int s2 = 0; s2 < 2 * CPW + 2; ++s2) mbar_inval(fbar + s2);
-        pipe_init();
-      }
-    } else {
-    // the warp that published a step applies it from its registers (the
-    // owner of column k published step k: no shared-memory round trip on
-    // the lookahead warp's path in five of six steps)
-    R mo[RPL];
-    int pk = 0;
-    if (warp == 0) {
-      R t[RPL];
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) t[r] = a[r][0];
-      pk = publish(t, 0u, 0, colb, pb, mo);
-    }
+    eliminate_pipelined(used);
     __syncthreads();
-    // ================================================================ elimination
-#pragma unroll 1
-    for (int w0 = 0; w0 < NW; ++w0) {
-      if (w0 * CPW >= n) break;
-#pragma unroll
-      for (int c = 0; c < CPW; ++c) {
-        const int k = w0 * CPW + c;
-        if (k < n) {
-          int p;
-          R m[RPL];
-          if (warp == w0) {
-            p = pk;
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) m[r] = mo[r];
-          } else {
-            p = pb[k & 1];
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) m[r] = colb[(k & 1) * NPR + lane + 32 * r];
-          }
-          const int ps = p >> 5, po = p & 31;
-#pragma unroll
-          for (int r = 0; r < RPL; ++r)
-            if (r == ps && lane == po) used |= 1u << r;
-          // this warp's part of the pivot row, from its owner lane (pair
-          // stores predicated on the slot: no selects)
-          R* ph = prs + warp * CPWP;
-#pragma unroll
-          for (int r = 0; r < RPL; ++r)
-            if (r == ps && lane == po) {
-#pragma unroll
-              for (int c2 = 0; c2 < CPWP; c2 += 2)
-                reinterpret_cast<R2*>(ph)[c2 / 2] = R2{a[r][c2], c2 + 1 < CPW ? a[r][c2 + 1] : R(0)};
-            }
-          __syncwarp();
-          R prow[CPWP];
-#pragma unroll
-          for (int c2 = 0; c2 < CPWP; c2 += 2) {
-            const R2 v = reinterpret_cast<const R2*>(ph)[c2 / 2];
-            prow[c2] = v.x;
-            prow[c2 + 1] = v.y;
-          }
-          const int cl = (c + 1) % CPW;                     // column k+1: slot and owner warp
-          const int wl = (c + 1 < CPW) ? w0 : w0 + 1;
-          if (k + 1 < n && warp == wl) {
-            R t[RPL], piv;
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) t[r] = fma(-m[r], prow[cl], a[r][cl]);
-            const int p1 = pivot_of(t, used, piv);
-            const R rp = rcp_rn(piv);   // in flight while the rest of step k is applied
-#pragma unroll
-            for (int r = 0; r < RPL; ++r)
-#pragma unroll
-              for (int c2 = 0; c2 < CPW; ++c2) a[r][c2] = fma(-m[r], prow[c2], a[r][c2]);
-            store_step_rp(t, p1, piv, rp, k + 1, colb + ((k + 1) & 1) * NPR, pb + ((k + 1) & 1), mo);
-            pk = p1;
-          } else {
-#pragma unroll
-            for (int r = 0; r < RPL; ++r)
-#pragma unroll
-              for (int c2 = 0; c2 < CPW; ++c2) a[r][c2] = fma(-m[r], prow[c2], a[r][c2]);
-          }
-          if (warp == w0) {
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) a[r][c] = (lane + 32 * r == p) ? R(1) : -m[r];
-          }
-          __syncthreads();
-        }
+    if (*abortp) {
+      // a wait gave up: drain the prefetch in flight, report, return
+      if (threadIdx.x == 0) {
+        if (DPF && j + 1 < nz) mbar_wait(bar, (uint32_t)((j + 1) & 1), WAIT_LIMIT);
+        atomicOr(status, VB_STATUS_WATCHDOG);
       }
+      return;
     }
+    if (threadIdx.x == 0) {   // every signal of this layer has completed: restart the phases
+#pragma unroll 1
+      for (int s2 = 0; s2 < 2 * CPW + 2; ++s2) mbar_inval(fbar + s2);
+      pipe_init();
     }
     // ---- scale rows by 1/piv, scatter B^{-1}[q(i)][p_m] = T[i][m] into Ib
     //      (A'^{-1}[p_m][q(i)] when tr; q(i) = qs[i], the step pivoting on row i)
@@ -1036,7 +865,23 @@ gj_pair_kernel(Batch B, double* __restrict__ ws, int32_t* __restrict__ status, i
 // out == nullptr: the inverses replace the blocks in the workspace (FP64
 // path); otherwise they go to out (layer-major, ni x ld per layer) and the
 // FP64 blocks stay. only != nullptr: atmospheres with only[b] == 0 are skipped.
-template <int RPL, int CPW, int NW, int MB, bool DPF, typename R, bool PIPE = false>
+// FP64, panels of 8 columns with DMMA trailing updates (one warp per panel).
+template <int NT, int MB, bool DPF>
+__global__ void __launch_bounds__(NT * 32, MB)
+dgj_factor_kernel(Batch B, double* __restrict__ ws, double* out, const int32_t* __restrict__ only,
+                  int32_t* __restrict__ status, int with_rhs, int tr, long long wlim) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const int b = blockIdx.x;
+  if (only && only[b] == 0) return;
+  Geo g = geo_of(B, b);
+  WsView w = ws_view(ws, g, B.ni, B.ld);
+  double* o = out ? out + g.z0 * B.ni * B.ld : w.inv;
+  dmma_factor_atmosphere<NT, DPF>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn, with_rhs ? w.rmod : nullptr, tr != 0,
+                                  status + b, smem_raw, wlim);
+}
+
+// FP32, scalar updates by panel; and either type through the pipelined ring.
+template <int RPL, int CPW, int NW, int MB, bool DPF, typename R, bool PIPE>
 __global__ void __launch_bounds__(NW * 32, MB)
 gj_factor_kernel(Batch B, double* __restrict__ ws, R* out, const int32_t* __restrict__ only,
                  int32_t* __restrict__ status, int with_rhs, int tr, long long wlim, long long plim) {
@@ -1046,15 +891,20 @@ gj_factor_kernel(Batch B, double* __restrict__ ws, R* out, const int32_t* __rest
   Geo g = geo_of(B, b);
   WsView w = ws_view(ws, g, B.ni, B.ld);
   R* o = out ? out + g.z0 * B.ni * B.ld : reinterpret_cast<R*>(w.inv);
-  gj_factor_atmosphere<RPL, CPW, NW, DPF, R, false, PIPE>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn,
-                                                          with_rhs ? w.rmod : nullptr, tr != 0, status + b, smem_raw,
-                                                          wlim, 0, nullptr, plim);
+  if constexpr (PIPE)
+    gj_factor_atmosphere<RPL, CPW, NW, DPF, R>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn,
+                                               with_rhs ? w.rmod : nullptr, tr != 0, status + b, smem_raw, wlim, 0,
+                                               nullptr, plim);
+  else
+    panel_factor_atmosphere<RPL, CPW, NW, DPF, R, false>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn,
+                                                         with_rhs ? w.rmod : nullptr, tr != 0, status + b, smem_raw,
+                                                         wlim, 0, nullptr);
 }
 
-// FP32 factor of the mixed-precision step by the scalar Gauss-Jordan kernel
+// FP32 factor of the mixed-precision step by the scalar Gauss-Jordan kernels
 // (row-equilibrated, transposed orientation): FP32 inverses and row scales
 // into the mixed region, the FP64 blocks stay in the workspace.
-template <int RPL, int CPW, int NW, int MB, bool DPF, bool PIPE = false>
+template <int RPL, int CPW, int NW, int MB, bool DPF, bool PIPE>
 __global__ void __launch_bounds__(NW * 32, MB)
 gj32_factor_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int32_t* __restrict__ status,
                    long long wlim, long long plim) {
@@ -1063,9 +913,12 @@ gj32_factor_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int
   Geo g = geo_of(B, b);
   WsView w = ws_view(ws, g, B.ni, B.ld);
   MxView m = mx_view(mxr, g.z0, g.nz, B.ni);
-  gj_factor_atmosphere<RPL, CPW, NW, DPF, float, true, PIPE>(g.nz, B.ni, B.ld, w.inv, m.X, w.supn, w.subn, nullptr,
-                                                             true, status + b, smem_raw, wlim, round4(B.ni), m.rs,
-                                                             plim);
+  if constexpr (PIPE)
+    gj_factor_atmosphere<RPL, CPW, NW, DPF, float, true>(g.nz, B.ni, B.ld, w.inv, m.X, w.supn, w.subn, nullptr, true,
+                                                         status + b, smem_raw, wlim, round4(B.ni), m.rs, plim);
+  else
+    panel_factor_atmosphere<RPL, CPW, NW, DPF, float, true>(g.nz, B.ni, B.ld, w.inv, m.X, w.supn, w.subn, nullptr,
+                                                            true, status + b, smem_raw, wlim, round4(B.ni), m.rs);
 }
 
 // ---------------------------------------------------------------- blocked Gauss-Jordan factor (tensor cores)
@@ -1123,14 +976,6 @@ struct BGJ {
            + 16;                                               // mbarrier of the prefetch
   }
 };
-
-// D += A B for one m8n8k4 FP64 tile (A: 8x4 row, B: 4x8 col; per lane a0 =
-// A[g][t], b0 = B[t][g], d = D[g][2t], D[g][2t+1]).
-__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
-}
 
 // D += A B for one m16n8k8 TF32 tile (FP32 accumulation; per lane a = A[g][t],
 // A[g+8][t], A[g][t+4], A[g+8][t+4]; b = B[t][g], B[t+4][g]; d = D[g][2t],
@@ -1775,7 +1620,8 @@ static bool one_cta_per_sm(const Batch& B) {
 template <int RPL, int CPW, int NW, int MB, bool DPF, typename R, bool PIPE>
 static cudaError_t launch_gj_t(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
                                R* out, const int32_t* only) {
-  size_t sm = GJK<RPL, CPW, NW, R>::smem_bytes(B.ni, B.ld, DPF, 0, PIPE);
+  size_t sm = PIPE ? GJK<RPL, CPW, NW, R>::smem_bytes(B.ni, B.ld, DPF)
+                   : PGJ<RPL, CPW, NW, R>::smem_bytes(B.ni, B.ld, DPF);
   cudaError_t e = cudaFuncSetAttribute(gj_factor_kernel<RPL, CPW, NW, MB, DPF, R, PIPE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -1785,9 +1631,9 @@ static cudaError_t launch_gj_t(const Batch& B, double* ws, int32_t* status, int 
   return cudaGetLastError();
 }
 
-// Factor kernel of the process: 0 = blocked Gauss-Jordan with the trailing
-// updates on the FP64 tensor cores, 1 = scalar Gauss-Jordan with one block
-// barrier per pivot step, 2 = scalar Gauss-Jordan pipelined per column panel
+// Factor kernel of the process: 0 = blocked Gauss-Jordan with the panel in
+// accumulator layout, 1 = Gauss-Jordan by panels (FP64: DMMA trailing updates,
+// FP32: scalar), 2 = scalar Gauss-Jordan pipelined per column panel
 // (no block barrier per step), 3 = scalar Gauss-Jordan with two atmospheres'
 // chains interleaved per CTA (FP64 factor of uniform batches of 65-72
 // species; the scalar kernel elsewhere). A network's tuning (factor_kernel
@@ -1834,7 +1680,8 @@ static cudaError_t launch_bgj32_t(const Batch& B, double* ws, void* mxr, int32_t
 
 template <int RPL, int CPW, int NW, int MB, bool DPF, bool PIPE>
 static cudaError_t launch_gj32_t(const Batch& B, double* ws, void* mxr, int32_t* status, cudaStream_t st) {
-  size_t sm = GJK<RPL, CPW, NW, float>::smem_bytes(B.ni, B.ld, DPF, round4(B.ni), PIPE);
+  size_t sm = PIPE ? GJK<RPL, CPW, NW, float>::smem_bytes(B.ni, B.ld, DPF, round4(B.ni))
+                   : PGJ<RPL, CPW, NW, float>::smem_bytes(B.ni, B.ld, DPF, round4(B.ni));
   cudaError_t e = cudaFuncSetAttribute(gj32_factor_kernel<RPL, CPW, NW, MB, DPF, PIPE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -1870,15 +1717,41 @@ cudaError_t launch_factor32(const Batch& B, double* ws, void* mxr, int32_t* stat
 
 
 
-// Tile shapes by block size: rows over 32 lanes x RPL, columns over NW warps
-// x CPW (the next diagonal block is prefetched into shared memory in every
-// shape whose two buffers fit). Up to 72 species: 12 warps of 6 columns, two
-// CTAs per SM when the batch has more atmospheres than SMs (register cap 85),
-// else one (no register cap). Measured on B200, ni=69, nz=120: 148
-// atmospheres 4.11 ms per factor (16 warps x 5: 4.77; 8 x 9: 5.30; 32 x 3:
-// 6.43), one atmosphere 4.84 ms per Ros2 step (16 x 5: 5.50; 8 x 9: 5.92),
-// 296 atmospheres 6.15 ms (two CTAs of 8 x 9: 6.29; 10 x 7: 6.15; 14 x 5:
-// 7.09; 16 x 5: 9.14).
+template <int NT, int MB, bool DPF>
+static cudaError_t launch_dgj_t(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
+                                double* out, const int32_t* only) {
+  size_t sm = DGJ<NT>::smem_bytes(B.ni, B.ld, DPF);
+  cudaError_t e = cudaFuncSetAttribute(dgj_factor_kernel<NT, MB, DPF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sm);
+  if (e != cudaSuccess) return e;
+  dgj_factor_kernel<NT, MB, DPF><<<B.count, NT * 32, sm, st>>>(B, ws, out, only, status, with_rhs, tr, g_wait_limit);
+  return cudaGetLastError();
+}
+
+// The FP64 Gauss-Jordan factor: one warp per panel of 8 columns, the smallest
+// instantiated count that holds ni. Up to 72 species two CTAs share an SM when
+// the batch has more atmospheres than SMs (registers capped for it), else one
+// (no cap); larger blocks leave shared memory for one.
+static cudaError_t launch_dgj(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
+                              double* out, const int32_t* only) {
+  if (B.ni <= 24) return launch_dgj_t<3, 4, true>(B, ws, status, with_rhs, tr, st, out, only);
+  if (B.ni <= 32) return launch_dgj_t<4, 4, true>(B, ws, status, with_rhs, tr, st, out, only);
+  if (B.ni <= 48) return launch_dgj_t<6, 2, true>(B, ws, status, with_rhs, tr, st, out, only);
+  if (B.ni <= 64) return launch_dgj_t<8, 2, true>(B, ws, status, with_rhs, tr, st, out, only);
+  if (B.ni <= 72) {
+    if (one_cta_per_sm(B)) return launch_dgj_t<9, 1, true>(B, ws, status, with_rhs, tr, st, out, only);
+    return launch_dgj_t<9, 2, true>(B, ws, status, with_rhs, tr, st, out, only);
+  }
+  if (B.ni <= 80) return launch_dgj_t<10, 1, true>(B, ws, status, with_rhs, tr, st, out, only);
+  if (B.ni <= 96) return launch_dgj_t<12, 1, true>(B, ws, status, with_rhs, tr, st, out, only);
+  return launch_dgj_t<16, 1, false>(B, ws, status, with_rhs, tr, st, out, only);
+}
+
+// Tile shapes of the scalar factors by block size: rows over 32 lanes x RPL,
+// columns over NW warps x CPW (the next diagonal block is prefetched into
+// shared memory in every shape whose two buffers fit). FP32 by panel, ms per
+// 40 layers at 148 atmospheres: ni=69: 12 warps of 6 columns 0.83 (8 x 9: 0.90,
+// 9 x 8: 0.86, 6 x 12: 0.98); ni=89: 16 of 6 1.20 (12 x 8: 1.24, 8 x 12: 1.33).
 template <typename R, bool PIPE>
 static cudaError_t launch_gj_p(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
                                R* out, const int32_t* only) {
@@ -1889,17 +1762,18 @@ static cudaError_t launch_gj_p(const Batch& B, double* ws, int32_t* status, int 
       return launch_gj_t<3, 6, 12, 1, true, R, PIPE>(B, ws, status, with_rhs, tr, st, out, only);
     return launch_gj_t<3, 6, 12, 2, true, R, PIPE>(B, ws, status, with_rhs, tr, st, out, only);
   }
-  // up to 96 species: 16 warps of 6 columns (the uneven 256-atmosphere batch,
-  // whose ni=89 atmospheres set its floor: 16.49 ms per step against 16.99
-  // with 12 warps of 8)
   if (B.ni <= 96) return launch_gj_t<3, 6, 16, 1, true, R, PIPE>(B, ws, status, with_rhs, tr, st, out, only);
   return launch_gj_t<4, 8, 16, 1, false, R, PIPE>(B, ws, status, with_rhs, tr, st, out, only);
 }
 template <typename R>
 static cudaError_t launch_gj(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
                              R* out, const int32_t* only, bool pipe = false) {
-  if (pipe) return launch_gj_p<R, true>(B, ws, status, with_rhs, tr, st, out, only);
-  return launch_gj_p<R, false>(B, ws, status, with_rhs, tr, st, out, only);
+  if constexpr (sizeof(R) == 8) {
+    if (!pipe) return launch_dgj(B, ws, status, with_rhs, tr, st, out, only);
+    return launch_gj_p<R, true>(B, ws, status, with_rhs, tr, st, out, only);
+  } else {
+    return launch_gj_p<R, false>(B, ws, status, with_rhs, tr, st, out, only);
+  }
 }
 
 // Paired factor: the pairs of atmospheres (2b, 2b+1), then an odd last
@@ -1916,8 +1790,7 @@ static cudaError_t launch_gj_pair(const Batch& B, double* ws, int32_t* status, i
   Batch B1 = B;
   B1.count = 1;
   const int64_t off = (int64_t)(B.count - 1) * B.nz * ws_per_layer(B.ni, B.ld);
-  return launch_gj_t<3, 6, 12, 1, true, double, false>(B1, ws + off, status + (B.count - 1), with_rhs, tr, st,
-                                                       nullptr, nullptr);
+  return launch_dgj_t<9, 1, true>(B1, ws + off, status + (B.count - 1), with_rhs, tr, st, nullptr, nullptr);
 }
 static bool pair_applies(const Batch& B) { return !B.zoff && B.ni > 64 && B.ni <= 72 && B.count >= 2; }
 
