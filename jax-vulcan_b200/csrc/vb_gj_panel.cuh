@@ -66,12 +66,6 @@ __device__ __forceinline__ void st_pair_if(uint32_t addr, float x, float y, bool
                : "memory");
 }
 
-// 8-byte asynchronous copy global -> shared (both 8-byte aligned).
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // Shared-memory plan of panel_factor_atmosphere (carved in this order, each
 // piece on a 16-byte boundary).
 template <int RPL, int CPW, int NW, typename R>

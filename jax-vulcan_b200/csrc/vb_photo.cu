@@ -1,9 +1,9 @@
 // Photochemistry kernels (reference photo.py):
 //   tau_kernel   optical depth, a top-down running sum per wavelength bin
 //                (photo.py:84-123);
-//   flux_kernel  two-stream Eddington flux: the down and the up recursions in
-//                z run in one thread per bin, all bins in parallel
-//                (photo.py:126-245);
+//   flux_kernel  two-stream Eddington flux: coefficients of every layer in
+//                parallel, the down and the up recursions in z in one thread
+//                per bin (photo.py:126-245);
 //   j_kernel     J-rates of a tile of layers and every branch, warp per
 //                branch, reductions over bins with the two-resolution
 //                trapezoid correction, fused with the write of the photolysis
@@ -28,8 +28,160 @@ constexpr int PHOTO_THREADS = 128;
 constexpr int64_t ACHG_STRIDE = sizeof(VbConvState) / sizeof(double);
 static_assert(sizeof(VbConvState) % sizeof(double) == 0, "VbConvState size");
 
-__global__ void __launch_bounds__(PHOTO_THREADS)
+// Tiled kernels (tau_kernel, flux_kernel): a CTA takes PB bins of one
+// atmosphere and all its layers. Everything that does not depend on the layer
+// before (absorber sums, exponentials, roots, divisions) runs with a thread per
+// (layer, bin) into shared memory; only the recursions in z run with one thread
+// per bin, from operands loaded ahead, and all threads write the results. The
+// arithmetic of each value is the reference's, in its order. One thread per bin
+// for the whole column left a chain of 120 layers x ~300 dependent FP64
+// instructions per thread, and 20 CTAs on 148 SMs for one atmosphere.
+// 32 bins a tile: the recursion, which one warp runs while the others wait,
+// serves 32 bins at a time; the flux tile's seven rows per layer then fill one
+// SM's shared memory at nz = 120. nz=120, 2500 bins, 40 branches (B200, us,
+// before -> now): tau 1 atmosphere 376 -> 21, 64: 420 -> 241; flux 580 -> 30,
+// 1420 -> 952 (about 220 FP64 instructions per layer and bin; the recursion's
+// share is a quarter); J (below) 62 -> 24, 640 -> 272.
+constexpr size_t PHOTO_SMEM_MAX = 220 * 1024;
+
+// Cross sections of the tile's bins (absorbers, then scatterers; 0 outside nbin)
+// in shared memory, [n_abs + n_scat][PB].
+template <int PB>
+__host__ __device__ inline size_t tile_table_doubles(const VbPhoto& P) {
+  return (size_t)(P.n_abs + P.n_scat) * PB;
+}
+template <int PB, int PT>
+__device__ inline void load_cross(const VbPhoto& P, double* cs, int bin0) {
+  for (int e = threadIdx.x; e < (P.n_abs + P.n_scat) * PB; e += PT) {
+    const int k = e / PB, bin = bin0 + e % PB;
+    double v = 0.0;
+    if (bin < P.nbin)
+      v = k < P.n_abs ? P.absp_cross[(int64_t)k * P.nbin + bin] : P.scat_cross[(int64_t)(k - P.n_abs) * P.nbin + bin];
+    cs[e] = v;
+  }
+}
+// Weights of a column's layers by species in table order (absorbers,
+// temperature-dependent absorbers, scatterers), [nz][n].
+template <int PT>
+__device__ inline void load_weights(const VbPhoto& P, double* wt, const double* __restrict__ w, int nz, int ni) {
+  const int n = P.n_abs + P.n_abs_T + P.n_scat;
+  for (int k = threadIdx.x & 31; k < n; k += 32) {   // lanes over species, warps over layers
+    const int i = k < P.n_abs ? P.absp_idx[k] : k < P.n_abs + P.n_abs_T ? P.absp_T_idx[k - P.n_abs]
+                                                                        : P.scat_idx[k - P.n_abs - P.n_abs_T];
+#pragma unroll 8
+    for (int j = threadIdx.x >> 5; j < nz; j += PT / 32) wt[j * n + k] = w[(int64_t)j * ni + i];
+  }
+}
+
+// Species-weighted cross-section sums of JL layers j, j + PR, .. (those below
+// nz) of one bin (c = bin in the tile): absorbers, temperature-dependent
+// absorbers, scatterers, each in table order. Four layers share a cross
+// section's load: with one layer at a time the loads (three per term) bounded
+// the tile.
+constexpr int JL = 4;
+template <int PB, int PR>
+__device__ __forceinline__ void column_sums(const VbPhoto& P, const double* cs, const double* wt,
+                                            const double* __restrict__ xT, int nz, int j, int bin, int c,
+                                            double (&sa)[JL], double (&sT)[JL], double (&ss)[JL]) {
+  const int n = P.n_abs + P.n_abs_T + P.n_scat;
+  const double* w[JL];
+  const double* x[JL];
+#pragma unroll
+  for (int l = 0; l < JL; ++l) {
+    const int jl = min(j + l * PR, nz - 1);   // beyond the column: a repeat nobody reads
+    w[l] = wt + jl * n;
+    x[l] = xT + (int64_t)jl * P.nbin + bin;
+    sa[l] = sT[l] = ss[l] = 0.0;
+  }
+  cs += c;
+#pragma unroll 2
+  for (int k = 0; k < P.n_abs; ++k) {
+    const double v = cs[k * PB];
+#pragma unroll
+    for (int l = 0; l < JL; ++l) sa[l] = sa[l] + w[l][k] * v;
+  }
+  const int64_t tstep = (int64_t)nz * P.nbin;
+#pragma unroll 2
+  for (int k = 0; k < P.n_abs_T; ++k)
+#pragma unroll
+    for (int l = 0; l < JL; ++l) sT[l] = sT[l] + w[l][P.n_abs + k] * x[l][k * tstep];
+  cs += P.n_abs * PB;
+  for (int k = 0; k < P.n_scat; ++k) {
+    const double v = cs[k * PB];
+#pragma unroll
+    for (int l = 0; l < JL; ++l) ss[l] = ss[l] + w[l][P.n_abs + P.n_abs_T + k] * v;
+  }
+}
+
+template <int PB>
+__host__ __device__ inline size_t tau_smem_bytes(const VbPhoto& P, int nz) {
+  return ((size_t)nz * (PB + P.n_abs + P.n_abs_T + P.n_scat) + tile_table_doubles<PB>(P)) * sizeof(double);
+}
+
+template <int PB, int PT>
+__global__ void __launch_bounds__(PT, 1024 / PT)
 tau_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const double* __restrict__ dz,
+           double* __restrict__ tau, const int32_t* __restrict__ due, double* __restrict__ achg) {
+  constexpr int PR = PT / PB;   // layers in flight
+  extern __shared__ double smp[];
+  const int b = blockIdx.y, bin0 = blockIdx.x * PB;
+  if (due && due[b] == 0) return;
+  if (achg && blockIdx.x == 0 && threadIdx.x == 0) achg[(int64_t)b * ACHG_STRIDE] = 0.0;
+  const int nbin = P.nbin, c = threadIdx.x % PB, bin = bin0 + c;
+  const bool on = bin < nbin;
+  double* a = smp;   // [nz][PB]: the layers' depths, then their running sum
+  double* cs = a + nz * PB;
+  double* wt = cs + tile_table_doubles<PB>(P);
+  load_cross<PB, PT>(P, cs, bin0);
+  load_weights<PT>(P, wt, y + (int64_t)b * nz * ni, nz, ni);
+  __syncthreads();
+  const double* dzb = dz + (int64_t)b * nz;
+  const double* xT = P.absp_T_cross + (int64_t)b * P.T_stride;
+  double* tb = tau + (int64_t)b * (nz + 1) * nbin;
+  for (int j0 = threadIdx.x / PB; j0 < nz && on; j0 += JL * PR) {
+    double sa[JL], sT[JL], ss[JL];
+    column_sums<PB, PR>(P, cs, wt, xT, nz, j0, bin, c, sa, sT, ss);
+#pragma unroll
+    for (int l = 0; l < JL; ++l) {
+      const int j = j0 + l * PR;
+      if (j < nz) {
+        double v = 0.0;
+        if (P.n_abs > 0) v = sa[l] * dzb[j];
+        if (P.n_abs_T > 0) v = v + sT[l] * dzb[j];
+        if (P.n_scat > 0) v = v + ss[l] * dzb[j];
+        a[j * PB + c] = v;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < PB && on) {
+    // eight layers' depths at a time in registers: the chain is one addition a layer
+    double acc = a[(nz - 1) * PB + c];
+    int j = nz - 2;
+    for (; j >= 7; j -= 8) {
+      double v[8];
+#pragma unroll
+      for (int l = 0; l < 8; ++l) v[l] = a[(j - l) * PB + c];
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        acc = acc + v[l];
+        a[(j - l) * PB + c] = acc;
+      }
+    }
+    for (; j >= 0; --j) {
+      acc = acc + a[j * PB + c];
+      a[j * PB + c] = acc;
+    }
+  }
+  __syncthreads();
+  if (on)
+    for (int j = threadIdx.x / PB; j <= nz; j += PR) tb[(int64_t)j * nbin + bin] = j < nz ? a[j * PB + c] : 0.0;
+}
+
+// The same with a thread per bin and column: columns whose tile does not fit
+// shared memory.
+__global__ void __launch_bounds__(PHOTO_THREADS)
+tau_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const double* __restrict__ dz,
            double* __restrict__ tau, const int32_t* __restrict__ due, double* __restrict__ achg) {
   const int b = blockIdx.y;
   const int bin = blockIdx.x * blockDim.x + threadIdx.x;
@@ -67,9 +219,21 @@ tau_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const double
   }
 }
 
+// a / b for a finite nonzero b. A zero numerator (opaque layers: no beam, no
+// flux) takes the product, whose value and sign are the quotient's, instead of
+// the division's out-of-range path.
+__device__ __forceinline__ double quot(double a, double b) { return a == 0.0 ? a * b : a / b; }
+
 struct TwoStream {
   double chi, xi, phi, gp, gm;
 };
+
+// w0 = scat / (abs + scat), NaN -> 0, at most 1 - 1e-8 (photo.py:166-170).
+__device__ __forceinline__ double albedo_of(double tot_abs, double tot_scat) {
+  double w0 = tot_scat / fmax(tot_abs + tot_scat, 1e-300);
+  if (isnan(w0)) w0 = 0.0;
+  return fmin(w0, 1.0 - 1e-8);
+}
 
 // Single-scattering albedo of one layer and bin (photo.py:150-170): the
 // ymix-weighted absorption (T-independent and T-dependent cross sections)
@@ -94,33 +258,39 @@ __device__ inline double albedo(const VbPhoto& P, const double* __restrict__ xT,
     for (int k = 0; k < P.n_scat; ++k) s = s + ymix_j[P.scat_idx[k]] * P.scat_cross[(int64_t)k * nbin + bin];
     tot_scat = s;
   }
-  double w0 = tot_scat / fmax(tot_abs + tot_scat, 1e-300);
-  if (isnan(w0)) w0 = 0.0;
-  return fmin(w0, 1.0 - 1e-8);
+  return albedo_of(tot_abs, tot_scat);
 }
 
+// The quotients of the two-stream formulas that depend on the atmosphere's
+// angles only, formed once per thread.
+struct StreamConst {
+  double mu, neg_redd, rmu2, redd2, redd, sum, dif;
+  __device__ explicit StreamConst(const VbPhoto& P)
+      : mu(-1.0 * P.mu_zenith), neg_redd(-1.0 / P.edd), rmu2(1.0 / (mu * mu)), redd2(1.0 / (P.edd * P.edd)),
+        redd(1.0 / P.edd), sum(redd + 1.0 / mu), dif(redd - 1.0 / mu) {}
+};
+
 // Two-stream coefficients of one layer from its albedo (photo.py:171-203).
-__device__ inline TwoStream two_stream(const VbPhoto& P, double w0, double dtau) {
-  const double mu_ang = -1.0 * P.mu_zenith;
-  const double edd = P.edd, ag0 = P.ag0;
+__device__ inline TwoStream two_stream(const VbPhoto& P, const StreamConst& k, double w0, double dtau) {
+  const double ag0 = P.ag0;
   double tran, zp, zm, ll, gp, gm;
   if (ag0 == 0.0) {
     const double sq = sqrt(1.0 - w0);
-    tran = exp(-1.0 / edd * sq * dtau);
+    tran = exp(k.neg_redd * sq * dtau);
     zp = 0.5 * (1.0 + sq);
     zm = 0.5 * (1.0 - sq);
-    ll = -1.0 * w0 / (1.0 / (mu_ang * mu_ang) - 1.0 / (edd * edd) * (1.0 - w0));
-    gp = 0.5 * (ll * (1.0 / edd + 1.0 / mu_ang));
-    gm = 0.5 * (ll * (1.0 / edd - 1.0 / mu_ang));
+    ll = -1.0 * w0 / (k.rmu2 - k.redd2 * (1.0 - w0));
+    gp = 0.5 * (ll * k.sum);
+    gm = 0.5 * (ll * k.dif);
   } else {
     const double wa = 1.0 - w0 * ag0;
-    tran = exp(-1.0 / edd * sqrt(wa * (1.0 - w0)) * dtau);
+    tran = exp(k.neg_redd * sqrt(wa * (1.0 - w0)) * dtau);
     const double rt = sqrt((1.0 - w0) / wa);
     zp = 0.5 * (1.0 + rt);
     zm = 0.5 * (1.0 - rt);
-    ll = ((1.0 - w0) * wa - 1.0) / (1.0 / (mu_ang * mu_ang) - 1.0 / (edd * edd) * (1.0 - w0) * wa);
-    gp = 0.5 * (ll * (1.0 / edd + 1.0 / (mu_ang * wa)) + w0 * ag0 * mu_ang / wa);
-    gm = 0.5 * (ll * (1.0 / edd - 1.0 / (mu_ang * wa)) - w0 * ag0 * mu_ang / wa);
+    ll = ((1.0 - w0) * wa - 1.0) / (k.rmu2 - k.redd2 * (1.0 - w0) * wa);
+    gp = 0.5 * (ll * (k.redd + 1.0 / (k.mu * wa)) + w0 * ag0 * k.mu / wa);
+    gm = 0.5 * (ll * (k.redd - 1.0 / (k.mu * wa)) - w0 * ag0 * k.mu / wa);
   }
   TwoStream c;
   c.chi = zm * zm * (tran * tran) - zp * zp;
@@ -131,8 +301,192 @@ __device__ inline TwoStream two_stream(const VbPhoto& P, double w0, double dtau)
   return c;
 }
 
-__global__ void __launch_bounds__(PHOTO_THREADS)
+// Rows per layer of the flux tile: phi, xi, 1/chi, the upward flux of the
+// previous call (then the downward flux), i_d/mu (then the upward flux), i_u/mu
+// and the direct beam of the nz + 1 levels.
+template <int PB>
+__host__ __device__ inline size_t flux_smem_bytes(const VbPhoto& P, int nz) {
+  return ((size_t)(7 * nz + 1) * PB + tile_table_doubles<PB>(P)) * sizeof(double);
+}
+// the weights' tile lies over the rows xi and 1/chi until the coefficients are formed
+template <int PB>
+constexpr int FLUX_MAX_SPECIES = 2 * PB;
+constexpr int FLUX_THREADS = 512;
+
+template <int PB, int PT>
+__global__ void __launch_bounds__(PT, PB == 32 ? 1 : 2)
 flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const double* __restrict__ ymix,
+            const double* du_prev, double* __restrict__ aflux, double* __restrict__ sflux,
+            double* __restrict__ dd, double* du, const int32_t* __restrict__ due, double flux_atol,
+            double* __restrict__ achg) {
+  // du_prev and du may be one buffer: the tile's bins of du_prev are read
+  // before the block writes du.
+  constexpr int PR = PT / PB;   // layers in flight
+  extern __shared__ double smp[];
+  const int b = blockIdx.y, bin0 = blockIdx.x * PB;
+  if (due && due[b] == 0) return;
+  const int nbin = P.nbin, c = threadIdx.x % PB, bin = bin0 + c, row = threadIdx.x / PB;
+  const bool on = bin < nbin;
+  const int L = nz * PB;
+  double* phi = smp + c;
+  double *xi = phi + L, *rc = xi + L, *ud = rc + L, *id = ud + L, *iu = id + L, *sb = iu + L;
+  double* cs = smp + (7 * nz + 1) * PB;
+  double* wt = smp + L;
+  const int64_t zb = (int64_t)b * (nz + 1) * nbin + bin;
+  const double* tb = tau + zb;
+  // the optical depths (parked in the i_u row) and dflux_u of the previous call
+  // come in while the tables are loaded
+  if (on)
+    for (int j = row; j < nz; j += PR) {
+      cp_async8(iu + j * PB, tb + (int64_t)j * nbin);
+      cp_async8(ud + j * PB, du_prev + zb + (int64_t)j * nbin);
+    }
+  load_cross<PB, PT>(P, cs, bin0);
+  load_weights<PT>(P, wt, ymix + (int64_t)b * nz * ni, nz, ni);
+  const double* xT = P.absp_T_cross + (int64_t)b * P.T_stride;
+  const StreamConst sc(P);
+  const double mu_ang = sc.mu;
+  cp_async_wait_all();
+  __syncthreads();
+  // the direct beam top * exp(tau / mu) of every level (photo.py:173-174), the
+  // layers' optical depths, parked in the i_d row, and their albedos, in the phi row
+  if (on) {
+    const double top = P.sflux_top[bin], t_top = tb[(int64_t)nz * nbin];
+    for (int j = row; j <= nz; j += PR) {
+      const double t0 = j < nz ? iu[j * PB] : t_top;
+      sb[j * PB] = top * exp(quot(t0, mu_ang));
+      if (j < nz) id[j * PB] = t0 - (j + 1 < nz ? iu[(j + 1) * PB] : t_top);
+    }
+  }
+  for (int j0 = row; j0 < nz && on; j0 += JL * PR) {
+    double sa[JL], sT[JL], ss[JL];
+    column_sums<PB, PR>(P, cs, wt, xT, nz, j0, bin, c, sa, sT, ss);
+#pragma unroll
+    for (int l = 0; l < JL; ++l) {
+      const int j = j0 + l * PR;
+      if (j < nz) {
+        double tot_abs = 0.0, tot_scat = 0.0;
+        if (P.n_abs > 0) tot_abs = sa[l];
+        if (P.n_abs_T > 0) tot_abs = tot_abs + sT[l];
+        if (P.n_scat > 0) tot_scat = ss[l];
+        phi[j * PB] = albedo_of(tot_abs, tot_scat);
+      }
+    }
+  }
+  __syncthreads();
+  if (on)
+    for (int j = row; j < nz; j += PR) {
+      const TwoStream q = two_stream(P, sc, phi[j * PB], id[j * PB]);
+      const double dir0 = sb[j * PB] * (-mu_ang), dir1 = sb[(j + 1) * PB] * (-mu_ang);
+      const double i_d = q.phi * q.gm * dir1 - (q.chi * q.gm + q.xi * q.gp) * dir0;
+      const double i_u = q.phi * q.gp * dir0 - (q.xi * q.gm + q.chi * q.gp) * dir1;
+      phi[j * PB] = q.phi;
+      xi[j * PB] = q.xi;
+      rc[j * PB] = 1.0 / q.chi;
+      id[j * PB] = quot(i_d, mu_ang);
+      iu[j * PB] = quot(i_u, mu_ang);
+    }
+  __syncthreads();
+  if (threadIdx.x < PB && on) {
+    // down recursion (photo.py:208-223) with dflux_u of the previous call, then
+    // up (photo.py:225-236)
+    // (a layer's chain is product, difference, sum and product; the operands of
+    // four layers are loaded together, ahead of the four before)
+    double v = 0.0;
+    struct Four {
+      double r[4], p[4], x[4], s[4];
+    };
+    // layers j, j + dir, ..: e walks the rows, all four inside the column
+    auto load = [&](Four& o, int e, int dir, const double* w, const double* src) {
+#pragma unroll
+      for (int l = 0; l < 4; ++l, e += dir * PB) {
+        o.r[l] = rc[e];
+        o.p[l] = phi[e];
+        o.x[l] = xi[e] * w[e];
+        o.s[l] = src[e];
+      }
+    };
+    auto chain = [&](const Four& o, double* out, int dir) {
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        v = o.r[l] * (o.p[l] * v - o.x[l] + o.s[l]);
+        out[dir * l * PB] = v;
+      }
+    };
+    // one direction: n layers from row e on, whole fours first
+    auto sweep = [&](int e, int n, int dir, const double* w, const double* src, double* out) {
+      Four a, c2;
+      int left = n;
+      if (left >= 4) load(a, e, dir, w, src);
+#pragma unroll 1
+      while (left >= 8) {
+        load(c2, e + 4 * dir * PB, dir, w, src);
+        chain(a, out + e, dir);
+        e += 4 * dir * PB;
+        left -= 4;
+        if (left < 8) {
+          a = c2;
+          break;
+        }
+        load(a, e + 4 * dir * PB, dir, w, src);
+        chain(c2, out + e, dir);
+        e += 4 * dir * PB;
+        left -= 4;
+      }
+      if (left >= 4) {
+        chain(a, out + e, dir);
+        e += 4 * dir * PB;
+        left -= 4;
+      }
+      for (; left > 0; --left, e += dir * PB) {
+        v = rc[e] * (phi[e] * v - xi[e] * w[e] + src[e]);
+        out[e] = v;
+      }
+    };
+    sweep((nz - 1) * PB, nz, -1, ud, id, ud);
+    v = 0.0;
+    sweep(0, nz - 1, 1, ud + PB, iu, id);   // level j + 1 into id[j]; the flux down into layer j from level j + 1
+    const int e = (nz - 1) * PB;
+    v = rc[e] * (phi[e] * v - xi[e] * 0.0 + iu[e]);
+    id[e] = v;
+  }
+  __syncthreads();
+  // actinic flux (photo.py:238-244) and the results of every level
+  double change = 0.0;  // largest relative aflux change of this thread's entries above flux_atol
+  if (on) {
+    const double conv = P.hc / P.bins[bin];
+    double* ab = aflux + (int64_t)b * nz * nbin + bin;
+    for (int j = row; j <= nz; j += PR) {
+      const double u_lo = j > 0 ? id[(j - 1) * PB] : 0.0, d_lo = j < nz ? ud[j * PB] : 0.0, s_lo = sb[j * PB];
+      sflux[zb + (int64_t)j * nbin] = s_lo;
+      dd[zb + (int64_t)j * nbin] = d_lo;
+      du[zb + (int64_t)j * nbin] = u_lo;
+      if (j < nz) {
+        const double u_up = id[j * PB], d_up = j + 1 < nz ? ud[(j + 1) * PB] : 0.0, s_up = sb[(j + 1) * PB];
+        const double ave = 0.5 * (s_lo + s_up);
+        const double tot = ave + quot(0.5 * (u_lo + u_up + d_up + d_lo), P.edd);
+        const double an = quot(tot, conv);
+        if (achg && an > flux_atol) {
+          const double r = fabs(an - ab[(int64_t)j * nbin]) / fmax(fabs(an), 1e-300);
+          change = (r > change || r != r) ? r : change;
+        }
+        ab[(int64_t)j * nbin] = an;
+      }
+    }
+  }
+  // the ratios are >= 0 or NaN, so their bit patterns order as their values
+  // do and a NaN wins the maximum, as it does in the reference's max
+  if (achg) {
+    unsigned long long m = static_cast<unsigned long long>(__double_as_longlong(change));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if ((threadIdx.x & 31) == 0 && m)
+      atomicMax(reinterpret_cast<unsigned long long*>(achg + (int64_t)b * ACHG_STRIDE), m);
+  }
+}
+
+__global__ void __launch_bounds__(PHOTO_THREADS)
+flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const double* __restrict__ ymix,
             const double* du_prev, double* __restrict__ aflux, double* __restrict__ sflux,
             double* __restrict__ dd, double* du, const int32_t* __restrict__ due, double flux_atol,
             double* __restrict__ achg) {
@@ -152,7 +506,8 @@ flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const dou
   double* ddb = dd + zb;
   double* dub = du + zb;
   double* ab = aflux + (int64_t)b * nz * nbin;
-  const double mu_ang = -1.0 * P.mu_zenith;
+  const StreamConst sc(P);
+  const double mu_ang = sc.mu;
   const double top = P.sflux_top[bin];
   // albedo of every layer, parked in the sflux rows until the up recursion
   // hands each row its direct beam (the sums over absorbers run once per
@@ -166,7 +521,7 @@ flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const dou
   for (int j = nz - 1; j >= 0; --j) {
     const double t0 = tb[(int64_t)j * nbin + bin], t1 = tb[(int64_t)(j + 1) * nbin + bin];
     const double s_lo = top * exp(t0 / mu_ang);
-    TwoStream c = two_stream(P, sb[(int64_t)j * nbin + bin], t0 - t1);
+    TwoStream c = two_stream(P, sc, sb[(int64_t)j * nbin + bin], t0 - t1);
     const double dir0 = s_lo * (-mu_ang);
     const double dir1 = s_hi * (-mu_ang);
     const double i_d = c.phi * c.gm * dir1 - (c.chi * c.gm + c.xi * c.gp) * dir0;
@@ -184,7 +539,7 @@ flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const dou
   for (int j = 1; j <= nz; ++j) {
     const double t0 = tb[(int64_t)(j - 1) * nbin + bin], t1 = tb[(int64_t)j * nbin + bin];
     const double s_up = top * exp(t1 / mu_ang);
-    TwoStream c = two_stream(P, sb[(int64_t)(j - 1) * nbin + bin], t0 - t1);
+    TwoStream c = two_stream(P, sc, sb[(int64_t)(j - 1) * nbin + bin], t0 - t1);
     const double dir0 = s_lo * (-mu_ang);
     const double dir1 = s_up * (-mu_ang);
     const double i_u = c.phi * c.gp * dir0 - (c.xi * c.gm + c.chi * c.gp) * dir1;
@@ -210,66 +565,103 @@ flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const dou
               static_cast<unsigned long long>(__double_as_longlong(change)));
 }
 
-// J-rates of a tile of JT layers of one atmosphere, all branches: the
-// actinic-flux rows of the tile are staged once in shared memory, each warp
-// takes every (JW)-th branch, and a branch's cross-section row (shared by
-// all layers, unless the branch is temperature dependent) is read once per
-// tile (a small batch splits the branches over gridDim.z block groups);
-// lanes hold the partial sums of the tile's layers, split at din12
-// for the two-resolution trapezoid (photo.py:316-349), then the k row
-// (photo.py:465-478).
+// J-rates of a tile of actinic-flux rows, all branches: JT layers of one
+// atmosphere, or (ATM) one layer of JT atmospheres that share the branch
+// tables, so a temperature-dependent branch's row of that layer serves all of
+// them as the others' rows serve every tile. The flux rows are staged once in
+// shared memory and each warp takes up to JB branches at a time, so a staged
+// flux value is read once per JB branches and a cross section once per tile (a
+// small batch splits the branches over gridDim.z block groups). Lanes hold the
+// partial sums, split at din12 for the two-resolution trapezoid
+// (photo.py:316-349), then the k row (photo.py:465-478). With a branch at a time
+// and tiles of layers, shared and L2 loads (two per product) bounded the
+// kernel: 64 atmospheres, 120 layers, 2500 bins, 40 branches 640 us -> 272.
 constexpr int J_THREADS = 256;
 constexpr int JW = J_THREADS / 32;
-constexpr int JT = 4;
+constexpr int J_ROWS = 4, J_BRANCHES = 5;   // of a full tile; a small batch takes single rows and branches
 
-__global__ void __launch_bounds__(J_THREADS)
-j_kernel(int nz, int nr, int lt, VbPhoto P, const double* __restrict__ aflux, double* __restrict__ J_br,
+template <bool ATM, int JT, int JB>
+__global__ void __launch_bounds__(J_THREADS, 2)
+j_kernel(int batch, int nz, int nr, int lt, VbPhoto P, const double* __restrict__ aflux, double* __restrict__ J_br,
          double* __restrict__ J_br_T, double* __restrict__ k, const int32_t* __restrict__ due) {
   extern __shared__ double fs[];   // [lt][nbin]
-  const int b = blockIdx.y, j0 = blockIdx.x * lt;
-  if (due && due[b] == 0) return;
+  const int b0 = ATM ? blockIdx.y * lt : blockIdx.y, j0 = ATM ? blockIdx.x : blockIdx.x * lt;
+  const int nl = ATM ? min(lt, batch - b0) : min(lt, nz - j0);
+  auto atm_of = [&](int l) { return ATM ? b0 + l : b0; };
+  auto layer_of = [&](int l) { return ATM ? j0 : j0 + l; };
+  bool any = due == nullptr;
+  for (int l = 0; l < (ATM ? nl : 1) && !any; ++l) any = due[atm_of(l)] != 0;
+  if (!any) return;
   const int nbin = P.nbin, d12 = P.din12;
-  const int nl = min(lt, nz - j0);
-  const double* fb = aflux + ((int64_t)b * nz + j0) * nbin;
-  for (int e = threadIdx.x; e < nl * nbin; e += J_THREADS) fs[e] = fb[e];
+  for (int l = 0; l < nl; ++l) {
+    const double* f = aflux + ((int64_t)atm_of(l) * nz + layer_of(l)) * nbin;
+    for (int e = threadIdx.x; e < nbin; e += J_THREADS) fs[l * nbin + e] = f[e];
+  }
+  for (int e = nl * nbin + threadIdx.x; e < lt * nbin; e += J_THREADS) fs[e] = 0.0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nb = P.n_br + P.n_br_T;
-  for (int br = blockIdx.z * JW + warp; br < nb; br += JW * gridDim.z) {
-    const bool is_T = br >= P.n_br;
-    const int brl = is_T ? br - P.n_br : br;
-    const double* c0 = is_T ? P.cross_J_T + (int64_t)b * P.T_stride_J + ((int64_t)brl * nz + j0) * nbin
-                            : P.cross_J + (int64_t)brl * nbin;
-    const int64_t cstep = is_T ? nbin : 0;   // next layer's row (T-dependent tables only)
-    double s1[JT], s2[JT];
+  const int nb = P.n_br + P.n_br_T, step = JW * gridDim.z;
+  for (int br0 = blockIdx.z * JW + warp; br0 < nb; br0 += step * JB) {
+    const double* c0[JB];
+    int64_t cstep[JB];   // next flux row's cross sections (temperature-dependent branches of a layer tile)
 #pragma unroll
-    for (int l = 0; l < JT; ++l) s1[l] = s2[l] = 0.0;
-    for (int q = lane; q < d12; q += 32) {
-#pragma unroll
-      for (int l = 0; l < JT; ++l)
-        if (l < nl) s1[l] = s1[l] + fs[l * nbin + q] * c0[l * cstep + q];
+    for (int u = 0; u < JB; ++u) {
+      const int br = min(br0 + u * step, nb - 1);   // past the last branch: a repeat nobody reads
+      const bool is_T = br >= P.n_br;
+      c0[u] = is_T ? P.cross_J_T + (int64_t)b0 * P.T_stride_J + ((int64_t)(br - P.n_br) * nz + j0) * nbin
+                   : P.cross_J + (int64_t)br * nbin;
+      cstep[u] = is_T && !ATM ? nbin : 0;
     }
-    for (int q = d12 + lane; q < nbin; q += 32) {
+    double sum[2][JB][JT];
 #pragma unroll
-      for (int l = 0; l < JT; ++l)
-        if (l < nl) s2[l] = s2[l] + fs[l * nbin + q] * c0[l * cstep + q];
-    }
+    for (int h = 0; h < 2; ++h) {
+      double(&s)[JB][JT] = sum[h];
 #pragma unroll
-    for (int l = 0; l < JT; ++l) {
+      for (int u = 0; u < JB; ++u)
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        s1[l] = s1[l] + __shfl_xor_sync(0xffffffffu, s1[l], off);
-        s2[l] = s2[l] + __shfl_xor_sync(0xffffffffu, s2[l], off);
+        for (int l = 0; l < JT; ++l) s[u][l] = 0.0;
+      const int q1 = h == 0 ? d12 : nbin;
+      for (int q = (h == 0 ? 0 : d12) + lane; q < q1; q += 32) {
+        double f[JT];
+#pragma unroll
+        for (int l = 0; l < JT; ++l) f[l] = l < lt ? fs[l * nbin + q] : 0.0;
+#pragma unroll
+        for (int u = 0; u < JB; ++u) {
+          if (ATM) {
+            const double cv = c0[u][q];
+#pragma unroll
+            for (int l = 0; l < JT; ++l) s[u][l] = s[u][l] + f[l] * cv;
+          } else {
+#pragma unroll
+            for (int l = 0; l < JT; ++l)
+              if (l < nl) s[u][l] = s[u][l] + f[l] * c0[u][l * cstep[u] + q];
+          }
+        }
       }
-    }
-    if (lane < nl) {
-      const int l = lane, j = j0 + l;
-      double a1 = 0.0, a2 = 0.0;
 #pragma unroll
-      for (int t = 0; t < JT; ++t)
-        if (t == l) { a1 = s1[t]; a2 = s2[t]; }
+      for (int u = 0; u < JB; ++u)
+#pragma unroll
+        for (int l = 0; l < JT; ++l)
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) s[u][l] = s[u][l] + __shfl_xor_sync(0xffffffffu, s[u][l], off);
+    }
+    // lane u JT + l finishes branch u of row l
+    double a1 = 0.0, a2 = 0.0;
+#pragma unroll
+    for (int u = 0; u < JB; ++u)
+#pragma unroll
+      for (int l = 0; l < JT; ++l)
+        if (lane == u * JT + l) {
+          a1 = sum[0][u][l];
+          a2 = sum[1][u][l];
+        }
+    const int u = lane / JT, l = lane % JT, br = br0 + u * step;
+    if (u < JB && l < nl && br < nb && (!due || due[atm_of(l)])) {
+      const bool is_T = br >= P.n_br;
+      const int brl = is_T ? br - P.n_br : br, b = atm_of(l), j = layer_of(l);
       const double* f = fs + l * nbin;
-      const double* c = c0 + l * cstep;
+      const double* c = is_T ? P.cross_J_T + (int64_t)b * P.T_stride_J + ((int64_t)brl * nz + j) * nbin
+                             : P.cross_J + (int64_t)brl * nbin;
       double J = 0.0;
       if (d12 > 0) {
         double J1 = a1 * P.dbin1;
@@ -297,17 +689,43 @@ j_kernel(int nz, int nr, int lt, VbPhoto P, const double* __restrict__ aflux, do
 
 cudaError_t launch_photo_tau(int batch, int nz, int ni, const VbPhoto& P, const double* y, const double* dz,
                              double* tau, const int32_t* due, double* achg, cudaStream_t st) {
-  dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
-  tau_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, y, dz, tau, due, achg);
+  constexpr int PB = 32, PT = 512;
+  const size_t sm = tau_smem_bytes<PB>(P, nz);
+  if (sm <= PHOTO_SMEM_MAX) {
+    cudaError_t e = cudaFuncSetAttribute(tau_kernel<PB, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    dim3 grid((P.nbin + PB - 1) / PB, batch);
+    tau_kernel<PB, PT><<<grid, PT, sm, st>>>(nz, ni, P, y, dz, tau, due, achg);
+  } else {
+    dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
+    tau_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, y, dz, tau, due, achg);
+  }
   return cudaGetLastError();
 }
 
 cudaError_t launch_photo_flux(int batch, int nz, int ni, const VbPhoto& P, const double* tau, const double* ymix,
                               const double* du_prev, double* aflux, double* sflux, double* dd, double* du,
                               const int32_t* due, double flux_atol, double* achg, cudaStream_t st) {
-  dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
-  flux_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol,
-                                              achg);
+  auto tiled = [&](auto kern, int pb, int threads, size_t sm) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    dim3 grid((P.nbin + pb - 1) / pb, batch);
+    kern<<<grid, threads, sm, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg);
+    return cudaGetLastError();
+  };
+  const int species = P.n_abs + P.n_abs_T + P.n_scat;
+  {
+    // 32 bins up to 120 layers or so, 16 up to 240
+    if (species <= FLUX_MAX_SPECIES<32> && flux_smem_bytes<32>(P, nz) <= PHOTO_SMEM_MAX)
+      return tiled(flux_kernel<32, FLUX_THREADS>, 32, FLUX_THREADS, flux_smem_bytes<32>(P, nz));
+    if (species <= FLUX_MAX_SPECIES<16> && flux_smem_bytes<16>(P, nz) <= PHOTO_SMEM_MAX)
+      return tiled(flux_kernel<16, 512>, 16, 512, flux_smem_bytes<16>(P, nz));
+  }
+  {
+    dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
+    flux_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due,
+                                                       flux_atol, achg);
+  }
   return cudaGetLastError();
 }
 
@@ -320,19 +738,24 @@ cudaError_t launch_photo_j(int batch, int nz, int nr, const VbPhoto& P, const do
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int lt = ((int64_t)batch * ((nz + JT - 1) / JT) >= 2 * (int64_t)sms) ? JT : 1;
+  int lt = ((int64_t)batch * ((nz + J_ROWS - 1) / J_ROWS) >= 2 * (int64_t)sms) ? J_ROWS : 1;
   while (lt > 1 && (size_t)lt * P.nbin * sizeof(double) > 200 * 1024) --lt;
   if ((size_t)lt * P.nbin * sizeof(double) > 200 * 1024) return cudaErrorInvalidValue;
   const size_t smem = (size_t)lt * P.nbin * sizeof(double);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(j_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  // a small batch also spreads its branches over blocks (gridDim.z groups of JW)
+  // a batch that shares its tables tiles over atmospheres; a small batch also
+  // spreads its branches over blocks (gridDim.z groups of JW)
+  const bool by_atm = lt == J_ROWS && batch >= J_ROWS && P.T_stride_J == 0;
   const int groups = lt == 1 ? (P.n_br + P.n_br_T + JW - 1) / JW : 1;
-  dim3 grid((nz + lt - 1) / lt, batch, groups);
-  j_kernel<<<grid, J_THREADS, smem, st>>>(nz, nr, lt, P, aflux, J_br, J_br_T, k, due);
-  return cudaGetLastError();
+  auto launch = [&](auto kern, dim3 grid) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, J_THREADS, smem, st>>>(batch, nz, nr, lt, P, aflux, J_br, J_br_T, k, due);
+    return cudaGetLastError();
+  };
+  if (by_atm) return launch(j_kernel<true, J_ROWS, J_BRANCHES>, dim3(nz, (batch + lt - 1) / lt, groups));
+  const dim3 grid((nz + lt - 1) / lt, batch, groups);
+  if (lt == 1) return launch(j_kernel<false, 1, 1>, grid);
+  return launch(j_kernel<false, J_ROWS, J_BRANCHES>, grid);
 }
 
 }  // namespace vb
