@@ -13,6 +13,7 @@
 
 #include "vb_common.cuh"
 #include "vb_launch.cuh"
+#include "vb_sweep.cuh"
 
 namespace vb {
 
@@ -169,224 +170,179 @@ cudaError_t launch_refine_finalize(int batch, const int32_t* state, int32_t* fal
 //   MX_FP64    FP64 inverses in place of its blocks (the FP32 factor failed or
 //              refinement stalled): solved directly, no refinement
 enum MxMode { MX_REFINE = 0, MX_DONE = 1, MX_FP64 = 3 };
-constexpr int MX_THREADS = 256;
 
 __host__ __device__ inline size_t mx_al(size_t x) { return (x + 127) & ~(size_t)127; }
-// Bytes of one ring stage: the FP64 block D_j (refinement passes) and one
-// inverse (FP32 X_j, or the FP64 inverse of an atmosphere in MX_FP64).
-__host__ __device__ inline size_t mx_stage_bytes(int ni, bool refine) {
-  const size_t d = (size_t)ni * round_even(ni) * 8, x = (size_t)ni * round4(ni) * 4;
-  return refine ? mx_al(d) + mx_al(x) : mx_al(d > x ? d : x);
+// Bytes of one ring stage: one inverse (FP32 X_j, or the FP64 inverse of an
+// atmosphere in MX_FP64, which is the larger). The ring is sized in FP64
+// stages; an FP32 atmosphere cuts it into as many of its own.
+__host__ __device__ inline size_t mx_stage_bytes(int ni, bool f64) {
+  return mx_al(f64 ? (size_t)ni * round_even(ni) * 8 : (size_t)ni * round4(ni) * 4);
 }
-__host__ __device__ inline size_t mx_pass_smem(int ni, bool refine) {
-  return 2 * mx_stage_bytes(ni, refine) + 64 + 5 * VB_MAX_NI * sizeof(double);
-}
-
-// out = A v for one n x n block in shared memory (FP32 or FP64 entries, FP64
-// products), four lanes per row, eight rows per warp per pass (warp-uniform passes).
-template <typename T>
-__device__ inline void mx_matvec(const T* __restrict__ A, int n, int lda, const double* v, double* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int sub = lane & 3;
-  for (int i0 = warp * 8; i0 < n; i0 += nw * 8) {
-    const int i = i0 + (lane >> 2);
-    double s0 = 0.0, s1 = 0.0;
-    if (i < n) {
-      const T* row = A + i * lda;
-      int m = sub;
-      for (; m + 4 < n; m += 8) {
-        s0 = fma((double)row[m], v[m], s0);
-        s1 = fma((double)row[m + 4], v[m + 4], s1);
-      }
-      if (m < n) s0 = fma((double)row[m], v[m], s0);
-    }
-    double s = s0 + s1;
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (sub == 0 && i < n) out[i] = s;
-  }
+__host__ __device__ inline size_t mx_pass_smem(int ni, int stages) {
+  return stages * mx_stage_bytes(ni, true) + 64 + 2 * VB_MAX_NI * sizeof(double);
 }
 
-// One pass of the mixed-precision block solve of every atmosphere (CTA each),
-// right-hand side b = the workspace's rmod rows, solution x = its k1 rows
-// (xsel 0) or aux rows (xsel 1).
-//  FIRST: x = M~^{-1} b with the factor's inverses (FP32 X_j with row scales,
+// A pass of the mixed-precision block solve of every atmosphere, right-hand
+// side b = the workspace's rmod rows, solution x = its k1 rows (xsel 0) or aux
+// rows (xsel 1).
+//  first: x = M~^{-1} b with the factor's inverses (FP32 X_j with row scales,
 //         or FP64 for MX_FP64 atmospheres); MX_DONE atmospheres restart as
 //         MX_REFINE (a new right-hand side).
 //  else:  MX_REFINE atmospheres: r = b - M x with the FP64 blocks D_j and
 //         off-diagonals (the system of reference solver.py:33-112),
 //         x += M~^{-1} r; MX_DONE once max|correction| <= tol max|x|.
-// only != nullptr: atmospheres with only[b] == 0 skip. The blocks stream
-// through a two-stage shared-memory ring filled by bulk copies with bounded
-// waits (a wait that gives up drains its copies, sets VB_STATUS_WATCHDOG
-// and the CTA returns). Stage s uses barrier s % 2 in phase (s / 2) % 2;
-// the backward stream's stages continue the forward stream's numbering.
-template <bool FIRST>
-__global__ void __launch_bounds__(MX_THREADS)
-mx_pass_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int xsel, int32_t* __restrict__ mode,
-               const int32_t* __restrict__ only, int32_t* __restrict__ passes, double tol,
-               int32_t* __restrict__ status, long long wlim) {
+// The residual's layers are independent: mx_residual_kernel forms them with a
+// CTA per layer, straight from HBM, ahead of the sweeps (mx_sweep_kernel), whose
+// chain then holds the FP32 inverses only (vb_sweep.cuh's form). With both in
+// one kernel, a layer's residual on the chain and four barriers a layer, a
+// refinement pass of 148 atmospheres (ni=69, nz=120) took 0.68 ms and a first
+// pass 0.27; the residual now takes 0.08, the sweeps of either 0.26.
+
+// Residual rows r_j = b_j - (M x)_j of the refining atmospheres into mv.tmp.
+template <int N8>
+__global__ void __launch_bounds__(32 * N8)
+mx_residual_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int xsel,
+                   const int32_t* __restrict__ mode, const int32_t* __restrict__ only) {
+  __shared__ double x0[VB_MAX_NI];
+  const int b = blockIdx.y, j = blockIdx.x;
+  if ((only && only[b] == 0) || mode[b] != MX_REFINE) return;
+  const Geo g = geo_of(B, b);
+  const int n = B.ni, nz = g.nz, ld = B.ld;
+  if (j >= nz) return;
+  WsView w = ws_view(ws, g, n, ld);
+  MxView mv = mx_view(mxr, g.z0, nz, n);
+  const double* xb = (xsel ? w.aux : w.k1) + (int64_t)j * n;
+  for (int i = threadIdx.x; i < n; i += 32 * N8) x0[i] = xb[i];
+  __syncthreads();
+  const int row = sweep_row();
+  const double p = row_dot<N8>(w.inv + (int64_t)j * n * ld, n, ld, row, x0);
+  if (row < n && (threadIdx.x & 3) == 0) {
+    const int64_t at = (int64_t)j * n + row;
+    double mx = p;
+    if (j > 0) mx = mx + w.subn[at - n] * xb[row - n];
+    if (j < nz - 1) mx = mx + w.supn[at] * xb[row + n];
+    mv.tmp[at] = w.rmod[at] - mx;
+  }
+}
+
+// The sweeps of one atmosphere: forward r'_j = r_j - sub[j-1] o (Inv_{j-1}
+// r'_{j-1}) (r: b on the first pass, else the residual rows) into mv.tmp,
+// backward c_j = Inv_j (r'_j - sup[j] o c_{j+1}), x_j += c_j (x_j = c_j on the
+// first pass). Blocks Inv_0 .. Inv_{nz-2}, then Inv_{nz-1} .. Inv_0, as one
+// stream; N8 = ceil(ni / 8) warps of rows and one that copies.
+template <int N8>
+__global__ void __launch_bounds__(32 * N8 + 32)
+mx_sweep_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int xsel, int first,
+                int32_t* __restrict__ mode, const int32_t* __restrict__ only, int32_t* __restrict__ passes, double tol,
+                int32_t* __restrict__ status, int stages64, long long wlim) {
   extern __shared__ __align__(128) char smem_raw[];
-  __shared__ double red[MX_THREADS / 32][2];
-  __shared__ int redb[MX_THREADS / 32];
+  __shared__ double red[N8][2];
+  __shared__ int redb[N8];
   const int b = blockIdx.x;
   if (only && only[b] == 0) return;
   const int md = mode[b];
-  if (!FIRST && md != MX_REFINE) return;
+  if (!first && md != MX_REFINE) return;
   const bool f64 = md == MX_FP64;
   const Geo g = geo_of(B, b);
   const int n = B.ni, nz = g.nz, ld = B.ld, ldf = round4(n);
   WsView w = ws_view(ws, g, n, ld);
   MxView mv = mx_view(mxr, g.z0, nz, n);
-  const double* bb = w.rmod;
   double* xb = xsel ? w.aux : w.k1;
-  const uint32_t dbytes = (uint32_t)(n * ld * 8);
-  const uint32_t xbytes = f64 ? dbytes : (uint32_t)(n * ldf * 4);
-  const size_t sb = mx_stage_bytes(n, !FIRST);
-  const size_t doff = 0, xoff = FIRST ? 0 : mx_al((size_t)dbytes);   // parts of a stage
-  char* ring = smem_raw;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + 2 * sb);
-  double* va = reinterpret_cast<double*>(bars + 8);   // running vector (r'_{j-1} / c_{j+1})
-  double* vs = va + VB_MAX_NI;                        // scaled operand of an FP32 product
-  double* vx = vs + VB_MAX_NI;                        // x_j, or the backward operand
-  double* vp = vx + VB_MAX_NI;                        // product D_j x_j
-  double* vq = vp + VB_MAX_NI;                        // product Inv v
-  const int tid = threadIdx.x;
-  const bool own = tid < n;
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-  }
-  __syncthreads();
-  // the inverse of layer j, FP32 or FP64
-  auto inv_src = [&](int j) -> const void* {
-    return f64 ? static_cast<const void*>(w.inv + (int64_t)j * n * ld)
-               : static_cast<const void*>(mv.X + (int64_t)j * n * ldf);
+  const uint32_t bytes = f64 ? (uint32_t)(n * ld * 8) : (uint32_t)(n * ldf * 4);
+  const size_t sb = mx_stage_bytes(n, f64), ring = stages64 * mx_stage_bytes(n, true);
+  const int stages = min(SWEEP_MAX_STAGES, (int)(ring / sb));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + ring);
+  double* v = reinterpret_cast<double*>(bars + 8);   // [2][VB_MAX_NI]: the (scaled) operand, by step parity
+  const int F = nz - 1, count = F + nz;              // forward blocks, all blocks
+  auto src = [&](int s) -> const void* {
+    const int64_t j = s < F ? s : count - 1 - s;
+    return f64 ? static_cast<const void*>(w.inv + j * n * ld) : static_cast<const void*>(mv.X + j * n * ldf);
   };
-  // stage contents: forward step j = [D_j (refinement)] + [Inv_{j-1} (j > 0)];
-  // backward step j = [Inv_j]
-  auto issue = [&](int s, bool fwd, int j) {
-    char* st = ring + (size_t)(s & 1) * sb;
-    const bool with_d = fwd && !FIRST;
-    const bool with_x = !fwd || j > 0;
-    const uint32_t bytes = (with_d ? dbytes : 0u) + (with_x ? xbytes : 0u);
-    mbar_expect_tx(&bars[s & 1], bytes);
-    if (with_d) bulk_g2s(st + doff, w.inv + (int64_t)j * n * ld, dbytes, &bars[s & 1]);
-    if (with_x) bulk_g2s(st + xoff, inv_src(fwd ? j - 1 : j), xbytes, &bars[s & 1]);
-  };
-  int issued = 0, waited = 0;   // stage counters (thread 0 issues; everyone waits)
-  auto wait_stage = [&]() -> bool {
-    const int s = waited;
-    const bool ok = mbar_wait(&bars[s & 1], (uint32_t)((s >> 1) & 1), wlim);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) {
-        for (int s3 = s; s3 < issued; ++s3) mbar_wait(&bars[s3 & 1], (uint32_t)((s3 >> 1) & 1), WAIT_LIMIT);
-        atomicOr(status + b, VB_STATUS_WATCHDOG);
-      }
-      return false;
+  BlockStream<decltype(src)> blocks{src, smem_raw, bars, bytes, sb, stages, count};
+  const int warp = threadIdx.x >> 5;
+  if (warp == N8) {
+    if (!blocks.copy(wlim)) {
+      if ((threadIdx.x & 31) == 0) atomicOr(status + b, VB_STATUS_WATCHDOG);
+      return;
     }
-    ++waited;
-    return true;
+    __syncthreads();   // of the reduction below
+    return;
+  }
+  const int row = sweep_row();
+  const bool own = row < n && (threadIdx.x & 3) == 0;
+  const double* rin = first ? w.rmod : mv.tmp;
+  // operands of a step, three sets in rotation: the right-hand side and the
+  // coupling of the layer the step forms an operand for, that layer's row scale
+  // (1 for FP64 inverses) and, backward, x of the step's layer
+  struct Ops {
+    double vec, cpl, sc, x;
   };
-  // product of the inverse held at stage offset xoff with r o v (FP32) or v (FP64)
-  auto inv_apply = [&](const char* st, const double* rs_j, const double* v, double* out) {
-    if (f64) {
-      mx_matvec(reinterpret_cast<const double*>(st + xoff), n, ld, v, out);
+  int loaded = 0;
+  auto load = [&](Ops& o) {
+    const int s = loaded++;
+    o.vec = o.cpl = o.x = 0.0;
+    o.sc = 1.0;
+    if (!own || s >= count) return;
+    if (s < F) {
+      const int64_t at = (int64_t)s * n + row;   // forms r'_{s+1}
+      o.vec = rin[at + n];
+      o.cpl = w.subn[at];
+      if (!f64) o.sc = mv.rs[at + n];
     } else {
-      if (own) vs[tid] = rs_j[tid] * v[tid];
-      __syncthreads();
-      mx_matvec(reinterpret_cast<const float*>(st + xoff), n, ldf, vs, out);
+      const int64_t at = (int64_t)(count - 1 - s) * n + row;   // c of this layer, the operand of the one below
+      if (!first) o.x = xb[at];
+      if (s < count - 1) {
+        o.vec = mv.tmp[at - n];
+        o.cpl = w.supn[at - n];
+        if (!f64) o.sc = mv.rs[at - n];
+      }
     }
   };
-
-  // ---- forward: r_j = b_j - (M x)_j, r'_j = r_j - sub[j-1] o (Inv_{j-1} r'_{j-1})
-  const int j0 = FIRST ? 1 : 0;   // FIRST: layer 0 needs no block
-  const int F = nz - j0;          // forward stages
-  if (FIRST && own) {
-    const double r0 = bb[tid];
-    va[tid] = r0;
-    mv.tmp[tid] = r0;
-  }
-  if (tid == 0) {
-    for (int q = 0; q < 2 && q < F; ++q) {
-      issue(q, true, j0 + q);
-      ++issued;
-    }
-  }
-  for (int j = j0; j < nz; ++j) {
-    const int s = j - j0;
-    double xm = 0.0, xp = 0.0, bj = 0.0, cm = 0.0, cp = 0.0;
-    if (own) {
-      bj = bb[(int64_t)j * n + tid];
-      cm = j > 0 ? w.subn[(int64_t)(j - 1) * n + tid] : 0.0;
-      if (!FIRST) {
-        vx[tid] = xb[(int64_t)j * n + tid];
-        xm = j > 0 ? xb[(int64_t)(j - 1) * n + tid] : 0.0;
-        xp = j < nz - 1 ? xb[(int64_t)(j + 1) * n + tid] : 0.0;
-        cp = j < nz - 1 ? w.supn[(int64_t)j * n + tid] : 0.0;
-      }
-    }
-    if (!wait_stage()) return;
-    const char* st = ring + (size_t)(s & 1) * sb;
-    if (!FIRST) mx_matvec(reinterpret_cast<const double*>(st + doff), n, ld, vx, vp);
-    if (j > 0) inv_apply(st, mv.rs + (int64_t)(j - 1) * n, va, vq);
-    __syncthreads();
-    if (tid == 0 && issued < F) {
-      fence_proxy_async();
-      issue(issued, true, j0 + issued);
-      ++issued;
-    }
-    if (own) {
-      double r = bj;
-      if (!FIRST) {
-        double mx = vp[tid];
-        if (j > 0) mx = mx + cm * xm;
-        if (j < nz - 1) mx = mx + cp * xp;
-        r = r - mx;
-      }
-      if (j > 0) r = r - cm * vq[tid];
-      mv.tmp[(int64_t)j * n + tid] = r;
-      va[tid] = r;
-    }
-    __syncthreads();
-  }
-  // ---- backward: c_j = Inv_j (r'_j - sup[j] o c_{j+1}); x_j += c_j (x_j = c_j on the first pass)
-  //      stage F + q holds Inv_{nz-1-q}
-  if (tid == 0) {
-    fence_proxy_async();
-    for (int q = 0; q < 2 && q < nz; ++q) {
-      issue(F + q, false, nz - 1 - q);
-      ++issued;
-    }
-  }
   double cmax = 0.0, xmax = 0.0;
   bool bad = false;
-  for (int q = 0; q < nz; ++q) {
-    const int j = nz - 1 - q;
+  // r'_{nz-2}, formed in the step that starts by loading the operands of the
+  // first backward step (which needs it); the later ones read this thread's
+  // earlier stores
+  double turn = 0.0;
+  auto step = [&](int s, const Ops& c, Ops& f) {
+    load(f);
+    const double* vc = v + (s & 1) * VB_MAX_NI;
+    double* vn = v + ((s + 1) & 1) * VB_MAX_NI;
+    const double u = f64 ? row_dot<N8>(reinterpret_cast<const double*>(blocks.block()), n, ld, row, vc)
+                         : row_dot<N8>(reinterpret_cast<const float*>(blocks.block()), n, ldf, row, vc);
     if (own) {
-      double v = mv.tmp[(int64_t)j * n + tid];
-      if (j < nz - 1) v = v - w.supn[(int64_t)j * n + tid] * va[tid];
-      vx[tid] = v;
+      const double x = (s == F && F >= 2 ? turn : c.vec) - c.cpl * u;
+      vn[row] = c.sc * x;
+      if (s == F - 2) turn = x;
+      if (s < F) {
+        mv.tmp[(int64_t)(s + 1) * n + row] = x;
+      } else {
+        const double xn = first ? u : c.x + u;
+        xb[(int64_t)(count - 1 - s) * n + row] = xn;
+        cmax = fmax(cmax, fabs(u));
+        xmax = fmax(xmax, fabs(xn));
+        bad |= !isfinite(xn);
+      }
     }
-    if (!wait_stage()) return;
-    const char* st = ring + (size_t)((F + q) & 1) * sb;
-    inv_apply(st, mv.rs + (int64_t)j * n, vx, vq);
-    __syncthreads();
-    if (tid == 0 && issued < F + nz) {
-      fence_proxy_async();
-      issue(issued, false, nz - 1 - (issued - F));
-      ++issued;
-    }
-    if (own) {
-      const double c = vq[tid];
-      const double xn = FIRST ? c : xb[(int64_t)j * n + tid] + c;
-      xb[(int64_t)j * n + tid] = xn;
-      va[tid] = c;
-      cmax = fmax(cmax, fabs(c));
-      xmax = fmax(xmax, fabs(xn));
-      bad |= !isfinite(xn);
-    }
-    __syncthreads();
+    blocks.next();
+    blocks.used();
+    return __syncthreads_or(0) == 0;
+  };
+  if (own) {
+    const double r0 = rin[row];
+    v[row] = (f64 ? 1.0 : mv.rs[row]) * r0;
+    mv.tmp[row] = r0;
+  }
+  Ops o0, o1, o2;
+  load(o0);
+  load(o1);
+  if (__syncthreads_or(0)) return;   // v written, the first block there
+  for (int s = 0; s < count; s += 3) {
+    if (!step(s, o0, o2)) return;
+    if (s + 1 >= count) break;
+    if (!step(s + 1, o1, o0)) return;
+    if (s + 2 >= count) break;
+    if (!step(s + 2, o2, o1)) return;
   }
   // ---- convergence of this atmosphere
 #pragma unroll
@@ -395,22 +351,22 @@ mx_pass_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, int xse
     xmax = fmax(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
   }
   const int anybad = __any_sync(0xffffffffu, bad);
-  if ((tid & 31) == 0) {
-    red[tid >> 5][0] = cmax;
-    red[tid >> 5][1] = xmax;
-    redb[tid >> 5] = anybad;
+  if ((threadIdx.x & 31) == 0) {
+    red[warp][0] = cmax;
+    red[warp][1] = xmax;
+    redb[warp] = anybad;
   }
   __syncthreads();
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
     double cm2 = red[0][0], xm2 = red[0][1];
     int nb = redb[0];
-    for (int q = 1; q < MX_THREADS / 32; ++q) {
+    for (int q = 1; q < N8; ++q) {
       cm2 = fmax(cm2, red[q][0]);
       xm2 = fmax(xm2, red[q][1]);
       nb |= redb[q];
     }
     if (passes) passes[b] += 1;
-    if (FIRST) {
+    if (first) {
       if (md != MX_FP64) mode[b] = MX_REFINE;
     } else if (!nb && cm2 <= tol * xm2) {
       mode[b] = MX_DONE;
@@ -466,22 +422,43 @@ __global__ void mx_finish_kernel(Batch B, const double* __restrict__ ws, const d
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status + b, VB_STATUS_NONFINITE);
 }
 
-template <bool FIRST>
-static cudaError_t launch_mx_pass_t(const Batch& B, double* ws, void* mxr, int xsel, int32_t* mode,
+template <int N8>
+static cudaError_t launch_mx_pass_t(const Batch& B, double* ws, void* mxr, int xsel, bool first, int32_t* mode,
                                     const int32_t* only, int32_t* passes, double tol, int32_t* status,
                                     long long wlim, cudaStream_t st) {
-  const size_t sm = mx_pass_smem(B.ni, !FIRST);
-  cudaError_t e = cudaFuncSetAttribute(mx_pass_kernel<FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (!first) {
+    dim3 grid(B.nz, B.count);
+    mx_residual_kernel<N8><<<grid, 32 * N8, 0, st>>>(B, ws, mxr, xsel, mode, only);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  // as deep a ring as fits, or as lets two CTAs share an SM
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int stages = SWEEP_MAX_STAGES;
+  while (B.count > sms && stages > 2 && 2 * mx_pass_smem(B.ni, stages) > 224 * 1024) --stages;
+  while (stages > 1 && mx_pass_smem(B.ni, stages) > 220 * 1024) --stages;
+  const size_t sm = mx_pass_smem(B.ni, stages);
+  cudaError_t e = cudaFuncSetAttribute(mx_sweep_kernel<N8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  mx_pass_kernel<FIRST><<<B.count, MX_THREADS, sm, st>>>(B, ws, mxr, xsel, mode, only, passes, tol, status, wlim);
+  mx_sweep_kernel<N8><<<B.count, 32 * N8 + 32, sm, st>>>(B, ws, mxr, xsel, first, mode, only, passes, tol, status,
+                                                         stages, wlim);
   return cudaGetLastError();
+}
+
+template <int N8 = 1>
+static cudaError_t launch_mx_pass_n(int n8, const Batch& B, double* ws, void* mxr, int xsel, bool first,
+                                    int32_t* mode, const int32_t* only, int32_t* passes, double tol, int32_t* status,
+                                    long long wlim, cudaStream_t st) {
+  if constexpr (N8 < VB_MAX_NI / 8)
+    if (n8 > N8) return launch_mx_pass_n<N8 + 1>(n8, B, ws, mxr, xsel, first, mode, only, passes, tol, status, wlim, st);
+  return launch_mx_pass_t<N8>(B, ws, mxr, xsel, first, mode, only, passes, tol, status, wlim, st);
 }
 
 cudaError_t launch_mx_pass(const Batch& B, double* ws, void* mxr, int xsel, bool first, int32_t* mode,
                            const int32_t* only, int32_t* passes, double tol, int32_t* status, cudaStream_t st) {
-  const long long wlim = wait_limit();
-  return first ? launch_mx_pass_t<true>(B, ws, mxr, xsel, mode, only, passes, tol, status, wlim, st)
-               : launch_mx_pass_t<false>(B, ws, mxr, xsel, mode, only, passes, tol, status, wlim, st);
+  return launch_mx_pass_n((B.ni + 7) / 8, B, ws, mxr, xsel, first, mode, only, passes, tol, status, wait_limit(), st);
 }
 
 cudaError_t launch_mx_mode(int batch, int op, int32_t* mode, int32_t* todo, int32_t* status32, int32_t* status,

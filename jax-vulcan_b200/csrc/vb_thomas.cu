@@ -17,6 +17,7 @@
 #include "vb_common.cuh"
 #include "vb_gj_panel.cuh"
 #include "vb_launch.cuh"
+#include "vb_sweep.cuh"
 
 namespace vb {
 
@@ -1387,161 +1388,140 @@ bgj32_factor_kernel(Batch B, double* __restrict__ ws, void* __restrict__ mxr, in
 }
 
 // ---------------------------------------------------------------- sweeps
-constexpr int SWEEP_THREADS = 256;
-constexpr int SWEEP_MAX_STAGES = 3;
-
 __host__ __device__ inline size_t sweep_smem_bytes(int ni, int stages) {
-  return (size_t)stages * ni * round_even(ni) * sizeof(double) + 64 + 2 * VB_MAX_NI * sizeof(double);
-}
-
-// out = Inv v (or Inv^T v) for one n x n block held in shared memory.
-// Inv v: four lanes per row (two interleaved partial sums each, then two
-// shuffle levels), eight rows per warp per pass; the pass loop is
-// warp-uniform so every lane reaches the shuffles.
-__device__ inline void block_matvec_s(const double* __restrict__ Inv, int n, int ld, bool trans,
-                                      const double* v, double* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (!trans) {
-    const int sub = lane & 3;
-    for (int i0 = warp * 8; i0 < n; i0 += nw * 8) {
-      const int i = i0 + (lane >> 2);
-      double s0 = 0.0, s1 = 0.0;
-      if (i < n) {
-        const double* row = Inv + i * ld;
-        int m = sub;
-        for (; m + 4 < n; m += 8) {
-          s0 = fma(row[m], v[m], s0);
-          s1 = fma(row[m + 4], v[m + 4], s1);
-        }
-        if (m < n) s0 = fma(row[m], v[m], s0);
-      }
-      double s = s0 + s1;
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      if (sub == 0 && i < n) out[i] = s;
-    }
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      double s = 0.0;
-      for (int m = 0; m < n; ++m) s = fma(Inv[m * ld + i], v[m], s);
-      out[i] = s;
-    }
-  }
+  return (size_t)stages * ni * round_even(ni) * sizeof(double) + 64 + 4 * VB_MAX_NI * sizeof(double);
 }
 
 // One sweep of one atmosphere over its stored inverses: forward elimination
 // (solver.py:73-88) or back substitution (solver.py:91-111), optionally fused
-// with the Ros2 combination (jax_step.py:313-314). The inverse blocks stream
-// through a ring of `stages` shared-memory buffers filled by bulk copies.
-__global__ void __launch_bounds__(SWEEP_THREADS)
+// with the Ros2 combination (jax_step.py:313-314). Warps: N8 of rows (N8 =
+// ceil(ni / 8)), one that copies and, for the Ros2 combination, one per 32
+// species that forms a layer's results while the chain takes the next. N8 = 0:
+// the transposed system (steady_state_grad.py:218-219: sub- and super-diagonal
+// exchanged, the blocks applied transposed), a thread per column. nz=120, ni=69
+// (B200, us a sweep, before -> now; vb_sweep.cuh): one atmosphere 246 -> 78, 148:
+// 249 -> 113 (94 % of measured HBM), 296: 280 -> 220 (96 %).
+template <int N8>
+__global__ void __launch_bounds__(N8 ? 32 * N8 + 32 + 32 * ((N8 + 3) / 4) : VB_MAX_NI + 32)
 sweep_kernel(Batch B, double* __restrict__ ws, SweepArgs A, int stages, long long wlim) {
+  constexpr bool TR = N8 == 0;
   extern __shared__ __align__(128) char smem_raw[];
   const int b = blockIdx.x;
   Geo g = geo_of(B, b);
   WsView w = ws_view(ws, g, B.ni, B.ld);
   const int n = B.ni, nz = g.nz, ld = B.ld;
   const int blk = n * ld;
-  const uint32_t blk_bytes = (uint32_t)(blk * sizeof(double));
-  double* ring = reinterpret_cast<double*>(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + (size_t)stages * blk);
-  double* v = reinterpret_cast<double*>(bars + 8);
-  double* u = v + VB_MAX_NI;
-  const bool tr = A.transposed != 0;
-  // transposed system: sub/super exchange roles (steady_state_grad.py:218-219)
-  const double* up = tr ? w.subn : w.supn;   // couples x[j+1] into row j
-  const double* lo = tr ? w.supn : w.subn;   // couples x[j-1] into row j
   double* vecs = A.user ? A.user + g.z0 * n : w.rmod;
-  const bool fwd = A.mode == SWEEP_FWD;
-  const int count = fwd ? nz - 1 : nz;                 // blocks used, in order
-  auto block_of = [&](int s2) { return fwd ? s2 : nz - 1 - s2; };
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < stages; ++st) mbar_init(&bars[st], 1);
+  const bool fwd = A.mode == SWEEP_FWD, fin = A.mode == SWEEP_BACK_FINAL;
+  const int count = fwd ? nz - 1 : nz;   // blocks used, in order
+  const int first = fwd ? 0 : nz - 1, dir = fwd ? 1 : -1;
+  auto src = [&](int s) -> const void* { return w.inv + (int64_t)(first + dir * s) * blk; };
+  const size_t sb = (size_t)blk * sizeof(double);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + stages * sb);
+  double* v = reinterpret_cast<double*>(bars + 8);   // [2][VB_MAX_NI]: the running vector, by step parity
+  double* us = v + 2 * VB_MAX_NI;                    // [2][VB_MAX_NI]: the products, for the Ros2 combination
+  BlockStream<decltype(src)> blocks{src, smem_raw, bars, (uint32_t)sb, sb, stages, count};
+  const int rows_warps = TR ? (n + 31) >> 5 : N8;
+  const int warp = threadIdx.x >> 5;
+  if (warp == rows_warps) {
+    if (!blocks.copy(wlim) && (threadIdx.x & 31) == 0 && A.status) atomicOr(A.status + b, VB_STATUS_WATCHDOG);
+    return;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < stages && st < count; ++st) {
-      mbar_expect_tx(&bars[st], blk_bytes);
-      bulk_g2s(ring + (size_t)st * blk, w.inv + (int64_t)block_of(st) * blk, blk_bytes, &bars[st]);
-    }
-  }
-  double* out = A.user ? A.user + g.z0 * n : w.k1;
-  const double r = ros2_r();
-  const int tid = threadIdx.x;
-  const bool own = tid < n;   // thread i owns element i of every vector (ni <= 128 < SWEEP_THREADS)
-  if (fwd && own) v[tid] = vecs[tid];
-  // Operands of a layer that do not depend on the running vector, loaded one
-  // layer ahead so their latency hides behind the block copy and the product
-  // (none of them is written by this kernel before it is read).
-  double p_vec = 0.0, p_cpl = 0.0, p_y = 0.0, p_k1 = 0.0;
-  auto prefetch = [&](int s2) {
-    if (!own || s2 >= count) return;
-    const int j = block_of(s2);
-    if (fwd) {
-      p_vec = vecs[(int64_t)(j + 1) * n + tid];
-      p_cpl = lo[(int64_t)j * n + tid];
-    } else {
-      p_vec = vecs[(int64_t)j * n + tid];
-      p_cpl = j < nz - 1 ? up[(int64_t)j * n + tid] : 0.0;
-      if (A.mode == SWEEP_BACK_FINAL) {
-        p_y = A.y[g.z0 * n + (int64_t)j * n + tid];
-        p_k1 = w.k1[(int64_t)j * n + tid];
+  if (warp > rows_warps) {
+    // sol = y + 3/(2r) k1 + 1/(2r) k2 ; delta = |sol - yk2| (jax_step.py:313-314)
+    const int i = threadIdx.x - 32 * (rows_warps + 1);
+    const double r = ros2_r();
+    bool bad = false;
+    for (int s = 0; s <= count; ++s) {
+      double y = 0.0, k1 = 0.0;
+      const int64_t at = (int64_t)(first + dir * (s - 1)) * n + i;
+      if (s > 0 && i < n) {
+        y = A.y[g.z0 * n + at];
+        k1 = w.k1[at];
+      }
+      if (s > 0) blocks.used();
+      if (__syncthreads_or(0)) return;
+      if (s > 0 && i < n) {
+        const double u = us[((s - 1) & 1) * VB_MAX_NI + i];
+        const int64_t e = g.z0 * n + at;
+        const double sv = y + (3.0 / (2.0 * r)) * k1 + (1.0 / (2.0 * r)) * u;
+        const double yk2 = y + k1 / r;
+        w.aux[at] = u;   // k2, kept for vb_ros2_stages
+        A.sol[e] = sv;
+        A.delta[e] = fabs(sv - yk2);
+        bad |= !isfinite(sv);
       }
     }
+    if (bad) atomicOr(A.status + b, VB_STATUS_NONFINITE);
+    return;
+  }
+  // element `row` of every vector belongs to one lane
+  const int row = TR ? (int)threadIdx.x : sweep_row();
+  const bool own = row < n && (TR || (threadIdx.x & 3) == 0);
+  const int64_t step_n = (int64_t)dir * n;
+  // the coupling of a step's layer with the next one: sub_d[j] forward,
+  // sup_d[j - 1] backward (exchanged for the transposed system)
+  const double* cpl = fwd == TR ? w.supn : w.subn;
+  int64_t at = (int64_t)first * n + row;   // this layer's element
+  const double* pv = vecs + at + step_n;   // of the layer two steps on, as loaded
+  const double* pc = cpl + at + (fwd ? 0 : -n);
+  // the next layer's right-hand side and coupling of steps s, s + 1 and s + 2
+  // in three sets taken in rotation (moving a set still being loaded would wait)
+  struct Ops {
+    double vec, cpl;
   };
-  prefetch(0);
-  int issued = min(stages, count);
-  for (int s2 = 0; s2 < count; ++s2) {
-    const int st = s2 % stages;
-    const uint32_t parity = (uint32_t)((s2 / stages) & 1);
-    const int j = block_of(s2);
-    const double c_vec = p_vec, c_cpl = p_cpl, c_y = p_y, c_k1 = p_k1;
-    prefetch(s2 + 1);
-    if (!fwd && own) {
-      double x = c_vec;
-      if (j < nz - 1) x = x - c_cpl * u[tid];
-      v[tid] = x;
+  int loaded = 0;
+  auto load = [&](Ops& o) {
+    o.vec = o.cpl = 0.0;
+    if (own && loaded < (fwd ? count : count - 1)) {
+      o.vec = *pv;
+      o.cpl = *pc;
     }
-    const bool ok = mbar_wait(&bars[st], parity, wlim);
-    if (__syncthreads_or(!ok)) {
-      // give up: wait (bounded) for the copies still in flight, report, return
-      if (threadIdx.x == 0) {
-        for (int s3 = s2; s3 < issued; ++s3)
-          mbar_wait(&bars[s3 % stages], (uint32_t)((s3 / stages) & 1), WAIT_LIMIT);
-        if (A.status) atomicOr(A.status + b, VB_STATUS_WATCHDOG);
-      }
-      return;
-    }
-    block_matvec_s(ring + (size_t)st * blk, n, ld, tr, v, u);
-    __syncthreads();
-    if (threadIdx.x == 0 && s2 + stages < count) {
-      fence_proxy_async();
-      mbar_expect_tx(&bars[st], blk_bytes);
-      bulk_g2s(ring + (size_t)st * blk, w.inv + (int64_t)block_of(s2 + stages) * blk, blk_bytes, &bars[st]);
-      ++issued;
+    ++loaded;
+    pv += step_n;
+    pc += step_n;
+  };
+  double* out = (A.user ? A.user + g.z0 * n : w.k1);
+  if (own) v[row] = vecs[at];
+  auto step = [&](int s, const Ops& c, Ops& f) {
+    load(f);
+    const double* vc = v + (s & 1) * VB_MAX_NI;
+    double* vn = v + ((s + 1) & 1) * VB_MAX_NI;
+    const double* Inv = reinterpret_cast<const double*>(blocks.block());
+    double u = 0.0;
+    if constexpr (!TR) {
+      u = row_dot<N8>(Inv, n, ld, row, vc);
+    } else if (own) {
+#pragma unroll 8
+      for (int m = 0; m < n; ++m) u = fma(Inv[m * ld + row], vc[m], u);
     }
     if (own) {
-      if (fwd) {
-        // rhs'[j+1] = rhs[j+1] - sub_d[j] o (Inv_j rhs'[j])
-        const double x = c_vec - c_cpl * u[tid];
-        vecs[(int64_t)(j + 1) * n + tid] = x;
-        v[tid] = x;
-      } else {
-        const double kj = u[tid];
-        if (A.mode == SWEEP_BACK) {
-          out[(int64_t)j * n + tid] = kj;
-        } else {
-          // sol = y + 3/(2r) k1 + 1/(2r) k2 ; delta = |sol - yk2| (jax_step.py:313-314)
-          const int64_t e = g.z0 * n + (int64_t)j * n + tid;
-          const double s = c_y + (3.0 / (2.0 * r)) * c_k1 + (1.0 / (2.0 * r)) * kj;
-          const double yk2 = c_y + c_k1 / r;
-          w.aux[(int64_t)j * n + tid] = kj;   // k2, kept for vb_ros2_stages
-          A.sol[e] = s;
-          A.delta[e] = fabs(s - yk2);
-          if (!isfinite(s)) atomicOr(A.status + b, VB_STATUS_NONFINITE);
-        }
-      }
+      // forward: rhs'[j+1] = rhs[j+1] - sub_d[j] o (Inv_j rhs'[j]); backward:
+      // x[j] = u, and the operand of layer j - 1
+      const double x = c.vec - c.cpl * u;
+      vn[row] = x;
+      if (fwd)
+        vecs[at + n] = x;
+      else if (fin)
+        us[(s & 1) * VB_MAX_NI + row] = u;
+      else
+        out[at] = u;
     }
-    __syncthreads();
+    at += step_n;
+    blocks.next();
+    blocks.used();
+    return __syncthreads_or(0) == 0;
+  };
+  Ops o0, o1, o2;
+  load(o0);
+  load(o1);
+  if (__syncthreads_or(0)) return;   // v written, the first block there
+  for (int s = 0; s < count; s += 3) {
+    if (!step(s, o0, o2)) return;
+    if (s + 1 >= count) break;
+    if (!step(s + 1, o1, o0)) return;
+    if (s + 2 >= count) break;
+    if (!step(s + 2, o2, o1)) return;
   }
 }
 
@@ -1826,17 +1806,30 @@ cudaError_t launch_factor_into<double>(const Batch& B, double* ws, double* out, 
   return launch_gj<double>(B, ws, status, 0, 1, st, out, only, v == 2);
 }
 
+template <int N8 = 1, typename Launch>
+static cudaError_t launch_sweep_n(int n8, int threads, Launch launch) {
+  if constexpr (N8 < VB_MAX_NI / 8)
+    if (n8 > N8) return launch_sweep_n<N8 + 1>(n8, threads, launch);
+  return launch(sweep_kernel<N8>, threads);
+}
+
 cudaError_t launch_sweep(const Batch& B, double* ws, const SweepArgs& A, cudaStream_t st) {
+  // as deep a ring as fits; more atmospheres than SMs: two CTAs share an SM (one
+  // wave), which takes a shallower one
   int stages = B.sweep_stages ? B.sweep_stages : SWEEP_MAX_STAGES;
   while (stages > 1 && sweep_smem_bytes(B.ni, stages) > 220 * 1024) --stages;
-  // more atmospheres than SMs: a shallower ring lets two CTAs share an SM (one wave)
   if (!B.sweep_stages && B.count > sm_count())
     while (stages > 2 && 2 * sweep_smem_bytes(B.ni, stages) > 224 * 1024) --stages;
   size_t sm = sweep_smem_bytes(B.ni, stages);
-  cudaError_t e = cudaFuncSetAttribute(sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
-  sweep_kernel<<<B.count, SWEEP_THREADS, sm, st>>>(B, ws, A, stages, g_wait_limit);
-  return cudaGetLastError();
+  auto launch = [&](auto kern, int threads) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    kern<<<B.count, threads, sm, st>>>(B, ws, A, stages, g_wait_limit);
+    return cudaGetLastError();
+  };
+  if (A.transposed) return launch(sweep_kernel<0>, 32 * ((B.ni + 31) / 32) + 32);
+  const int n8 = (B.ni + 7) / 8;
+  return launch_sweep_n(n8, 32 * n8 + 32 + (A.mode == SWEEP_BACK_FINAL ? 32 * ((B.ni + 31) / 32) : 0), launch);
 }
 
 cudaError_t launch_pack_blocks(const Batch& B, const double* diag, const double* sup_d,
