@@ -545,12 +545,14 @@ struct DGJ {
 //  * The first right-hand side's sweep of the layer before and the store of
 //    its inverse run in the idle warps while the first panel is eliminated.
 // Bound by the chain of pivot steps: about 270 cycles a step alone (150
-// instructions of one warp, issued in order), 400 beside the other warps of
-// the block, 670 with two blocks on the SM. Factor of nz=120, ni=69 (B200, ms,
+// instructions of one warp, issued in order), 370 beside the other warps of
+// the block, 600 with two blocks on the SM. Factor of nz=120, ni=69 (B200, ms,
 // one block barrier per step before, this kernel now): one atmosphere 3.07,
-// 2.39; 148 (one per SM) 3.21, 2.40; 296 (two per SM) 5.64, 3.61; ni=89,
-// nz=150, 128 atmospheres 6.03, 4.58; ni=30, nz=43, one 0.349, 0.269.
-template <int NT, bool DPF>
+// 2.10; 148 (one per SM) 3.21, 2.11; 296 (two per SM) 5.64, 3.65; ni=89,
+// nz=150, 128 atmospheres 6.03, 4.13; ni=30, nz=43, one 0.349, 0.242.
+// WIDE: registers for both halves of a panel's update at once (one block on the
+// SM).
+template <int NT, bool DPF, bool WIDE>
 __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, const double* Din, double* out,
                                                        const double* __restrict__ supn,
                                                        const double* __restrict__ subn, double* rhs, bool tr,
@@ -763,7 +765,7 @@ __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, co
     int sl[NT];   // the panel's step of each row (others out of 0..7)
 #pragma unroll
     for (int a = 0; a < NT; ++a) sl[a] = qs[8 * a + g] - k0;
-#pragma unroll 1
+#pragma unroll(WIDE ? 2 : 1)
     for (int h = 0; h < 2; ++h) {
       double* U = Uw + 32 * h;
       const uint32_t us = smem_u32(Uw + 2 * t4);
@@ -793,25 +795,27 @@ __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, co
     {
       double2* O = reinterpret_cast<double2*>(out + (int64_t)j * blk);
       const double2* S2 = reinterpret_cast<const double2*>(Ib);
+#pragma unroll 4
       for (int e = (warp - w0) * 32 + lane; e < blk / 2; e += (NW - w0) * 32) O[e] = S2[e];
     }
     if (!rhs || j + 1 >= nz) return;
     const double* cj = cpl + (j & 1) * 3 * NP;
     const double* vc = vecs + (j & 1) * NP;
     double* vn = vecs + ((j + 1) & 1) * NP;
-    // four lanes per row, eight rows per warp per pass (warp-uniform passes)
+    // four lanes per row, eight rows per warp per pass (warp-uniform passes), the
+    // rows dealt against bank conflicts as in the sweeps
     const int sub = lane & 3;
     for (int i0 = (warp - w0) * 8; i0 < n; i0 += (NW - w0) * 8) {
-      const int i = i0 + (lane >> 2);
+      const int i = i0 + ((2 * g) & 7) + (g >> 2);
+      const double* row = Ib + min(i, n - 1) * ld;
       double s0 = 0.0, s1 = 0.0;
-      if (i < n) {
-        int m = sub;
-        for (; m + 4 < n; m += 8) {
-          s0 = fma(Ib[i * ld + m], vc[m], s0);
-          s1 = fma(Ib[i * ld + m + 4], vc[m + 4], s1);
-        }
-        if (m < n) s0 = fma(Ib[i * ld + m], vc[m], s0);
+      int m = sub;
+#pragma unroll 4
+      for (; m + 4 < n; m += 8) {
+        s0 = fma(row[m], vc[m], s0);
+        s1 = fma(row[m + 4], vc[m + 4], s1);
       }
+      if (m < n) s0 = fma(row[m], vc[m], s0);
       double s = s0 + s1;
       s += __shfl_xor_sync(FULL, s, 1);
       s += __shfl_xor_sync(FULL, s, 2);
@@ -846,29 +850,36 @@ __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, co
       const double* cr = cp + (tr ? 0 : NP);             // the sub_d / sup_d factor of tile row i
       const double* cm = cp + (tr ? NP : 0);             // and column m
       const int si = tr ? 1 : ld, sm = tr ? ld : 1;      // element strides of tile rows / columns in D and Ib
-      auto element = [&](int i, int m) {
-        if (i >= n || m >= n) return 0.0;
-        double v = D[i * si + m * sm];
-        if (j > 0) {
-          const double cb = tr ? cm[m] * cr[i] : cr[i] * cm[m];
-          v = v - cb * Ib[i * si + m * sm];
-        }
+      // element at offset o with the coupling factors f (sup_d sub_d of row and column)
+      auto element = [&](bool in, int o, double f) {
+        double v = in ? D[o] : 0.0;
+        if (j > 0 && in) v = v - f * Ib[o];
         return v;
       };
       if (warp < 2) {
+        double f[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) f[c] = 8 * warp + c < n ? cm[8 * warp + c] : 0.0;
 #pragma unroll
         for (int r = 0; r < RPL; ++r) {
           const int i = lane + 32 * r;
+          const double fr = i < n ? cr[i] : 0.0;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) XR(r, c) = element(i, 8 * warp + c);
+          for (int c = 0; c < 8; ++c)
+            XR(r, c) = element(i < n && 8 * warp + c < n, i * si + (8 * warp + c) * sm, f[c] * fr);
           msk[r] = i < n ? 0xffffff00u : 0u;
           cc[r] = i < n ? 255u - (unsigned)i : 0u;
         }
       } else {
+        const int m = 8 * warp + 2 * t4;
+        const double f0 = m < n ? cm[m] : 0.0, f1 = m + 1 < n ? cm[m + 1] : 0.0;
 #pragma unroll
-        for (int a = 0; a < NT; ++a)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) XF(a, e) = element(8 * a + g, 8 * warp + 2 * t4 + e);
+        for (int a = 0; a < NT; ++a) {
+          const int i = 8 * a + g;
+          const double fr = i < n ? cr[i] : 0.0;
+          XF(a, 0) = element(i < n && m < n, i * si + m * sm, f0 * fr);
+          XF(a, 1) = element(i < n && m + 1 < n, i * si + (m + 1) * sm, f1 * fr);
+        }
       }
     }
     for (int i = threadIdx.x; i < NP; i += NW * 32) qs[i] = -1;
@@ -921,27 +932,29 @@ __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, co
     // ---- scale rows by 1/piv, scatter B^{-1}[q(i)][p_m] = T[i][m] into Ib
     //      (A'^{-1}[p_m][q(i)] when tr; q(i) = qs[i], the step pivoting on row i)
     if (warp < np) {
-      int pm[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int m = 8 * warp + 2 * t4 + e;
-        pm[e] = m < n ? pivs[m] : -1;
-      }
+      const int m = 8 * warp + 2 * t4;
+      const int qstr = tr ? 1 : ld, pstr = tr ? ld : 1;
+      const bool on0 = m < n, on1 = m + 1 < n;
+      double* d0 = Ib + (on0 ? pivs[m] * pstr : 0);
+      double* d1 = Ib + (on1 ? pivs[m + 1] * pstr : 0);
+      unsigned top = 0;   // largest exponent field of the results: all ones when not finite
 #pragma unroll
       for (int a = 0; a < NT; ++a) {
         const int i = 8 * a + g;
         if (i < n) {
-          const double s = rps[i];
-          const int qi = qs[i];
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            if (pm[e] >= 0) {
-              const double v = XF(a, e) * s;
-              if (!isfinite(v)) st_local |= VB_STATUS_NONFINITE;
-              Ib[tr ? pm[e] * ld + qi : qi * ld + pm[e]] = v;
-            }
+          const double s = rps[i], v0 = XF(a, 0) * s, v1 = XF(a, 1) * s;
+          const int at = qs[i] * qstr;
+          if (on0) {
+            d0[at] = v0;
+            top = max(top, (unsigned)__double2hiint(v0) & 0x7ff00000u);
+          }
+          if (on1) {
+            d1[at] = v1;
+            top = max(top, (unsigned)__double2hiint(v1) & 0x7ff00000u);
+          }
         }
       }
+      if (top == 0x7ff00000u) st_local |= VB_STATUS_NONFINITE;
     }
     cp_async_wait_all();
   }

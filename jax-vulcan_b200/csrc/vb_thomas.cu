@@ -877,7 +877,7 @@ dgj_factor_kernel(Batch B, double* __restrict__ ws, double* out, const int32_t* 
   Geo g = geo_of(B, b);
   WsView w = ws_view(ws, g, B.ni, B.ld);
   double* o = out ? out + g.z0 * B.ni * B.ld : w.inv;
-  dmma_factor_atmosphere<NT, DPF>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn, with_rhs ? w.rmod : nullptr, tr != 0,
+  dmma_factor_atmosphere<NT, DPF, MB == 1>(g.nz, B.ni, B.ld, w.inv, o, w.supn, w.subn, with_rhs ? w.rmod : nullptr, tr != 0,
                                   status + b, smem_raw, wlim);
 }
 
