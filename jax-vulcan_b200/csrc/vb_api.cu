@@ -150,75 +150,86 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
     coef_id[bits] = id;
     return id;
   };
-  std::vector<uint32_t> lw(le.size()), pw(pe.size()), jw(je.size());
-  for (size_t e = 0; e < le.size(); ++e) lw[e] = vb::term_word(le[e] / T, cid_of(r_st[le[e]]));
-  for (size_t e = 0; e < pe.size(); ++e) pw[e] = vb::term_word(pe[e] / T, cid_of(p_st[pe[e]]));
-  for (size_t e = 0; e < je.size(); ++e) {
-    int fe = je[e], s = fe % T, ro = fe / T, o = ro % (2 * T), r = ro / (2 * T);
-    double c = o < T ? -r_st[(int64_t)r * T + o] : p_st[(int64_t)r * T + (o - T)];
-    jw[e] = vb::term_word(r * T + s, cid_of(c));
-  }
+  for (size_t e = 0; e < le.size(); ++e) cid_of(r_st[le[e]]);
+  for (size_t e = 0; e < pe.size(); ++e) cid_of(p_st[pe[e]]);
+  auto jac_coef = [&](int32_t fe) {
+    const int ro = fe / T, o = ro % (2 * T), r = ro / (2 * T);
+    return o < T ? -r_st[(int64_t)r * T + o] : p_st[(int64_t)r * T + (o - T)];
+  };
+  for (size_t e = 0; e < je.size(); ++e) cid_of(jac_coef(je[e]));
   if (too_many) return fail(VB_ERR_ARG, "more than 256 distinct stoichiometric coefficients");
   if (coefs.empty()) coefs.push_back(0.0);
-  // destinations in decreasing term count (ties: increasing index); threads
-  // take them in rank bands (thread t: ranks t, t + LAYER_THREADS, ...) so the
-  // lanes of a warp sum lists of similar length. The term words of each group
-  // of 32 consecutive ranks are interleaved: term i of rank q at
-  // base(q / 32) + 32 i + q % 32, the group padded to its longest list (the
-  // first rank's), so a warp holding a group loads one line per term.
-  // Descriptor of rank q: its first word, then count | row << 16 | col << 24
-  // (one load per destination).
-  std::vector<uint32_t> order(2 * (size_t)ni * ni), jwi;
-  {
-    const size_t nd = (size_t)ni * ni;
-    std::vector<int32_t> perm(nd);
-    for (size_t d = 0; d < nd; ++d) perm[d] = (int32_t)d;
-    std::stable_sort(perm.begin(), perm.end(),
-                     [&](int32_t x, int32_t y) { return jp[x + 1] - jp[x] > jp[y + 1] - jp[y]; });
-    std::vector<size_t> gbase((nd + 31) / 32 + 1, 0);
-    for (size_t g = 0; g + 1 < gbase.size(); ++g) {
-      const int32_t d = perm[32 * g];
-      gbase[g + 1] = gbase[g] + 32 * (size_t)(jp[d + 1] - jp[d]);
+  bool packed = true;
+  for (const auto& c : coef_id) packed = packed && (c.first & 0xffffffffffffull) == 0;
+  auto code_of = [&](double c) {
+    uint64_t bits;
+    std::memcpy(&bits, &c, sizeof bits);
+    return packed ? (int)(bits >> 48) : coef_id[bits];
+  };
+  std::vector<uint32_t> lw(le.size()), pw(pe.size()), jw(je.size());
+  if (lp.back())
+    for (size_t e = 0; e < le.size(); ++e) lw[e] = vb::term_word(le[e] / T, code_of(r_st[le[e]]));
+  if (pp.back())
+    for (size_t e = 0; e < pe.size(); ++e) pw[e] = vb::term_word(pe[e] / T, code_of(p_st[pe[e]]));
+  if (jp.back())
+    for (size_t e = 0; e < je.size(); ++e) {
+      const int fe = je[e], s = fe % T, r = fe / (2 * T * T);
+      jw[e] = vb::term_word(r * T + s, code_of(jac_coef(fe)));
     }
-    if (gbase.back() > 0xffffffffu) return fail(VB_ERR_ARG, "Jacobian gather table too large");
-    jwi.assign(std::max<size_t>(gbase.back(), 1), 0u);
-    for (size_t q = 0; q < nd; ++q) {
-      const uint32_t d = (uint32_t)perm[q];
-      const uint32_t cnt = (uint32_t)(jp[d + 1] - jp[d]);
-      if (cnt > 0xffffu) return fail(VB_ERR_ARG, "a Jacobian entry has more than 65535 terms");
-      const size_t first = gbase[q / 32] + q % 32;
-      for (uint32_t i = 0; i < cnt; ++i) jwi[first + 32 * (size_t)i] = jw[jp[d] + i];
-      order[2 * q] = (uint32_t)first;
-      order[2 * q + 1] = cnt | ((d / (uint32_t)ni) << 16) | ((d % (uint32_t)ni) << 24);
+  // groups of 32 lists of falling term count (ties: increasing index)
+  std::vector<uint32_t> gbase{0u}, gdesc, gw;
+  auto add_lists = [&](std::vector<uint32_t> ids, auto len, auto word, auto tag) {
+    std::stable_sort(ids.begin(), ids.end(), [&](uint32_t x, uint32_t y) { return len(x) > len(y); });
+    for (size_t q0 = 0; q0 < ids.size(); q0 += 32) {
+      const size_t first = gw.size(), most = len(ids[q0]);
+      gw.resize(first + 32 * most, 0u);
+      for (size_t q = q0; q < q0 + 32; ++q) {
+        const bool on = q < ids.size();
+        const size_t c = on ? len(ids[q]) : 0;
+        for (size_t i = 0; i < c; ++i) gw[first + 32 * i + (q - q0)] = word(ids[q], i);
+        gdesc.push_back(on ? (uint32_t)c | tag(ids[q]) : ~0u);
+      }
+      gbase.push_back((uint32_t)gw.size());
     }
+    return (int)gbase.size() - 1;
+  };
+  auto sum_ptr = [&](uint32_t t) -> const std::vector<int32_t>& { return (t & 1) ? pp : lp; };
+  auto sum_len = [&](uint32_t t) { return (size_t)(sum_ptr(t)[t / 2 + 1] - sum_ptr(t)[t / 2]); };
+  auto jac_len = [&](uint32_t d) { return (size_t)(jp[d + 1] - jp[d]); };
+  std::vector<uint32_t> sums, diag, rest, brief[vb::GL_SHORT + 1];
+  size_t padded = 0;   // a bound of the table's words
+  for (uint32_t t = 0; t < 2 * (uint32_t)ni; ++t) {
+    sums.push_back(t);
+    padded += 32 * sum_len(t);
   }
-  // species lists t = 2 i (loss), 2 i + 1 (production), words interleaved by
-  // groups of 32 consecutive lists (term k of list t at base(t / 32) + 32 k +
-  // t % 32, each group padded to its longest list); descriptor {first, count}
-  std::vector<uint32_t> sdesc(4 * (size_t)ni), swi;
-  {
-    const size_t nl = 2 * (size_t)ni;
-    auto len = [&](size_t t) -> size_t {
-      const std::vector<int32_t>& ptr = (t & 1) ? pp : lp;
-      return (size_t)(ptr[t / 2 + 1] - ptr[t / 2]);
-    };
-    std::vector<size_t> gbase((nl + 31) / 32 + 1, 0);
-    for (size_t g = 0; g + 1 < gbase.size(); ++g) {
-      size_t mx = 0;
-      for (size_t t = 32 * g; t < std::min(nl, 32 * g + 32); ++t) mx = std::max(mx, len(t));
-      gbase[g + 1] = gbase[g] + 32 * mx;
-    }
-    if (gbase.back() > 0xffffffffu) return fail(VB_ERR_ARG, "species gather table too large");
-    swi.assign(std::max<size_t>(gbase.back(), 1), 0u);
-    for (size_t t = 0; t < nl; ++t) {
-      const std::vector<int32_t>& ptr = (t & 1) ? pp : lp;
-      const std::vector<uint32_t>& w = (t & 1) ? pw : lw;
-      const size_t first = gbase[t / 32] + t % 32, n = len(t);
-      for (size_t k = 0; k < n; ++k) swi[first + 32 * k] = w[ptr[t / 2] + k];
-      sdesc[2 * t] = (uint32_t)first;
-      sdesc[2 * t + 1] = (uint32_t)n;
-    }
+  for (uint32_t d = 0; d < (uint32_t)ni * ni; ++d) {
+    const size_t len = jac_len(d);
+    if (len > 0xffffu) return fail(VB_ERR_ARG, "a Jacobian entry has more than 65535 terms");
+    padded += 32 * len;
+    (d / ni == d % ni ? diag : len > vb::GL_SHORT ? rest : brief[len]).push_back(d);
   }
+  if (padded > 0xffffffffu) return fail(VB_ERR_ARG, "Jacobian gather table too large");
+  auto jac_word = [&](uint32_t d, size_t i) { return jw[jp[d] + i]; };
+  auto jac_tag = [&](uint32_t d) { return (d / ni) << 16 | (d % ni) << 23; };
+  const int n_sums = add_lists(sums, sum_len, [&](uint32_t t, size_t i) { return ((t & 1) ? pw : lw)[sum_ptr(t)[t / 2] + i]; },
+                               [&](uint32_t t) { return t << 16; });
+  const int n_diag = add_lists(diag, jac_len, jac_word, jac_tag);
+  const int n_long = add_lists(rest, jac_len, jac_word, jac_tag);
+  int first[vb::GL_SHORT + 1], count[vb::GL_SHORT + 1];
+  for (int c = vb::GL_SHORT, at = n_long; c >= 0; --c) {
+    first[c] = at;
+    at = add_lists(brief[c], jac_len, jac_word, jac_tag);
+    count[c] = at - first[c];
+  }
+  if (gw.empty()) gw.push_back(0u);
+  std::vector<uint64_t> rx(R, 0);
+  if (T <= vb::RX_TERMS)
+    for (int r = 0; r < R; ++r) {
+      rx[r] = three[r] ? 1ull << 60 : 0ull;
+      for (int s = 0; s < T; ++s)
+        rx[r] |= (uint64_t)r_idx[(int64_t)r * T + s] << (8 * s) |
+                 (uint64_t)vb::st_code(r_st[(int64_t)r * T + s]) << (48 + 2 * s);
+    }
   // species lists in natural order (t = 2 i loss, 2 i + 1 production)
   std::vector<int32_t> snp(2 * (size_t)ni + 1, 0);
   std::vector<uint32_t> snw;
@@ -237,10 +248,10 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   std::vector<Part> parts = {
       {ri.data(), ri.size() * 4, 0}, {pi.data(), pi.size() * 4, 0},
       {r_st, (size_t)R * T * 8, 0},  {p_st, (size_t)R * T * 8, 0},
-      {three, (size_t)R, 0},         {sdesc.data(), sdesc.size() * 4, 0},
-      {swi.data(), swi.size() * 4, 0}, {jp.data(), jp.size() * 4, 0},
-      {jwi.data(), jwi.size() * 4, 0}, {coefs.data(), coefs.size() * 8, 0},
-      {order.data(), order.size() * 4, 0}, {snp.data(), snp.size() * 4, 0}, {snw.data(), snw.size() * 4, 0}};
+      {three, (size_t)R, 0},         {gbase.data(), gbase.size() * 4, 0},
+      {gdesc.data(), gdesc.size() * 4, 0}, {gw.data(), gw.size() * 4, 0},
+      {coefs.data(), coefs.size() * 8, 0}, {snp.data(), snp.size() * 4, 0}, {snw.data(), snw.size() * 4, 0},
+      {rx.data(), rx.size() * 8, 0}};
   size_t total = 0;
   for (auto& p : parts) { p.off = total; total += (p.bytes + 255) & ~(size_t)255; }
   void* base = nullptr;
@@ -260,15 +271,22 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   d.r_st = (const double*)(b + parts[2].off);
   d.p_st = (const double*)(b + parts[3].off);
   d.three = (const uint8_t*)(b + parts[4].off);
-  d.sum_desc = (const uint2*)(b + parts[5].off);
-  d.sum_w = (const uint32_t*)(b + parts[6].off);
-  d.jac_ptr = (const int32_t*)(b + parts[7].off);
-  d.jac_w = (const uint32_t*)(b + parts[8].off);
-  d.coef_tab = (const double*)(b + parts[9].off);
+  d.gl_base = (const uint32_t*)(b + parts[5].off);
+  d.gl_desc = (const uint32_t*)(b + parts[6].off);
+  d.gl_w = (const uint32_t*)(b + parts[7].off);
+  d.gl_sums = n_sums;
+  d.gl_diag = n_diag;
+  d.gl_long = n_long;
+  for (int c = 0; c <= vb::GL_SHORT; ++c) {
+    d.gl_first[c] = first[c];
+    d.gl_count[c] = count[c];
+  }
+  d.coef_tab = (const double*)(b + parts[8].off);
   d.n_coef = (int)coefs.size();
-  d.jac_desc = (const uint2*)(b + parts[10].off);
-  d.sum_nptr = (const int32_t*)(b + parts[11].off);
-  d.sum_nw = (const uint32_t*)(b + parts[12].off);
+  d.coef_packed = packed;
+  d.sum_nptr = (const int32_t*)(b + parts[9].off);
+  d.sum_nw = (const uint32_t*)(b + parts[10].off);
+  d.rx = (const uint64_t*)(b + parts[11].off);
   net->base = base;
   net->bytes = total;
   *out = net;

@@ -48,49 +48,136 @@ __device__ inline LayerSmem carve(double* s, int ni, int nr, int T, bool jac, bo
   return L;
 }
 
-// Rate of one reaction from its reactant values yr[] and stoichiometries
-// st[] (padding slots st = 0), and with jac its derivative by each reactant
-// slot into d[], in the reference's expression order (chem.py:92-99,
-// 156-182). Shared by the per-layer and the layer-vectorized assembly.
+// A reaction slot: its reactants' indices, the codes of their
+// stoichiometries st[] (2 bits each; code 3: the value is read), and the
+// three-body flag. One 8-byte word of a table that stays small in L1 for up to
+// RX_TERMS terms; gathered from the wide tables above that.
+struct Slot {
+  uint64_t w;
+  uint32_t codes;
+  const int32_t* idx;
+  const double* st;
+  bool three;
+};
+
 template <int TT>
-__device__ __forceinline__ double rate_terms(const double (&yr)[TT], const double (&st)[TT], double kr, double M,
-                                             bool three, bool jac, double (&d)[TT]) {
+__device__ __forceinline__ Slot load_slot(const NetDev& net, int r) {
+  Slot S;
+  S.idx = net.r_idx + r * TT;
+  S.st = net.r_st + r * TT;
+  if (TT <= RX_TERMS) {
+    S.w = __ldg(net.rx + r);
+    S.codes = (uint32_t)(S.w >> 48);
+    S.three = (S.w >> 60) & 1;
+  } else {
+    S.codes = 0;
+#pragma unroll
+    for (int s = 0; s < TT; ++s) S.codes |= st_code(S.st[s]) << (2 * s);
+    S.three = net.three[r] != 0;
+  }
+  return S;
+}
+
+template <int TT>
+__device__ __forceinline__ int slot_species(const Slot& S, int s) {
+  return TT <= RX_TERMS ? (int)((S.w >> (8 * s)) & 0xff) : S.idx[s];
+}
+
+// Powers by code (pow_st's values): y**st (1 for a padding slot), and
+// st y**(st-1), 0 unless st > 0.
+struct WholePowers {
+  template <int TT>
+  __device__ __forceinline__ static double p(const Slot& S, int s, double y) {
+    const uint32_t c = (S.codes >> (2 * s)) & 3u;
+    return c == 0u ? 1.0 : c == 1u ? y : y * y;
+  }
+  template <int TT>
+  __device__ __forceinline__ static double dp(const Slot& S, int s, double y) {
+    const uint32_t c = (S.codes >> (2 * s)) & 3u;
+    return c == 0u ? 0.0 : c == 1u ? 1.0 : 2.0 * y;
+  }
+};
+struct AnyPowers {
+  template <int TT>
+  __device__ __forceinline__ static double p(const Slot& S, int s, double y) {
+    return S.st[s] > 0.0 ? pow_st(y, S.st[s]) : 1.0;
+  }
+  template <int TT>
+  __device__ __forceinline__ static double dp(const Slot& S, int s, double y) {
+    return S.st[s] * (S.st[s] > 0.0 ? pow_st(y, S.st[s] - 1.0) : 0.0);
+  }
+};
+
+// Rate of one reaction from its reactant values yr[] (padding slots st = 0),
+// and with jac its derivative by each reactant slot into d[], in the
+// reference's expression order (chem.py:92-99, 156-182). Shared by the
+// per-layer and the layer-vectorized assembly.
+template <int TT, class Powers>
+__device__ __forceinline__ double rate_terms_p(const double (&yr)[TT], const Slot& S, double kr, double M, bool jac,
+                                               double (&d)[TT]) {
   double f[TT];
 #pragma unroll
-  for (int s = 0; s < TT; ++s) f[s] = st[s] > 0.0 ? pow_st(yr[s], st[s]) : 1.0;
+  for (int s = 0; s < TT; ++s) f[s] = Powers::template p<TT>(S, s, yr[s]);
   double prod = f[0];
 #pragma unroll
   for (int s = 1; s < TT; ++s) prod = prod * f[s];
   double rt = kr * prod;
-  if (three) rt = rt * M;
+  if (S.three) rt = rt * M;
   if (jac) {
 #pragma unroll
     for (int s = 0; s < TT; ++s) {
       double lo = (s == 0) ? 1.0 : f[0];
 #pragma unroll
       for (int t = 1; t < TT; ++t) lo = lo * ((t == s) ? 1.0 : f[t]);
-      double pm1 = st[s] > 0.0 ? pow_st(yr[s], st[s] - 1.0) : 0.0;
-      double dd = st[s] * pm1;
+      double dd = Powers::template dp<TT>(S, s, yr[s]);
       dd = dd * lo;
       dd = dd * kr;
-      if (three) dd = dd * M;
+      if (S.three) dd = dd * M;
       d[s] = dd;
     }
   }
   return rt;
 }
 
+// A stoichiometry other than 0, 1 and 2 in the slot: out of line, so that pow
+// takes neither registers nor instruction cache from the rest.
+template <int TT>
+__device__ __noinline__ double rate_terms_any(const double* y, Slot S, double kr, double M, bool jac, double* dout) {
+  double yr[TT], d[TT];
+#pragma unroll
+  for (int s = 0; s < TT; ++s) yr[s] = y[s];
+  const double rt = rate_terms_p<TT, AnyPowers>(yr, S, kr, M, jac, d);
+  if (jac) {
+#pragma unroll
+    for (int s = 0; s < TT; ++s) dout[s] = d[s];
+  }
+  return rt;
+}
+
+template <int TT>
+__device__ __forceinline__ double rate_terms(const double (&yr)[TT], const Slot& S, double kr, double M, bool jac,
+                                             double (&d)[TT]) {
+  constexpr uint32_t LOW = 0x5555u & ((1u << (2 * TT)) - 1u);
+  if ((S.codes & (S.codes >> 1) & LOW) == 0) return rate_terms_p<TT, WholePowers>(yr, S, kr, M, jac, d);
+  double y[TT], dd[TT];
+#pragma unroll
+  for (int s = 0; s < TT; ++s) y[s] = yr[s];
+  const double rt = rate_terms_any<TT>(y, S, kr, M, jac, dd);
+  if (jac) {
+#pragma unroll
+    for (int s = 0; s < TT; ++s) d[s] = dd[s];
+  }
+  return rt;
+}
+
 // Rate (and drate) of reaction slot r with TT terms of one layer.
 template <int TT>
-__device__ inline void rate_slot(const NetDev& net, int r, const double* yrow, double kr, double M, double* rate,
+__device__ inline void rate_slot(const Slot& S, int r, const double* yrow, double kr, double M, double* rate,
                                  double* drate, bool jac) {
-  double yr[TT], st[TT], d[TT];
+  double yr[TT], d[TT];
 #pragma unroll
-  for (int s = 0; s < TT; ++s) {
-    st[s] = net.r_st[r * TT + s];
-    yr[s] = yrow[net.r_idx[r * TT + s]];
-  }
-  rate[r] = rate_terms<TT>(yr, st, kr, M, net.three[r] != 0, jac, d);
+  for (int s = 0; s < TT; ++s) yr[s] = yrow[slot_species<TT>(S, s)];
+  rate[r] = rate_terms<TT>(yr, S, kr, M, jac, d);
   if (jac) {
 #pragma unroll
     for (int s = 0; s < TT; ++s) drate[r * TT + s] = d[s];
@@ -105,15 +192,18 @@ __device__ inline void rates_t(const NetDev& net, const double* yrow, const doub
                                double* rate, double* drate, bool jac) {
   for (int r0 = threadIdx.x; r0 <= net.nr; r0 += RU * blockDim.x) {
     double kv[RU];
+    Slot S[RU];
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
       kv[u] = r <= net.nr ? __ldcg(kcol + (int64_t)r * kstride) : 0.0;
+      if (TT <= RX_TERMS) S[u] = load_slot<TT>(net, min(r, net.nr));
     }
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
-      if (r <= net.nr) rate_slot<TT>(net, r, yrow, kv[u], M, rate, drate, jac);
+      if (TT > RX_TERMS && r <= net.nr) S[u] = load_slot<TT>(net, r);
+      if (r <= net.nr) rate_slot<TT>(S[u], r, yrow, kv[u], M, rate, drate, jac);
     }
   }
 }
@@ -146,63 +236,172 @@ __device__ inline void layer_rates(const NetDev& net, const double* yrow, const 
   }
 }
 
-// Loss and production sums of every species, each a sequential gather in
-// segment_sum order (one thread per sum): part[2i] = loss_i, part[2i+1] = prod_i.
-// The caller synchronises before reading dy_i/dt = part[2i+1] - part[2i].
-__device__ inline void species_sums(const NetDev& net, const double* coef, const double* rate, double* part) {
-  for (int t = threadIdx.x; t < 2 * net.ni; t += blockDim.x) {
-    const uint2 d = net.sum_desc[t];
-    double acc = 0.0;
-    const int e1 = (int)d.x + 32 * (int)d.y;
-#pragma unroll 4
-    for (int e = (int)d.x; e < e1; e += 32) {
-      const uint32_t x = net.sum_w[e];
-      acc = acc + coef[x >> 16] * rate[x & 0xffffu];
-    }
-    part[t] = acc;
-  }
-}
-
 // The coefficient table of the gathers into shared memory (coef[MAX_COEF]).
 __device__ inline void load_coefs(const NetDev& net, double* coef) {
+  if (net.coef_packed) return;
   for (int c = threadIdx.x; c < net.n_coef; c += blockDim.x) coef[c] = net.coef_tab[c];
 }
 
-// Dense Jacobian of one layer (chem.py:183-208), each entry summed in the
-// reference's scatter order. Threads take the destinations in rank bands of
-// decreasing term count (jac_desc), so the lanes of a warp run loops of
-// similar length; the terms of 32 consecutive ranks are interleaved in
-// jac_w (term i of a rank at its first word + 32 i), so a warp whose lanes
-// hold one such group reads one 128-byte line per term.
-// busy: the first threads are also summing species lists in the same phase;
-// the rank bands are rotated (by whole warps, keeping the groups aligned) so
-// those threads take the lightest ranks of each band.
-__device__ inline int warp_rotation(int busy) { return (busy + 31) & ~31; }
+// Coefficient of a term word: its own upper half (PK) or the table's entry.
+template <bool PK>
+__device__ __forceinline__ double term_coef(const double* coef, uint32_t x) {
+  return PK ? __hiloint2double((int)(x & 0xffff0000u), 0) : coef[x >> 16];
+}
 
-template <typename Store>
-__device__ inline void layer_jacobian_each(const NetDev& net, const double* coef, const double* drate, Store store,
-                                           int busy = 0) {
-  const int nd = net.ni * net.ni;
-  const int stride = blockDim.x;
-  int q = ((int)threadIdx.x - warp_rotation(busy) % stride + stride) % stride;
-  uint2 dn = q < nd ? net.jac_desc[q] : make_uint2(0u, 0u);
-  for (; q < nd; q += stride) {
-    const uint2 dc = dn;
-    if (q + stride < nd) dn = net.jac_desc[q + stride];   // the next destination's descriptor, one ahead
-    const int e0 = (int)dc.x, e1 = e0 + 32 * (int)(dc.y & 0xffffu);
-    double J = 0.0;
-#pragma unroll 4
-    for (int e = e0; e < e1; e += 32) {
-      const uint32_t x = net.jac_w[e];
-      J = J + coef[x >> 16] * drate[x & 0xffffu];
+constexpr int GW = 8;   // term words of a list held ahead by a lane
+
+// Words k .. of a group (wp: the lane's first word) that exist.
+__device__ __forceinline__ void group_words(const uint32_t* wp, int len, uint32_t (&w)[GW]) {
+#pragma unroll
+  for (int u = 0; u < GW; ++u) w[u] = u < len ? __ldg(wp + 32 * u) : 0u;
+}
+
+// Sum of a lane's list of cnt terms, in list order; len: the group's longest.
+// w holds the first GW words; each half is reloaded GW terms ahead as it is used.
+template <bool PK>
+__device__ __forceinline__ double gather_list(const double* coef, const double* src, const uint32_t* wp, int len,
+                                              int cnt, uint32_t (&w)[GW]) {
+  constexpr int H = GW / 2;
+  double acc = 0.0;
+  for (int k = 0; k < len; k += GW) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k0 = k + h * H;
+      if (k0 >= len) break;
+      double v[H], c[H];
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        v[u] = src[w[h * H + u] & 0xffffu];
+        c[u] = term_coef<PK>(coef, w[h * H + u]);
+      }
+#pragma unroll
+      for (int u = 0; u < H; ++u) w[h * H + u] = k0 + GW + u < len ? __ldg(wp + 32 * (k0 + GW + u)) : 0u;
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        const double t = acc + c[u] * v[u];
+        if (k0 + u < cnt) acc = t;
+      }
     }
-    store((int)((dc.y >> 16) & 0xffu), (int)(dc.y >> 24), J);
+  }
+  return acc;
+}
+
+// A long group's lane sum.
+template <bool PK>
+__device__ __forceinline__ double gather_group(const NetDev& net, const double* coef, const double* src, int g,
+                                               uint32_t desc) {
+  const uint32_t b0 = net.gl_base[g], b1 = net.gl_base[g + 1];
+  const int len = (int)(b1 - b0) / 32;
+  const uint32_t* wp = net.gl_w + b0 + (threadIdx.x & 31);
+  uint32_t w[GW];
+  group_words(wp, len, w);
+  return gather_list<PK>(coef, src, wp, len, (int)(desc & 0xffffu), w);
+}
+
+// GB groups of entries of exactly C terms each, from group g (n of them
+// exist): all words first, so the table's latency is paid once.
+constexpr int GB = 4;
+template <int C, bool PK, typename Off>
+__device__ __forceinline__ void gather_short(const NetDev& net, const double* coef, const double* drate, int g, int n,
+                                             Off off) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t* wp = net.gl_w + net.gl_base[net.gl_first[C]] + 32 * C * (g - net.gl_first[C]) + lane;
+  uint32_t desc[GB], w[GB][C ? C : 1];
+#pragma unroll
+  for (int q = 0; q < GB; ++q) {
+    desc[q] = q < n ? __ldg(net.gl_desc + 32 * (g + q) + lane) : ~0u;
+#pragma unroll
+    for (int u = 0; u < C; ++u) w[q][u] = q < n ? __ldg(wp + 32 * (C * q + u)) : 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < GB; ++q) {
+    double J = 0.0;
+#pragma unroll
+    for (int u = 0; u < C; ++u) J = J + term_coef<PK>(coef, w[q][u]) * drate[w[q][u] & 0xffffu];
+    if (desc[q] != ~0u) off((int)((desc[q] >> 16) & 0x7fu), (int)(desc[q] >> 23), J);
   }
 }
 
-__device__ inline void layer_jacobian(const NetDev& net, const double* coef, const double* drate, double* jac) {
-  const int ni = net.ni;
-  layer_jacobian_each(net, coef, drate, [&](int row, int col, double J) { jac[row * ni + col] = J; });
+// The gathers of one layer: the species lists' sums to part[t] (sums), the
+// Jacobian's diagonal entries to diag(row, J), the others to off(row, col, J),
+// each in the reference's order. The warps take work from a queue in shared
+// memory (zeroed before the barrier ahead of this), the long groups first and
+// one by one, then the short ones GB at a time, so they finish together. What
+// bounds this is instructions issued and shared-memory wavefronts, not the
+// latency of the tables: hence exact code for the short lists (three quarters
+// of the entries), the diagonal's extra terms out of the common path, and the
+// coefficient in the word.
+template <bool PK, typename Diag, typename Off>
+__device__ __forceinline__ void gather_layer_t(const NetDev& net, const double* coef, const double* rate,
+                                               const double* drate, bool sums, int* queue, double* part, Diag diag,
+                                               Off off) {
+  const int lane = threadIdx.x & 31;
+  const int g0 = sums ? 0 : net.gl_sums;
+  while (true) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(queue, 1);
+    g = g0 + __shfl_sync(0xffffffffu, g, 0);
+    if (g < net.gl_long) {
+      const uint32_t desc = net.gl_desc[32 * g + lane];
+      const bool on = desc != ~0u;
+      const double acc = gather_group<PK>(net, coef, g < net.gl_sums ? rate : drate, g, on ? desc : 0u);
+      if (!on) continue;
+      const int row = (int)((desc >> 16) & 0x7fu);
+      if (g < net.gl_sums)
+        part[desc >> 16] = acc;
+      else if (g < net.gl_diag)
+        diag(row, acc);
+      else
+        off(row, (int)(desc >> 23), acc);
+      continue;
+    }
+    g -= net.gl_long;
+    int c = GL_SHORT;
+    for (; c >= 0; --c) {
+      const int nb = (net.gl_count[c] + GB - 1) / GB;
+      if (g < nb) break;
+      g -= nb;
+    }
+    if (c < 0) break;
+    const int n = net.gl_count[c] - GB * g;
+    g = net.gl_first[c] + GB * g;
+    switch (c) {
+      case 4: gather_short<4, PK>(net, coef, drate, g, n, off); break;
+      case 3: gather_short<3, PK>(net, coef, drate, g, n, off); break;
+      case 2: gather_short<2, PK>(net, coef, drate, g, n, off); break;
+      case 1: gather_short<1, PK>(net, coef, drate, g, n, off); break;
+      default: gather_short<0, PK>(net, coef, drate, g, n, off); break;
+    }
+  }
+}
+
+template <typename Diag, typename Off>
+__device__ __forceinline__ void gather_layer(const NetDev& net, const double* coef, const double* rate,
+                                             const double* drate, bool sums, int* queue, double* part, Diag diag,
+                                             Off off) {
+  if (net.coef_packed)
+    gather_layer_t<true>(net, coef, rate, drate, sums, queue, part, diag, off);
+  else
+    gather_layer_t<false>(net, coef, rate, drate, sums, queue, part, diag, off);
+}
+
+// Loss and production sums of every species: part[2i] = loss_i, part[2i+1] =
+// prod_i. The caller synchronises before reading dy_i/dt = part[2i+1] - part[2i].
+template <bool PK>
+__device__ __forceinline__ void species_sums_t(const NetDev& net, const double* coef, const double* rate,
+                                               double* part) {
+  for (int g = (int)threadIdx.x / 32; g < net.gl_sums; g += (int)blockDim.x / 32) {
+    const uint32_t desc = net.gl_desc[32 * g + (threadIdx.x & 31)];
+    const double acc = gather_group<PK>(net, coef, rate, g, desc == ~0u ? 0u : desc);
+    if (desc != ~0u) part[desc >> 16] = acc;
+  }
+}
+
+__device__ inline void species_sums(const NetDev& net, const double* coef, const double* rate, double* part) {
+  if (net.coef_packed)
+    species_sums_t<true>(net, coef, rate, part);
+  else
+    species_sums_t<false>(net, coef, rate, part);
 }
 
 // Loads state rows j-1..j+1 (stage 2: yk2 = y + k1/r) and their gas sums.
@@ -313,9 +512,14 @@ __device__ inline void layer_diffusion(const AtmRef& a, int nz, int ni, int j, i
 
 // Stage-1 assembly: rmod[j] = rhs(y), inv[j] = c0*I - J - diag(diag_d),
 // supn[j] = -sup_d, subn[j-1] = -sub_d, with fix_mask (jax_step.py:263-298).
-// Latency-bound gathers: four CTAs per SM (the shared-memory limit with the
-// drate buffer) beat three without spills (measured on B200, ni=69, nr=1400:
-// 4.79 vs 4.89 ms at 296 atmospheres; two per SM: 6.32 ms).
+// Four CTAs per SM, the shared-memory limit with the drate buffer (three,
+// without spills, were slower when the gathers were latency-bound). Measured
+// on B200, ni=69, nr=1400, nz=120, 296 atmospheres, with the diffusion rows:
+// 2.71 ms with the lists dealt out in fixed bands, coefficients in a table and
+// pow in line (681 M instructions in a ragged batch of 85, issue slots 70 %
+// busy); 2.92 with the queue alone; 2.46 with exact code for the short lists
+// and packed reaction words (406 M); 2.35 with pow out of line. What is left
+// is the wavefronts of the scattered shared-memory reads.
 __global__ void __launch_bounds__(LAYER_THREADS, 4)
 stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
               const double* __restrict__ dt, const double* __restrict__ atm, int flags,
@@ -335,6 +539,8 @@ stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   const double c0 = adj ? 0.0 : 1.0 / (r * dt[b]);
 
   __shared__ double coefs[MAX_COEF];
+  __shared__ int queue;
+  if (threadIdx.x == 0) queue = 0;
   load_coefs(net, coefs);
   // state row j (the rates; padding slot 1.0) and diag_d of row j, written
   // with the row's diffusion terms by diffusion_rows_kernel ahead of this kernel
@@ -344,39 +550,42 @@ stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   __syncthreads();
   layer_rates(net, yj, k + g.z0 * (B.nr + 1) + j, nz, a.M[j], L.rate, L.drate, true);
   __syncthreads();
-  // One phase for the species sums and the Jacobian gather: the first 2*ni
-  // threads sum a species list, then join the gather on the light end of
-  // each rank band. The gather writes each block entry in its final form.
-  if (!adj) species_sums(net, coefs, L.rate, L.part);
+  // One phase for the species sums and the Jacobian gather. The gather writes
+  // each block entry in its final form.
   double* blk = w.inv + (int64_t)j * ni * B.ld;
   const int ld = B.ld;
   const double bot = (j == 0 && (flags & VB_USE_BOTFLUX)) ? 1.0 : 0.0;
   if (adj) {
     // steady_state_grad.py:153-175: diag = J + diag(A_eddy + A_mol) (+ deposition
-    // at the bottom), sup_d = B[:-1], sub_d = C[1:] (no c0, not negated)
-    layer_jacobian_each(net, coefs, L.drate, [&](int row, int col, double J) {
-      double v = J;
-      if (row == col) {
-        v = v + L.diagd[row];
-        if (j == 0) v = v + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
-      }
-      blk[(int64_t)row * ld + col] = v;
-    });
+    // at the bottom), sup_d = B[:-1], sub_d = C[1:] (no c0, not negated); no sums
+    gather_layer(
+        net, coefs, L.rate, L.drate, false, &queue, L.part,
+        [&](int row, double J) {
+          double v = J + L.diagd[row];
+          if (j == 0) v = v + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
+          blk[(int64_t)row * ld + row] = v;
+        },
+        [&](int row, int col, double J) { blk[(int64_t)row * ld + col] = J; });
     for (int i = threadIdx.x; i < ni; i += blockDim.x)
       w.rmod[(int64_t)j * ni + i] = adj_v[g.z0 * ni + (int64_t)j * ni + i];
     return;
   }
-  layer_jacobian_each(net, coefs, L.drate, [&](int row, int col, double J) {
-    double v = (row == col ? c0 : 0.0) - J;
-    if (row == col) {
-      // jax_step.py:283,288: the deposition term joins diag_d before -diag_d is added
-      double dd = L.diagd[row];
-      if (j == 0) dd = dd + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
-      v = v + (-dd);
-    }
-    if (fm && fm[row]) v = (row == col) ? c0 : 0.0;
-    blk[(int64_t)row * ld + col] = v;
-  }, min(2 * ni, (int)blockDim.x));
+  gather_layer(
+      net, coefs, L.rate, L.drate, true, &queue, L.part,
+      [&](int row, double J) {
+        double v = c0 - J;
+        // jax_step.py:283,288: the deposition term joins diag_d before -diag_d is added
+        double dd = L.diagd[row];
+        if (j == 0) dd = dd + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
+        v = v + (-dd);
+        if (fm && fm[row]) v = c0;
+        blk[(int64_t)row * ld + row] = v;
+      },
+      [&](int row, int col, double J) {
+        double v = 0.0 - J;
+        if (fm && fm[row]) v = 0.0;
+        blk[(int64_t)row * ld + col] = v;
+      });
   __syncthreads();   // the species sums
   for (int i = threadIdx.x; i < ni; i += blockDim.x) {
     // rmod[j] holds the row's diffusion term (diffusion_rows_kernel)
@@ -443,8 +652,8 @@ __device__ inline void rates_pair_t(const NetDev& net, const double* y0, const d
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
       if (r < R) {
-        rate_slot<TT>(net, r, y0, kv[u][0], M0, rate, drate, true);
-        if (two) rate_slot<TT>(net, r, y1, kv[u][1], M1, rate + R, drate + (int64_t)R * TT, true);
+        rate_slot<TT>(load_slot<TT>(net, r), r, y0, kv[u][0], M0, rate, drate, true);
+        if (two) rate_slot<TT>(load_slot<TT>(net, r), r, y1, kv[u][1], M1, rate + R, drate + (int64_t)R * TT, true);
       }
     }
   }
@@ -464,49 +673,56 @@ __device__ inline void rates_pair(const NetDev& net, const double* y0, const dou
   }
 }
 
+// Sums of a lane's list for both layers (off: the second layer's rates or drates).
+template <bool PK>
+__device__ __forceinline__ void gather_pair(const double* coef, const double* src, int64_t off, const uint32_t* wp,
+                                            int cnt, double& a0, double& a1) {
+  a0 = 0.0;
+  a1 = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
+    const uint32_t x = wp[32 * k];
+    const double c = term_coef<PK>(coef, x);
+    const int s = x & 0xffffu;
+    a0 = a0 + c * src[s];
+    a1 = a1 + c * src[off + s];
+  }
+}
+
+__device__ __forceinline__ void gather_pair_any(const NetDev& net, const double* coef, const double* src, int64_t off,
+                                                int q, double& a0, double& a1) {
+  const uint32_t* wp = net.gl_w + net.gl_base[q >> 5] + (q & 31);
+  const int cnt = (int)(net.gl_desc[q] & 0xffffu);
+  if (net.coef_packed)
+    gather_pair<true>(coef, src, off, wp, cnt, a0, a1);
+  else
+    gather_pair<false>(coef, src, off, wp, cnt, a0, a1);
+}
+
 // Loss and production sums of both layers (species_sums' order per layer).
 __device__ inline void species_sums_pair(const NetDev& net, const double* coef, const double* rate, double* part) {
-  const int R = net.nr + 1;
-  for (int t = threadIdx.x; t < 2 * net.ni; t += blockDim.x) {
-    const uint2 d = net.sum_desc[t];
-    double a0 = 0.0, a1 = 0.0;
-    const int e1 = (int)d.x + 32 * (int)d.y;
-#pragma unroll 4
-    for (int e = (int)d.x; e < e1; e += 32) {
-      const uint32_t x = net.sum_w[e];
-      const double c = coef[x >> 16];
-      const int s = x & 0xffffu;
-      a0 = a0 + c * rate[s];
-      a1 = a1 + c * rate[R + s];
-    }
+  for (int q = threadIdx.x; q < 2 * net.ni; q += blockDim.x) {
+    double a0, a1;
+    gather_pair_any(net, coef, rate, net.nr + 1, q, a0, a1);
+    const int t = (int)(net.gl_desc[q] >> 16);
     part[t] = a0;
     part[2 * net.ni + t] = a1;
   }
 }
 
-// Dense Jacobians of both layers (layer_jacobian_each's order and rank bands).
+// Dense Jacobians of both layers, the entries in bands of falling term count.
+// busy: threads that summed species lists just before; the bands are rotated
+// (by whole warps) so those take the lightest entries of each band.
 template <typename Store>
 __device__ inline void jacobian_pair(const NetDev& net, const double* coef, const double* drate, Store store,
                                      int busy) {
-  const int nd = net.ni * net.ni;
-  const int64_t D = (int64_t)(net.nr + 1) * net.T;
-  const int stride = blockDim.x;
-  int q = ((int)threadIdx.x - warp_rotation(busy) % stride + stride) % stride;
-  uint2 dn = q < nd ? net.jac_desc[q] : make_uint2(0u, 0u);
-  for (; q < nd; q += stride) {
-    const uint2 dc = dn;
-    if (q + stride < nd) dn = net.jac_desc[q + stride];
-    const int e0 = (int)dc.x, e1 = e0 + 32 * (int)(dc.y & 0xffffu);
-    double J0 = 0.0, J1 = 0.0;
-#pragma unroll 4
-    for (int e = e0; e < e1; e += 32) {
-      const uint32_t x = net.jac_w[e];
-      const double c = coef[x >> 16];
-      const int s = x & 0xffffu;
-      J0 = J0 + c * drate[s];
-      J1 = J1 + c * drate[D + s];
-    }
-    store((int)((dc.y >> 16) & 0xffu), (int)(dc.y >> 24), J0, J1);
+  const int q0 = 32 * net.gl_sums, nq = 32 * (net.gl_first[0] + net.gl_count[0]) - q0, stride = blockDim.x;
+  for (int q = ((int)threadIdx.x - ((busy + 31) & ~31) % stride + stride) % stride; q < nq; q += stride) {
+    const uint32_t d = net.gl_desc[q0 + q];
+    if (d == ~0u) continue;
+    double J0, J1;
+    gather_pair_any(net, coef, drate, (int64_t)(net.nr + 1) * net.T, q0 + q, J0, J1);
+    store((int)((d >> 16) & 0x7fu), (int)(d >> 23), J0, J1);
   }
 }
 
@@ -528,8 +744,8 @@ __device__ inline void rates_pair_rhs_t(const NetDev& net, const double* y0, con
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
       if (r < R) {
-        rate_slot<TT>(net, r, y0, kv[u][0], M0, rate, nullptr, false);
-        if (two) rate_slot<TT>(net, r, y1, kv[u][1], M1, rate + R, nullptr, false);
+        rate_slot<TT>(load_slot<TT>(net, r), r, y0, kv[u][0], M0, rate, nullptr, false);
+        if (two) rate_slot<TT>(load_slot<TT>(net, r), r, y1, kv[u][1], M1, rate + R, nullptr, false);
       }
     }
   }
@@ -777,14 +993,20 @@ chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __re
   LayerSmem L = carve(smem, ni, net.nr, net.T, want_jac, want_jac);
   const double* yrow = y + ((int64_t)b * nz + j) * ni;
   __shared__ double coefs[MAX_COEF];
+  __shared__ int queue;
+  if (threadIdx.x == 0) queue = 0;
   load_coefs(net, coefs);
   for (int i = threadIdx.x; i <= ni; i += blockDim.x) L.y3[i] = i < ni ? yrow[i] : 1.0;
   __syncthreads();
   layer_rates(net, L.y3, k + (int64_t)b * (net.nr + 1) * nz + j, nz, M[(int64_t)b * nz + j], L.rate,
               L.drate, want_jac);
   __syncthreads();
-  species_sums(net, coefs, L.rate, L.part);
-  if (want_jac) layer_jacobian(net, coefs, L.drate, L.jac);
+  if (want_jac)
+    gather_layer(
+        net, coefs, L.rate, L.drate, true, &queue, L.part, [&](int row, double J) { L.jac[row * ni + row] = J; },
+        [&](int row, int col, double J) { L.jac[row * ni + col] = J; });
+  else
+    species_sums(net, coefs, L.rate, L.part);
   __syncthreads();
   if (dydt)
     for (int i = threadIdx.x; i < ni; i += blockDim.x)
@@ -965,7 +1187,7 @@ __host__ __device__ inline size_t lv_rates_smem_bytes(int ni) {
 }
 
 template <int TT>
-__global__ void __launch_bounds__(LV_RATE_THREADS)
+__global__ void __launch_bounds__(LV_RATE_THREADS, 2)
 lv_rates_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
                 const double* __restrict__ atm, double* __restrict__ ws) {
   extern __shared__ double smem[];
@@ -1007,13 +1229,11 @@ lv_rates_kernel(NetDev net, Batch B, const double* __restrict__ y, const double*
       for (int u = 0; u < RU; ++u) {
         const int rr = r0 + u * ngrp;
         if (rr < r_hi) {
-          double yr[TT], st[TT], d[TT];
+          const Slot sl = load_slot<TT>(net, rr);
+          double yr[TT], d[TT];
 #pragma unroll
-          for (int s = 0; s < TT; ++s) {
-            st[s] = net.r_st[rr * TT + s];
-            yr[s] = yT[net.r_idx[rr * TT + s] * S + zl];
-          }
-          const double rt = rate_terms<TT>(yr, st, kv[u], M, net.three[rr] != 0, false, d);
+          for (int s = 0; s < TT; ++s) yr[s] = yT[slot_species<TT>(sl, s) * S + zl];
+          const double rt = rate_terms<TT>(yr, sl, kv[u], M, false, d);
           if (on) rate[(int64_t)rr * nzb + z] = rt;
         }
       }
@@ -1041,10 +1261,18 @@ lv_sums_kernel(NetDev net, Batch B, const double* __restrict__ dt, const uint8_t
     for (int t = 0; t < 2; ++t) {
       const int e0 = net.sum_nptr[2 * i + t], e1 = net.sum_nptr[2 * i + t + 1];
       double acc = 0.0;
+      if (net.coef_packed) {
 #pragma unroll 8
-      for (int e = e0; e < e1; ++e) {
-        const uint32_t x = net.sum_nw[e];
-        acc = acc + coefs[x >> 16] * rate[(int64_t)(x & 0xffffu) * nzb + z];
+        for (int e = e0; e < e1; ++e) {
+          const uint32_t x = net.sum_nw[e];
+          acc = acc + term_coef<true>(coefs, x) * rate[(int64_t)(x & 0xffffu) * nzb + z];
+        }
+      } else {
+#pragma unroll 8
+        for (int e = e0; e < e1; ++e) {
+          const uint32_t x = net.sum_nw[e];
+          acc = acc + term_coef<false>(coefs, x) * rate[(int64_t)(x & 0xffffu) * nzb + z];
+        }
       }
       part[t] = acc;
     }

@@ -7,6 +7,15 @@
 
 namespace vb {
 
+constexpr int GL_SHORT = 4;   // longest Jacobian list with code of its own
+constexpr int RX_TERMS = 6;   // reactant slots that fit a packed reaction word
+
+// Code of a stoichiometry: 0, 1, 2, or 3 for any other value.
+__host__ __device__ __forceinline__ uint32_t st_code(double st) {
+  return st == 0.0 ? 0u : st == 1.0 ? 1u : st == 2.0 ? 2u : 3u;
+}
+
+
 // Device-resident network tables (reference chem.py:28-80 plus gather tables).
 struct NetDev {
   int ni, nr, T;                 // species, reaction slots (rows nr+1), max_terms
@@ -15,29 +24,36 @@ struct NetDev {
   const double* r_st;            // [nr+1][T]
   const double* p_st;            // [nr+1][T]
   const uint8_t* three;          // [nr+1]
+  // Reaction slot in one word (T <= RX_TERMS): reactant index s in byte s, its
+  // stoichiometry's code (st_code) at bits 48 + 2 s, the three-body flag at bit 60.
+  const uint64_t* rx;            // [nr+1]
   // Gather tables, one 32-bit word per term: the low 16 bits index a rate
-  // (loss / prod: reaction r) or a drate slot (Jacobian: r*T+s), the high 16
-  // bits a coefficient in coef_tab (the distinct stoichiometries, <= 256).
-  // RHS: list t = 2 i (loss) or 2 i + 1 (production) of species i, the
-  // (r*T+s) slots whose reactant (loss) or product index is i, in increasing
-  // flat order (segment_sum order); the coefficient is r_st[r*T+s] or
-  // p_st[r*T+s]. The words of each group of 32 consecutive lists are
-  // interleaved (term k of list t at its first word + 32 k), so the lanes of
-  // a warp summing lists t = 32 g .. 32 g + 31 load one line per term.
-  const uint2* sum_desc;         // [2 ni]: {first word in sum_w, term count}
-  const uint32_t* sum_w;
-  // Jacobian: for destination d = row*ni+col, the contributions (r, o, s) in
-  // increasing flat order (r*2T + o)*T + s (chem.py:193-207 scatter order);
-  // the coefficient is -r_st[r][o] (o < T) or p_st[r][o-T]. jac_ptr is the
-  // CSR of that order; jac_w holds the words interleaved by groups of 32
-  // consecutive ranks of jac_desc (term i of a rank at its first word + 32 i).
-  const int32_t* jac_ptr;        // [ni*ni+1]
-  const uint32_t* jac_w;
+  // (species lists: reaction r) or a drate slot (Jacobian: r*T+s), the high 16
+  // bits give the coefficient: the top half of the double's high word where
+  // every coefficient of the network is zero below it (coef_packed; whole and
+  // half stoichiometries are), else its id in coef_tab (<= 256 distinct ones).
+  // The lists, in groups of 32 of falling term count (ties: increasing index):
+  // * the 2 ni species lists, t = 2 i (loss) or 2 i + 1 (production) of
+  //   species i: the (r*T+s) slots whose reactant (loss) or product index is
+  //   i, in increasing flat order (segment_sum order), with r_st or p_st;
+  // * the ni*ni Jacobian entries: the contributions (r, o, s) in increasing
+  //   flat order (r*2T + o)*T + s (chem.py:193-207 scatter order), with
+  //   -r_st[r][o] (o < T) or p_st[r][o-T].
+  // Groups [0, gl_sums) hold the species lists, [gl_sums, gl_diag) the
+  // diagonal entries, [gl_diag, gl_long) the off-diagonal entries of more than
+  // GL_SHORT terms, and [gl_first[c], gl_first[c] + gl_count[c]) those of
+  // exactly c <= GL_SHORT terms (the last group of each kind padded with
+  // lanes whose descriptor is ~0). The words of a group are interleaved and
+  // padded (with 0) to its longest list: term k of lane l of group g at
+  // gl_w[gl_base[g] + 32 k + l], so a warp that holds a group loads one line
+  // per term.
+  const uint32_t* gl_base;       // [groups + 1]
+  const uint32_t* gl_desc;       // [32 groups]: count | t << 16, or count | row << 16 | col << 23
+  const uint32_t* gl_w;
+  int gl_sums, gl_diag, gl_long;
+  int gl_first[GL_SHORT + 1], gl_count[GL_SHORT + 1];
   const double* coef_tab;        // [n_coef]
-  int n_coef;
-  // Destinations in decreasing term count: {first term in jac_w,
-  // count | row << 16 | col << 24}.
-  const uint2* jac_desc;         // [ni*ni]
+  int n_coef, coef_packed;
   // The species lists in natural order, for the layer-vectorized stage 2
   // (one thread per layer, every term of a list read by the whole warp):
   // list t (2 i loss, 2 i + 1 production) at sum_nw[sum_nptr[t] .. sum_nptr[t+1]).
@@ -48,9 +64,10 @@ struct NetDev {
 constexpr int LAYER_THREADS = 256;
 constexpr int MAX_COEF = 256;   // distinct stoichiometric coefficients of a network
 
-// Term word of a gather table: index (low 16 bits) and coefficient id.
-__host__ __device__ __forceinline__ uint32_t term_word(int idx, int cid) {
-  return (uint32_t)idx | ((uint32_t)cid << 16);
+// Term word of a gather table: index (low 16 bits) and the coefficient's
+// high half-word or id.
+__host__ __device__ __forceinline__ uint32_t term_word(int idx, int code) {
+  return (uint32_t)idx | ((uint32_t)code << 16);
 }
 
 // Offsets (in doubles) of the fields of one atmosphere in the atm blob.
