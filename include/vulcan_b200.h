@@ -96,7 +96,8 @@ int vb_net_destroy(VbNet* net);
  *                  the other half's factor; 0 or 1 = one stream
  *   stage1_layers: layers per CTA of the stage-1 and stage-2 assembly, 1 or
  *                  2 (two share every gather-table word and rate-constant
- *                  sector; 0 = the default, 1) */
+ *                  sector; 0 = by size in stage 1, thread-per-layer or 1 in
+ *                  stage 2) */
 typedef struct VbTuning {
   int32_t factor_kernel, factor_ctas, sweep_stages, streams, stage1_layers, reserved;
 } VbTuning;

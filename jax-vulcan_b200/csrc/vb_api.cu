@@ -158,7 +158,8 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   };
   for (size_t e = 0; e < je.size(); ++e) cid_of(jac_coef(je[e]));
   if (too_many) return fail(VB_ERR_ARG, "more than 256 distinct stoichiometric coefficients");
-  if (coefs.empty()) coefs.push_back(0.0);
+  const int zero_id = (int)coefs.size();   // of the terms that fill up short lists
+  coefs.push_back(0.0);
   bool packed = true;
   for (const auto& c : coef_id) packed = packed && (c.first & 0xffffffffffffull) == 0;
   auto code_of = [&](double c) {
@@ -196,7 +197,7 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   auto sum_ptr = [&](uint32_t t) -> const std::vector<int32_t>& { return (t & 1) ? pp : lp; };
   auto sum_len = [&](uint32_t t) { return (size_t)(sum_ptr(t)[t / 2 + 1] - sum_ptr(t)[t / 2]); };
   auto jac_len = [&](uint32_t d) { return (size_t)(jp[d + 1] - jp[d]); };
-  std::vector<uint32_t> sums, diag, rest, brief[vb::GL_SHORT + 1];
+  std::vector<uint32_t> sums, diag, rest, brief;
   size_t padded = 0;   // a bound of the table's words
   for (uint32_t t = 0; t < 2 * (uint32_t)ni; ++t) {
     sums.push_back(t);
@@ -206,7 +207,8 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
     const size_t len = jac_len(d);
     if (len > 0xffffu) return fail(VB_ERR_ARG, "a Jacobian entry has more than 65535 terms");
     padded += 32 * len;
-    (d / ni == d % ni ? diag : len > vb::GL_SHORT ? rest : brief[len]).push_back(d);
+    (d / ni == d % ni ? diag : len > vb::GL_SHORT ? rest : brief).push_back(d);
+    if (len <= vb::GL_SHORT) padded += 32 * vb::GL_SHORT;
   }
   if (padded > 0xffffffffu) return fail(VB_ERR_ARG, "Jacobian gather table too large");
   auto jac_word = [&](uint32_t d, size_t i) { return jw[jp[d] + i]; };
@@ -215,12 +217,9 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
                                [&](uint32_t t) { return t << 16; });
   const int n_diag = add_lists(diag, jac_len, jac_word, jac_tag);
   const int n_long = add_lists(rest, jac_len, jac_word, jac_tag);
-  int first[vb::GL_SHORT + 1], count[vb::GL_SHORT + 1];
-  for (int c = vb::GL_SHORT, at = n_long; c >= 0; --c) {
-    first[c] = at;
-    at = add_lists(brief[c], jac_len, jac_word, jac_tag);
-    count[c] = at - first[c];
-  }
+  const uint32_t filler = vb::term_word(R * T, packed ? 0 : zero_id);
+  add_lists(brief, [](uint32_t) { return (size_t)vb::GL_SHORT; },
+            [&](uint32_t d, size_t i) { return i < jac_len(d) ? jac_word(d, i) : filler; }, jac_tag);
   if (gw.empty()) gw.push_back(0u);
   std::vector<uint64_t> rx(R, 0);
   if (T <= vb::RX_TERMS)
@@ -277,10 +276,7 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   d.gl_sums = n_sums;
   d.gl_diag = n_diag;
   d.gl_long = n_long;
-  for (int c = 0; c <= vb::GL_SHORT; ++c) {
-    d.gl_first[c] = first[c];
-    d.gl_count[c] = count[c];
-  }
+  d.gl_groups = (int)gbase.size() - 1;
   d.coef_tab = (const double*)(b + parts[8].off);
   d.n_coef = (int)coefs.size();
   d.coef_packed = packed;

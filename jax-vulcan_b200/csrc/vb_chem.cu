@@ -19,31 +19,20 @@ namespace vb {
 
 struct LayerSmem {
   double* y3;      // [3][ni+1]: layers j-1, j, j+1 (padding slot = 1.0)
-  double* rate;    // [nr+1]
-  double* drate;   // [(nr+1)*T]
-  double* jac;     // [ni*ni] gathered Jacobian
   double* diff;    // [ni]
   double* diagd;   // [ni]
-  double* part;    // [2*ni] loss / production partial sums
-  double* scal;    // [8]: ysum(j-1), ysum(j), ysum(j+1)
+  double* scal;    // [3]: ysum(j-1), ysum(j), ysum(j+1)
 };
 
-// jac: drate buffer for the Jacobian; jsm: also a shared-memory Jacobian block.
-__host__ __device__ inline size_t layer_smem_bytes(int ni, int nr, int T, bool jac, bool jsm = false) {
-  size_t d = 3 * (size_t)(ni + 1) + (nr + 1) + (jac ? (size_t)(nr + 1) * T : 0) + (jsm ? (size_t)ni * ni : 0) +
-             4 * (size_t)ni + 8;
-  return d * sizeof(double);
+__host__ __device__ inline size_t layer_smem_bytes(int ni) {
+  return (3 * (size_t)(ni + 1) + 2 * (size_t)ni + 3) * sizeof(double);
 }
 
-__device__ inline LayerSmem carve(double* s, int ni, int nr, int T, bool jac, bool jsm = false) {
+__device__ inline LayerSmem carve(double* s, int ni) {
   LayerSmem L;
   L.y3 = s; s += 3 * (ni + 1);
-  L.rate = s; s += nr + 1;
-  L.drate = s; s += jac ? (nr + 1) * T : 0;
-  L.jac = s; s += jsm ? ni * ni : 0;
   L.diff = s; s += ni;
   L.diagd = s; s += ni;
-  L.part = s; s += 2 * ni;
   L.scal = s;
   return L;
 }
@@ -170,73 +159,113 @@ __device__ __forceinline__ double rate_terms(const double (&yr)[TT], const Slot&
   return rt;
 }
 
-// Rate (and drate) of reaction slot r with TT terms of one layer.
-template <int TT>
-__device__ inline void rate_slot(const Slot& S, int r, const double* yrow, double kr, double M, double* rate,
-                                 double* drate, bool jac) {
-  double yr[TT], d[TT];
+// Values of NL layers at one index, interleaved in shared memory.
+template <int NL>
+struct Vals {
+  double v[NL];
+};
+template <int NL>
+__device__ __forceinline__ Vals<NL> ld_vals(const double* p, int i) {
+  Vals<NL> r;
+  if (NL == 2) {
+    const double2 d = *reinterpret_cast<const double2*>(p + 2 * i);
+    r.v[0] = d.x;
+    r.v[NL - 1] = d.y;
+  } else {
+    r.v[0] = p[i];
+  }
+  return r;
+}
+template <int NL>
+__device__ __forceinline__ void st_vals(double* p, int i, const double (&v)[NL]) {
+  if (NL == 2)
+    *reinterpret_cast<double2*>(p + 2 * i) = make_double2(v[0], v[NL - 1]);
+  else
+    p[i] = v[0];
+}
+
+// Rates (and drates) of reaction slot r with TT terms; yrow: the layers' state
+// rows, ystride apart.
+template <int TT, int NL>
+__device__ inline void rate_slot(const Slot& S, int r, const double* yrow, int ystride, const double (&kr)[NL],
+                                 const double (&M)[NL], double* rate, double* drate, bool jac) {
+  double rt[NL], d[NL][TT];
 #pragma unroll
-  for (int s = 0; s < TT; ++s) yr[s] = yrow[slot_species<TT>(S, s)];
-  rate[r] = rate_terms<TT>(yr, S, kr, M, jac, d);
+  for (int l = 0; l < NL; ++l) {
+    double yr[TT];
+#pragma unroll
+    for (int s = 0; s < TT; ++s) yr[s] = yrow[l * ystride + slot_species<TT>(S, s)];
+    rt[l] = rate_terms<TT>(yr, S, kr[l], M[l], jac, d[l]);
+  }
+  st_vals<NL>(rate, r, rt);
   if (jac) {
 #pragma unroll
-    for (int s = 0; s < TT; ++s) drate[r * TT + s] = d[s];
+    for (int s = 0; s < TT; ++s) {
+      double v[NL];
+#pragma unroll
+      for (int l = 0; l < NL; ++l) v[l] = d[l][s];
+      st_vals<NL>(drate, r * TT + s, v);
+    }
   }
 }
 
 // Rate constants of RU consecutive passes, loaded before any arithmetic so the
 // strided L2 loads overlap (L2 only: the column of k would flush the gather
-// tables from L1).
-template <int TT, int RU>
-__device__ inline void rates_t(const NetDev& net, const double* yrow, const double* kcol, int64_t kstride, double M,
-                               double* rate, double* drate, bool jac) {
+// tables from L1). kcol: the first layer's column; zs: the second's offset.
+template <int TT, int NL, int RU>
+__device__ inline void rates_t(const NetDev& net, const double* yrow, int ystride, const double* kcol,
+                               int64_t kstride, int zs, const double (&M)[NL], double* rate, double* drate, bool jac) {
   for (int r0 = threadIdx.x; r0 <= net.nr; r0 += RU * blockDim.x) {
-    double kv[RU];
+    double kv[RU][NL];
     Slot S[RU];
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
-      kv[u] = r <= net.nr ? __ldcg(kcol + (int64_t)r * kstride) : 0.0;
+#pragma unroll
+      for (int l = 0; l < NL; ++l) kv[u][l] = r <= net.nr ? __ldcg(kcol + (int64_t)r * kstride + l * zs) : 0.0;
       if (TT <= RX_TERMS) S[u] = load_slot<TT>(net, min(r, net.nr));
     }
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       const int r = r0 + u * blockDim.x;
       if (TT > RX_TERMS && r <= net.nr) S[u] = load_slot<TT>(net, r);
-      if (r <= net.nr) rate_slot<TT>(S[u], r, yrow, kv[u], M, rate, drate, jac);
+      if (r <= net.nr) rate_slot<TT, NL>(S[u], r, yrow, ystride, kv[u], M, rate, drate, jac);
     }
   }
 }
 
-// rate[r] = k[r] * prod_s y^st (* M) for every reaction slot of one layer
+// rate[r] = k[r] * prod_s y^st (* M) for every reaction slot of NL layers
 // (chem.py:92-99); with jac, also drate[r][s] (chem.py:156-182).
-__device__ inline void layer_rates(const NetDev& net, const double* yrow, const double* kcol,
-                                   int64_t kstride, double M, double* rate, double* drate, bool jac) {
+template <int NL>
+__device__ inline void layer_rates(const NetDev& net, const double* yrow, int ystride, const double* kcol,
+                                   int64_t kstride, int zs, const double (&M)[NL], double* rate, double* drate,
+                                   bool jac) {
+  constexpr int D = NL == 2 ? 3 : 6, DW = NL == 2 ? 2 : 4;
   if (!jac) {   // the right-hand-side kernels run at full occupancy: fewer loads in flight per thread
     switch (net.T) {
-      case 1: rates_t<1, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 2: rates_t<2, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 3: rates_t<3, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 4: rates_t<4, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 5: rates_t<5, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 6: rates_t<6, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      case 7: rates_t<7, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-      default: rates_t<8, 2>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
+      case 1: rates_t<1, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 2: rates_t<2, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 3: rates_t<3, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 4: rates_t<4, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 5: rates_t<5, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 6: rates_t<6, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 7: rates_t<7, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      default: rates_t<8, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
     }
   }
   switch (net.T) {
-    case 1: rates_t<1, 6>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 2: rates_t<2, 6>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 3: rates_t<3, 6>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 4: rates_t<4, 6>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 5: rates_t<5, 4>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 6: rates_t<6, 4>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    case 7: rates_t<7, 4>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
-    default: rates_t<8, 4>(net, yrow, kcol, kstride, M, rate, drate, jac); return;
+    case 1: rates_t<1, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 2: rates_t<2, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 3: rates_t<3, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 4: rates_t<4, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 5: rates_t<5, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 6: rates_t<6, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 7: rates_t<7, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    default: rates_t<8, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
   }
 }
 
-// The coefficient table of the gathers into shared memory (coef[MAX_COEF]).
+// The coefficient table of the gathers into shared memory (coef[MAX_COEF + 1]).
 __device__ inline void load_coefs(const NetDev& net, double* coef) {
   if (net.coef_packed) return;
   for (int c = threadIdx.x; c < net.n_coef; c += blockDim.x) coef[c] = net.coef_tab[c];
@@ -256,57 +285,70 @@ __device__ __forceinline__ void group_words(const uint32_t* wp, int len, uint32_
   for (int u = 0; u < GW; ++u) w[u] = u < len ? __ldg(wp + 32 * u) : 0u;
 }
 
-// Sum of a lane's list of cnt terms, in list order; len: the group's longest.
+// Sums of a lane's list of cnt terms, in list order; len: the group's longest.
 // w holds the first GW words; each half is reloaded GW terms ahead as it is used.
-template <bool PK>
-__device__ __forceinline__ double gather_list(const double* coef, const double* src, const uint32_t* wp, int len,
-                                              int cnt, uint32_t (&w)[GW]) {
+template <bool PK, int NL>
+__device__ __forceinline__ void gather_list(const double* coef, const double* src, const uint32_t* wp, int len,
+                                            int cnt, uint32_t (&w)[GW], double (&acc)[NL]) {
   constexpr int H = GW / 2;
-  double acc = 0.0;
+#pragma unroll
+  for (int l = 0; l < NL; ++l) acc[l] = 0.0;
   for (int k = 0; k < len; k += GW) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int k0 = k + h * H;
       if (k0 >= len) break;
-      double v[H], c[H];
+      Vals<NL> v[H];
+      double c[H];
 #pragma unroll
       for (int u = 0; u < H; ++u) {
-        v[u] = src[w[h * H + u] & 0xffffu];
+        v[u] = ld_vals<NL>(src, (int)(w[h * H + u] & 0xffffu));
         c[u] = term_coef<PK>(coef, w[h * H + u]);
       }
 #pragma unroll
       for (int u = 0; u < H; ++u) w[h * H + u] = k0 + GW + u < len ? __ldg(wp + 32 * (k0 + GW + u)) : 0u;
 #pragma unroll
       for (int u = 0; u < H; ++u) {
-        const double t = acc + c[u] * v[u];
-        if (k0 + u < cnt) acc = t;
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          const double t = acc[l] + c[u] * v[u].v[l];
+          if (k0 + u < cnt) acc[l] = t;
+        }
       }
     }
   }
-  return acc;
 }
 
-// A long group's lane sum.
-template <bool PK>
-__device__ __forceinline__ double gather_group(const NetDev& net, const double* coef, const double* src, int g,
-                                               uint32_t desc) {
+// A long group's lane sums.
+template <bool PK, int NL>
+__device__ __forceinline__ void gather_group(const NetDev& net, const double* coef, const double* src, int g,
+                                             uint32_t desc, double (&acc)[NL]) {
   const uint32_t b0 = net.gl_base[g], b1 = net.gl_base[g + 1];
   const int len = (int)(b1 - b0) / 32;
   const uint32_t* wp = net.gl_w + b0 + (threadIdx.x & 31);
   uint32_t w[GW];
   group_words(wp, len, w);
-  return gather_list<PK>(coef, src, wp, len, (int)(desc & 0xffffu), w);
+  gather_list<PK, NL>(coef, src, wp, len, (int)(desc & 0xffffu), w, acc);
 }
 
-// GB groups of entries of exactly C terms each, from group g (n of them
-// exist): all words first, so the table's latency is paid once.
+// Up to GB groups of short entries, from group g (n of them exist): all words
+// first, so the table's latency is paid once. Every list has GL_SHORT words,
+// though three quarters of the entries have fewer terms: without classes by
+// length the entries stay in storage order, and a warp's store touches 9
+// sectors, not 27. Measured on B200 (stage 1 with the diffusion rows, 296
+// atmospheres of 69 species, two layers per CTA / 128 of 89 species): a class
+// per length 2.08 / 1.94 ms, lists filled up to 2 or 4 terms 1.97 / 1.79, to 4
+// 1.97 / 1.76, to 3 or 8 2.05 / 1.75. Ordering the lists of equal length so
+// that a quarter-warp's reads share fewer banks, at the cost of the stores'
+// order, was slower (2.14 / 2.08).
 constexpr int GB = 4;
-template <int C, bool PK, typename Off>
+template <bool PK, int NL, typename Off>
 __device__ __forceinline__ void gather_short(const NetDev& net, const double* coef, const double* drate, int g, int n,
                                              Off off) {
+  constexpr int C = GL_SHORT;
   const int lane = threadIdx.x & 31;
-  const uint32_t* wp = net.gl_w + net.gl_base[net.gl_first[C]] + 32 * C * (g - net.gl_first[C]) + lane;
-  uint32_t desc[GB], w[GB][C ? C : 1];
+  const uint32_t* wp = net.gl_w + net.gl_base[g] + lane;
+  uint32_t desc[GB], w[GB][C];
 #pragma unroll
   for (int q = 0; q < GB; ++q) {
     desc[q] = q < n ? __ldg(net.gl_desc + 32 * (g + q) + lane) : ~0u;
@@ -315,23 +357,30 @@ __device__ __forceinline__ void gather_short(const NetDev& net, const double* co
   }
 #pragma unroll
   for (int q = 0; q < GB; ++q) {
-    double J = 0.0;
+    double J[NL];
 #pragma unroll
-    for (int u = 0; u < C; ++u) J = J + term_coef<PK>(coef, w[q][u]) * drate[w[q][u] & 0xffffu];
+    for (int l = 0; l < NL; ++l) J[l] = 0.0;
+#pragma unroll
+    for (int u = 0; u < C; ++u) {
+      const double c = term_coef<PK>(coef, w[q][u]);
+      const Vals<NL> v = ld_vals<NL>(drate, (int)(w[q][u] & 0xffffu));
+#pragma unroll
+      for (int l = 0; l < NL; ++l) J[l] = J[l] + c * v.v[l];
+    }
     if (desc[q] != ~0u) off((int)((desc[q] >> 16) & 0x7fu), (int)(desc[q] >> 23), J);
   }
 }
 
-// The gathers of one layer: the species lists' sums to part[t] (sums), the
+// The gathers of NL layers: the species lists' sums to part[t] (sums), the
 // Jacobian's diagonal entries to diag(row, J), the others to off(row, col, J),
 // each in the reference's order. The warps take work from a queue in shared
 // memory (zeroed before the barrier ahead of this), the long groups first and
 // one by one, then the short ones GB at a time, so they finish together. What
 // bounds this is instructions issued and shared-memory wavefronts, not the
-// latency of the tables: hence exact code for the short lists (three quarters
-// of the entries), the diagonal's extra terms out of the common path, and the
-// coefficient in the word.
-template <bool PK, typename Diag, typename Off>
+// latency of the tables: hence code without counts for the short lists, the
+// diagonal's extra terms out of the common path, and the coefficient in the
+// word. drate[(nr+1)*T] of each layer is 0 (fillers of short lists).
+template <bool PK, int NL, typename Diag, typename Off>
 __device__ __forceinline__ void gather_layer_t(const NetDev& net, const double* coef, const double* rate,
                                                const double* drate, bool sums, int* queue, double* part, Diag diag,
                                                Off off) {
@@ -344,101 +393,78 @@ __device__ __forceinline__ void gather_layer_t(const NetDev& net, const double* 
     if (g < net.gl_long) {
       const uint32_t desc = net.gl_desc[32 * g + lane];
       const bool on = desc != ~0u;
-      const double acc = gather_group<PK>(net, coef, g < net.gl_sums ? rate : drate, g, on ? desc : 0u);
+      double acc[NL];
+      gather_group<PK, NL>(net, coef, g < net.gl_sums ? rate : drate, g, on ? desc : 0u, acc);
       if (!on) continue;
       const int row = (int)((desc >> 16) & 0x7fu);
       if (g < net.gl_sums)
-        part[desc >> 16] = acc;
+        st_vals<NL>(part, (int)(desc >> 16), acc);
       else if (g < net.gl_diag)
         diag(row, acc);
       else
         off(row, (int)(desc >> 23), acc);
       continue;
     }
-    g -= net.gl_long;
-    int c = GL_SHORT;
-    for (; c >= 0; --c) {
-      const int nb = (net.gl_count[c] + GB - 1) / GB;
-      if (g < nb) break;
-      g -= nb;
-    }
-    if (c < 0) break;
-    const int n = net.gl_count[c] - GB * g;
-    g = net.gl_first[c] + GB * g;
-    switch (c) {
-      case 4: gather_short<4, PK>(net, coef, drate, g, n, off); break;
-      case 3: gather_short<3, PK>(net, coef, drate, g, n, off); break;
-      case 2: gather_short<2, PK>(net, coef, drate, g, n, off); break;
-      case 1: gather_short<1, PK>(net, coef, drate, g, n, off); break;
-      default: gather_short<0, PK>(net, coef, drate, g, n, off); break;
-    }
+    g = net.gl_long + GB * (g - net.gl_long);
+    if (g >= net.gl_groups) break;
+    gather_short<PK, NL>(net, coef, drate, g, net.gl_groups - g, off);
   }
 }
 
-template <typename Diag, typename Off>
+template <int NL, typename Diag, typename Off>
 __device__ __forceinline__ void gather_layer(const NetDev& net, const double* coef, const double* rate,
                                              const double* drate, bool sums, int* queue, double* part, Diag diag,
                                              Off off) {
   if (net.coef_packed)
-    gather_layer_t<true>(net, coef, rate, drate, sums, queue, part, diag, off);
+    gather_layer_t<true, NL>(net, coef, rate, drate, sums, queue, part, diag, off);
   else
-    gather_layer_t<false>(net, coef, rate, drate, sums, queue, part, diag, off);
+    gather_layer_t<false, NL>(net, coef, rate, drate, sums, queue, part, diag, off);
 }
 
 // Loss and production sums of every species: part[2i] = loss_i, part[2i+1] =
 // prod_i. The caller synchronises before reading dy_i/dt = part[2i+1] - part[2i].
-template <bool PK>
+template <bool PK, int NL>
 __device__ __forceinline__ void species_sums_t(const NetDev& net, const double* coef, const double* rate,
                                                double* part) {
   for (int g = (int)threadIdx.x / 32; g < net.gl_sums; g += (int)blockDim.x / 32) {
     const uint32_t desc = net.gl_desc[32 * g + (threadIdx.x & 31)];
-    const double acc = gather_group<PK>(net, coef, rate, g, desc == ~0u ? 0u : desc);
-    if (desc != ~0u) part[desc >> 16] = acc;
+    double acc[NL];
+    gather_group<PK, NL>(net, coef, rate, g, desc == ~0u ? 0u : desc, acc);
+    if (desc != ~0u) st_vals<NL>(part, (int)(desc >> 16), acc);
   }
 }
 
+template <int NL>
 __device__ inline void species_sums(const NetDev& net, const double* coef, const double* rate, double* part) {
   if (net.coef_packed)
-    species_sums_t<true>(net, coef, rate, part);
+    species_sums_t<true, NL>(net, coef, rate, part);
   else
-    species_sums_t<false>(net, coef, rate, part);
+    species_sums_t<false, NL>(net, coef, rate, part);
 }
 
-// Loads state rows j-1..j+1 (stage 2: yk2 = y + k1/r) and their gas sums.
-template <bool STAGE_GAS = false>
-__device__ inline void load_rows(const double* y, const double* k1, const double* gas, int nz, int ni,
-                                 int j, double rinv_r, bool stage2, LayerSmem& L) {
+// Loads state rows j-1..j+1 and their gas sums.
+__device__ inline void load_rows(const double* y, const double* gas, int nz, int ni, int j, LayerSmem& L) {
   for (int t = threadIdx.x; t < 3 * (ni + 1); t += blockDim.x) {
     int w = t / (ni + 1), i = t % (ni + 1);
     int jj = j - 1 + w;
     double v = 1.0;
-    if (i < ni) {
-      if (jj >= 0 && jj < nz) {
-        v = y[(int64_t)jj * ni + i];
-        if (stage2) v = v + k1[(int64_t)jj * ni + i] / rinv_r;
-      } else {
-        v = 0.0;
-      }
-    }
+    if (i < ni) v = (jj >= 0 && jj < nz) ? y[(int64_t)jj * ni + i] : 0.0;
     L.y3[t] = v;
   }
-  // STAGE_GAS: the gas mask staged in diagd (free until the diffusion writes
-  // it), so the three sums below read shared memory
-  if (STAGE_GAS)
-    for (int i = threadIdx.x; i < ni; i += blockDim.x) L.diagd[i] = gas[i];
+  // the gas mask staged in diagd (free until the diffusion writes it), so the
+  // three sums below read shared memory
+  for (int i = threadIdx.x; i < ni; i += blockDim.x) L.diagd[i] = gas[i];
   __syncthreads();
   if (threadIdx.x < 3) {
     int w = threadIdx.x;
     int jj = j - 1 + w;
     double s = 0.0;
-    if (jj >= 0 && jj < nz) s = pairwise_sum_masked(L.y3 + w * (ni + 1), STAGE_GAS ? L.diagd : gas, ni);
+    if (jj >= 0 && jj < nz) s = pairwise_sum_masked(L.y3 + w * (ni + 1), L.diagd, ni);
     L.scal[w] = s;
   }
   __syncthreads();
 }
 
-// diff[i] (with BC fluxes) and the diagonal diffusion term diag_d[i] of row j;
-// also the sup/sub coefficients of row j when requested.
 // Diffusion term of species i on row j from its combined coefficients and
 // state values y(j), y(j-1), y(j+1): the stencil and the boundary fluxes
 // (jax_step.py:223-246, _apply_diffusion_jax).
@@ -461,30 +487,15 @@ __device__ inline double diffusion_term(const AtmRef& a, int nz, int j, int i, i
   return d;
 }
 
-// STAGED 2: the row's atmosphere fields are loaded in one round before the
-// arithmetic (RowAcc: per-layer fields in shared memory, the species' own in
-// registers; faster in the stage-2 kernels, slower in stage 1, where the
-// extra live registers spill); 0: read where used. again: a second call in
-// the same kernel (waits until the first has read eddy and lay).
-template <int STAGED = 0>
+// diff[i] (with BC fluxes) and the diagonal diffusion term diag_d[i] of row j;
+// also the sup/sub coefficients of row j when requested.
 __device__ inline void layer_diffusion(const AtmRef& a, int nz, int ni, int j, int flags, LayerSmem& L,
-                                       double* sup_out, double* sub_out, bool want_diag, bool again = false) {
+                                       double* sup_out, double* sub_out) {
   double ysm = L.scal[0], ys0 = L.scal[1], ysp = L.scal[2];
-  // the row's per-layer fields staged in one round of loads (the eddy and
-  // molecular terms then read them between their divisions from shared
-  // memory; each species' own fields are loaded together below)
-  __shared__ double eddy[3], lay[21];
-  if (again) __syncthreads();   // the previous call has finished reading eddy and lay
-  if (STAGED) {
-    stage_row_layers(a, nz, j, lay);
-    __syncthreads();
-  }
+  __shared__ double eddy[3];
   if (threadIdx.x == 0) {
     double A, B, C;
-    if (STAGED)
-      eddy_row_t<double>(layer_acc(lay, j), nz, j, ysm, ys0, ysp, A, B, C);
-    else
-      eddy_row(a, nz, j, ysm, ys0, ysp, A, B, C);
+    eddy_row(a, nz, j, ysm, ys0, ysp, A, B, C);
     eddy[0] = A; eddy[1] = B; eddy[2] = C;
   }
   __syncthreads();
@@ -495,454 +506,168 @@ __device__ inline void layer_diffusion(const AtmRef& a, int nz, int ni, int j, i
   const double* yp = L.y3 + 2 * (ni + 1);
   for (int i = threadIdx.x; i < ni; i += blockDim.x) {
     double Am, Bm, Cm;
-    if (STAGED)
-      mol_row_t<double>(row_acc(a, lay, ni, j, i, j - 1, 3), nz, j, i, ysm, ys0, ysp, use_vm, use_set, Am, Bm,
-                        Cm);
-    else
-      mol_row(a, nz, ni, j, i, ysm, ys0, ysp, use_vm, use_set, Am, Bm, Cm);
+    mol_row(a, nz, ni, j, i, ysm, ys0, ysp, use_vm, use_set, Am, Bm, Cm);
     double At = eddy[0] + Am;
     double Bt = eddy[1] + Bm;
     double Ct = eddy[2] + Cm;
     L.diff[i] = diffusion_term(a, nz, j, i, flags, At, Bt, Ct, y0[i], ym[i], yp[i]);
-    if (want_diag) L.diagd[i] = At;
+    L.diagd[i] = At;
     if (sup_out && j < nz - 1) sup_out[i] = Bt;
     if (sub_out && j > 0) sub_out[i] = Ct;
   }
 }
 
+// Shared memory of stage1_kernel<NL>: the drates (and a 0) and rates of NL
+// layers interleaved (16-byte aligned at NL = 2), then sums, rows and diagonals.
+__host__ __device__ inline size_t stage1_smem_bytes(int ni, int nr, int T, int NL) {
+  return (size_t)NL * ((size_t)(nr + 1) * (T + 1) + 1 + 2 * (size_t)ni + (ni + 1) + ni) * sizeof(double);
+}
+
 // Stage-1 assembly: rmod[j] = rhs(y), inv[j] = c0*I - J - diag(diag_d),
-// supn[j] = -sup_d, subn[j-1] = -sub_d, with fix_mask (jax_step.py:263-298).
-// Four CTAs per SM, the shared-memory limit with the drate buffer (three,
-// without spills, were slower when the gathers were latency-bound). Measured
-// on B200, ni=69, nr=1400, nz=120, 296 atmospheres, with the diffusion rows:
-// 2.71 ms with the lists dealt out in fixed bands, coefficients in a table and
-// pow in line (681 M instructions in a ragged batch of 85, issue slots 70 %
-// busy); 2.92 with the queue alone; 2.46 with exact code for the short lists
-// and packed reaction words (406 M); 2.35 with pow out of line. What is left
-// is the wavefronts of the scattered shared-memory reads.
-__global__ void __launch_bounds__(LAYER_THREADS, 4)
+// supn[j] = -sup_d, subn[j-1] = -sub_d, with fix_mask (jax_step.py:263-298),
+// of layers j0 .. j0 + NL - 1, j0 = NL blockIdx.x.
+// Measured on B200, ni=69, nr=1400, nz=120, 296 atmospheres, with the diffusion
+// rows, one layer per CTA, four CTAs per SM (the shared-memory limit): 2.71 ms
+// with the lists dealt out in fixed bands, coefficients in a table and pow in
+// line (681 M instructions in a ragged batch of 85, issue slots 70 % busy);
+// 2.92 with the queue alone; 2.46 with code without counts for the short lists
+// and packed reaction words (406 M); 2.35 with pow out of line; 2.02 with the
+// short entries in storage order; 1.98 with two layers per CTA, where 512
+// threads beat 384 (2.20 against 2.07 at that point) and 256 (2.44). What is
+// left is the wavefronts of the scattered shared-memory reads.
+template <int NL>
+__global__ void __launch_bounds__(NL * LAYER_THREADS, 4 / NL)
 stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
               const double* __restrict__ dt, const double* __restrict__ atm, int flags,
               const uint8_t* __restrict__ fix_mask, double* __restrict__ ws, const double* __restrict__ adj_v) {
   extern __shared__ double smem[];
-  const int b = blockIdx.y, j = blockIdx.x;
+  const int b = blockIdx.y, j = NL * blockIdx.x;
   Geo g = geo_of(B, b);
   if (j >= g.nz) return;
-  const int ni = B.ni, nz = g.nz;
-  LayerSmem L = carve(smem, ni, B.nr, net.T, true);
+  const int ni = B.ni, nz = g.nz, ld = B.ld;
+  const int nl = min(NL, nz - j);                 // layers here
+  const int last = nl - 1;                        // a missing layer repeats the last, without stores
+  double* drate = smem;                           // [(nr+1)*T + 1][NL]
+  double* rate = drate + NL * ((B.nr + 1) * net.T + 1);   // [nr+1][NL]
+  double* part = rate + NL * (B.nr + 1);          // [2 ni][NL]
+  double* yj = part + NL * 2 * ni;                // [NL][ni+1]
+  double* diagd = yj + NL * (ni + 1);             // [NL][ni]
   AtmRef a = atm_ref(atm + g.atm, nz, ni);
-  WsView w = ws_view(ws, g, ni, B.ld);
+  WsView w = ws_view(ws, g, ni, ld);
   const double* yb = y + g.z0 * ni;
   const uint8_t* fm = fix_mask ? fix_mask + g.z0 * ni + (int64_t)j * ni : nullptr;
   const bool adj = adj_v != nullptr;   // J_y blocks of the steady-state adjoint
   const double r = ros2_r();
   const double c0 = adj ? 0.0 : 1.0 / (r * dt[b]);
 
-  __shared__ double coefs[MAX_COEF];
+  __shared__ double coefs[MAX_COEF + 1];
   __shared__ int queue;
   if (threadIdx.x == 0) queue = 0;
+  if (threadIdx.x < NL) drate[NL * (B.nr + 1) * net.T + threadIdx.x] = 0.0;
   load_coefs(net, coefs);
-  // state row j (the rates; padding slot 1.0) and diag_d of row j, written
-  // with the row's diffusion terms by diffusion_rows_kernel ahead of this kernel
-  double* yj = L.y3 + (ni + 1);
-  for (int t = threadIdx.x; t <= ni; t += blockDim.x) yj[t] = t < ni ? yb[(int64_t)j * ni + t] : 1.0;
-  for (int i = threadIdx.x; i < ni; i += blockDim.x) L.diagd[i] = w.aux[(int64_t)j * ni + i];
+  // state rows (the rates; padding slot 1.0) and diag_d, written with the rows'
+  // diffusion terms by diffusion_rows_kernel ahead of this kernel
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    const int64_t q = (int64_t)(j + min(l, last)) * ni;
+    for (int t = threadIdx.x; t <= ni; t += blockDim.x) yj[l * (ni + 1) + t] = t < ni ? yb[q + t] : 1.0;
+    for (int i = threadIdx.x; i < ni; i += blockDim.x) diagd[l * ni + i] = w.aux[q + i];
+  }
   __syncthreads();
-  layer_rates(net, yj, k + g.z0 * (B.nr + 1) + j, nz, a.M[j], L.rate, L.drate, true);
+  double M[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) M[l] = a.M[j + min(l, last)];
+  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, rate, drate, true);
   __syncthreads();
   // One phase for the species sums and the Jacobian gather. The gather writes
   // each block entry in its final form.
-  double* blk = w.inv + (int64_t)j * ni * B.ld;
-  const int ld = B.ld;
+  double* blk = w.inv + (int64_t)j * ni * ld;
+  const int64_t lstep = (int64_t)ni * ld;
   const double bot = (j == 0 && (flags & VB_USE_BOTFLUX)) ? 1.0 : 0.0;
+  auto depth = [&](int row, int l) { return l == 0 && j == 0 ? (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0) : 0.0; };
   if (adj) {
     // steady_state_grad.py:153-175: diag = J + diag(A_eddy + A_mol) (+ deposition
     // at the bottom), sup_d = B[:-1], sub_d = C[1:] (no c0, not negated); no sums
-    gather_layer(
-        net, coefs, L.rate, L.drate, false, &queue, L.part,
-        [&](int row, double J) {
-          double v = J + L.diagd[row];
-          if (j == 0) v = v + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
-          blk[(int64_t)row * ld + row] = v;
+    gather_layer<NL>(
+        net, coefs, rate, drate, false, &queue, part,
+        [&](int row, const double (&J)[NL]) {
+#pragma unroll
+          for (int l = 0; l < NL; ++l) {
+            double v = J[l] + diagd[l * ni + row];
+            if (l == 0 && j == 0) v = v + depth(row, l);
+            if (l < nl) blk[l * lstep + (int64_t)row * ld + row] = v;
+          }
         },
-        [&](int row, int col, double J) { blk[(int64_t)row * ld + col] = J; });
-    for (int i = threadIdx.x; i < ni; i += blockDim.x)
+        [&](int row, int col, const double (&J)[NL]) {
+#pragma unroll
+          for (int l = 0; l < NL; ++l)
+            if (l < nl) blk[l * lstep + (int64_t)row * ld + col] = J[l];
+        });
+    for (int i = threadIdx.x; i < nl * ni; i += blockDim.x)
       w.rmod[(int64_t)j * ni + i] = adj_v[g.z0 * ni + (int64_t)j * ni + i];
     return;
   }
-  gather_layer(
-      net, coefs, L.rate, L.drate, true, &queue, L.part,
-      [&](int row, double J) {
-        double v = c0 - J;
-        // jax_step.py:283,288: the deposition term joins diag_d before -diag_d is added
-        double dd = L.diagd[row];
-        if (j == 0) dd = dd + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
-        v = v + (-dd);
-        if (fm && fm[row]) v = c0;
-        blk[(int64_t)row * ld + row] = v;
+  gather_layer<NL>(
+      net, coefs, rate, drate, true, &queue, part,
+      [&](int row, const double (&J)[NL]) {
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          double v = c0 - J[l];
+          // jax_step.py:283,288: the deposition term joins diag_d before -diag_d is added
+          double dd = diagd[l * ni + row];
+          if (l == 0 && j == 0) dd = dd + depth(row, l);
+          v = v + (-dd);
+          if (l < nl) {
+            if (fm && fm[l * ni + row]) v = c0;
+            blk[l * lstep + (int64_t)row * ld + row] = v;
+          }
+        }
       },
-      [&](int row, int col, double J) {
-        double v = 0.0 - J;
-        if (fm && fm[row]) v = 0.0;
-        blk[(int64_t)row * ld + col] = v;
+      [&](int row, int col, const double (&J)[NL]) {
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          if (l < nl) {
+            double v = 0.0 - J[l];
+            if (fm && fm[l * ni + row]) v = 0.0;
+            blk[l * lstep + (int64_t)row * ld + col] = v;
+          }
+        }
       });
   __syncthreads();   // the species sums
-  for (int i = threadIdx.x; i < ni; i += blockDim.x) {
+  for (int t = threadIdx.x; t < nl * ni; t += blockDim.x) {
+    const int l = t >= ni ? 1 : 0, i = t - l * ni;
     // rmod[j] holds the row's diffusion term (diffusion_rows_kernel)
-    double v = (L.part[2 * i + 1] - L.part[2 * i]) + w.rmod[(int64_t)j * ni + i];
-    if (fm && fm[i]) v = 0.0;
-    w.rmod[(int64_t)j * ni + i] = v;
+    double v = (part[NL * (2 * i + 1) + l] - part[NL * 2 * i + l]) + w.rmod[(int64_t)j * ni + t];
+    if (fm && fm[t]) v = 0.0;
+    w.rmod[(int64_t)j * ni + t] = v;
   }
 }
 
-// ---------------------------------------------------------------- stage 1, two layers per CTA
-// The same assembly as stage1_kernel for layers j0 = 2 blockIdx.x and j0 + 1
-// of one atmosphere: every gather word, rate-constant sector and network
-// table entry is loaded once for both layers, and each sum runs as two
-// independent chains (each in the reference's order, so every value is
-// bit-identical to the one-layer kernel's).
-constexpr int PAIR_THREADS = 512;
-
-struct PairSmem {
-  double* y4;      // [4][ni+1]: layers j0-1 .. j0+2 (padding slot 1.0)
-  double* rate;    // [2][nr+1]
-  double* drate;   // [2][(nr+1)*T]
-  double* diff;    // [2][ni]
-  double* diagd;   // [2][ni]
-  double* part;    // [2][2*ni]
-  double* scal;    // [8]: ysums of the four rows
-  double* supb;    // [2][ni]
-  double* subb;    // [2][ni]
-};
-
-__host__ __device__ inline size_t pair_smem_bytes(int ni, int nr, int T) {
-  const size_t d = 4 * (size_t)(ni + 1) + 2 * (size_t)(nr + 1) + 2 * (size_t)(nr + 1) * T + 10 * (size_t)ni + 8 +
-                   4 * (size_t)ni;
-  return d * sizeof(double);
-}
-
-__device__ inline PairSmem carve_pair(double* s, int ni, int nr, int T) {
-  PairSmem P;
-  P.y4 = s; s += 4 * (ni + 1);
-  P.rate = s; s += 2 * (nr + 1);
-  P.drate = s; s += 2 * (nr + 1) * T;
-  P.diff = s; s += 2 * ni;
-  P.diagd = s; s += 2 * ni;
-  P.part = s; s += 4 * ni;
-  P.scal = s; s += 8;
-  P.supb = s; s += 2 * ni;
-  P.subb = s;
-  return P;
-}
-
-// Rates and drates of both layers (rate_slot's expression order per layer).
-template <int TT, int RU>
-__device__ inline void rates_pair_t(const NetDev& net, const double* y0, const double* y1, const double* kcol,
-                                    int64_t kstride, bool two, double M0, double M1, double* rate, double* drate) {
-  const int R = net.nr + 1;
-  for (int r0 = threadIdx.x; r0 < R; r0 += RU * blockDim.x) {
-    double kv[RU][2];
-#pragma unroll
-    for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
-      kv[u][0] = r < R ? __ldcg(kcol + (int64_t)r * kstride) : 0.0;
-      kv[u][1] = (two && r < R) ? __ldcg(kcol + (int64_t)r * kstride + 1) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
-      if (r < R) {
-        rate_slot<TT>(load_slot<TT>(net, r), r, y0, kv[u][0], M0, rate, drate, true);
-        if (two) rate_slot<TT>(load_slot<TT>(net, r), r, y1, kv[u][1], M1, rate + R, drate + (int64_t)R * TT, true);
-      }
-    }
-  }
-}
-
-__device__ inline void rates_pair(const NetDev& net, const double* y0, const double* y1, const double* kcol,
-                                  int64_t kstride, bool two, double M0, double M1, double* rate, double* drate) {
-  switch (net.T) {
-    case 1: rates_pair_t<1, 3>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 2: rates_pair_t<2, 3>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 3: rates_pair_t<3, 3>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 4: rates_pair_t<4, 3>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 5: rates_pair_t<5, 2>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 6: rates_pair_t<6, 2>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    case 7: rates_pair_t<7, 2>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-    default: rates_pair_t<8, 2>(net, y0, y1, kcol, kstride, two, M0, M1, rate, drate); return;
-  }
-}
-
-// Sums of a lane's list for both layers (off: the second layer's rates or drates).
-template <bool PK>
-__device__ __forceinline__ void gather_pair(const double* coef, const double* src, int64_t off, const uint32_t* wp,
-                                            int cnt, double& a0, double& a1) {
-  a0 = 0.0;
-  a1 = 0.0;
-#pragma unroll 4
-  for (int k = 0; k < cnt; ++k) {
-    const uint32_t x = wp[32 * k];
-    const double c = term_coef<PK>(coef, x);
-    const int s = x & 0xffffu;
-    a0 = a0 + c * src[s];
-    a1 = a1 + c * src[off + s];
-  }
-}
-
-__device__ __forceinline__ void gather_pair_any(const NetDev& net, const double* coef, const double* src, int64_t off,
-                                                int q, double& a0, double& a1) {
-  const uint32_t* wp = net.gl_w + net.gl_base[q >> 5] + (q & 31);
-  const int cnt = (int)(net.gl_desc[q] & 0xffffu);
-  if (net.coef_packed)
-    gather_pair<true>(coef, src, off, wp, cnt, a0, a1);
-  else
-    gather_pair<false>(coef, src, off, wp, cnt, a0, a1);
-}
-
-// Loss and production sums of both layers (species_sums' order per layer).
-__device__ inline void species_sums_pair(const NetDev& net, const double* coef, const double* rate, double* part) {
-  for (int q = threadIdx.x; q < 2 * net.ni; q += blockDim.x) {
-    double a0, a1;
-    gather_pair_any(net, coef, rate, net.nr + 1, q, a0, a1);
-    const int t = (int)(net.gl_desc[q] >> 16);
-    part[t] = a0;
-    part[2 * net.ni + t] = a1;
-  }
-}
-
-// Dense Jacobians of both layers, the entries in bands of falling term count.
-// busy: threads that summed species lists just before; the bands are rotated
-// (by whole warps) so those take the lightest entries of each band.
-template <typename Store>
-__device__ inline void jacobian_pair(const NetDev& net, const double* coef, const double* drate, Store store,
-                                     int busy) {
-  const int q0 = 32 * net.gl_sums, nq = 32 * (net.gl_first[0] + net.gl_count[0]) - q0, stride = blockDim.x;
-  for (int q = ((int)threadIdx.x - ((busy + 31) & ~31) % stride + stride) % stride; q < nq; q += stride) {
-    const uint32_t d = net.gl_desc[q0 + q];
-    if (d == ~0u) continue;
-    double J0, J1;
-    gather_pair_any(net, coef, drate, (int64_t)(net.nr + 1) * net.T, q0 + q, J0, J1);
-    store((int)((d >> 16) & 0x7fu), (int)(d >> 23), J0, J1);
-  }
-}
-
-// Rates of both layers without drates (the stage-2 right-hand side).
-template <int TT>
-__device__ inline void rates_pair_rhs_t(const NetDev& net, const double* y0, const double* y1, const double* kcol,
-                                        int64_t kstride, bool two, double M0, double M1, double* rate) {
-  const int R = net.nr + 1;
-  constexpr int RU = 2;
-  for (int r0 = threadIdx.x; r0 < R; r0 += RU * blockDim.x) {
-    double kv[RU][2];
-#pragma unroll
-    for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
-      kv[u][0] = r < R ? __ldcg(kcol + (int64_t)r * kstride) : 0.0;
-      kv[u][1] = (two && r < R) ? __ldcg(kcol + (int64_t)r * kstride + 1) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
-      if (r < R) {
-        rate_slot<TT>(load_slot<TT>(net, r), r, y0, kv[u][0], M0, rate, nullptr, false);
-        if (two) rate_slot<TT>(load_slot<TT>(net, r), r, y1, kv[u][1], M1, rate + R, nullptr, false);
-      }
-    }
-  }
-}
-
-// Stage-2 right-hand side for layers j0 = 2 blockIdx.x and j0 + 1 (the rates
-// and species sums of stage2_kernel, gather words shared by the pair; every
-// value bit-identical to the one-layer kernel's).
-__host__ __device__ inline size_t pair2_smem_bytes(int ni, int nr) {
-  return (4 * (size_t)(ni + 1) + 2 * (size_t)(nr + 1) + 8 * (size_t)ni + 8) * sizeof(double);
-}
-
-__global__ void __launch_bounds__(PAIR_THREADS, 4)
-stage2_pair_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
-                   const double* __restrict__ dt, const double* __restrict__ atm, int flags,
-                   const uint8_t* __restrict__ fix_mask, double* __restrict__ ws) {
-  extern __shared__ double smem[];
-  const int b = blockIdx.y, j0 = 2 * blockIdx.x;
-  Geo g = geo_of(B, b);
-  if (j0 >= g.nz) return;
-  const int ni = B.ni, nz = g.nz, R = B.nr + 1;
-  const bool two = j0 + 1 < nz;
-  double* y4 = smem;
-  double* rate = y4 + 4 * (ni + 1);
-  double* diff = rate + 2 * R;
-  double* part = diff + 2 * ni;
-  double* scal = part + 4 * ni;
-  AtmRef a = atm_ref(atm + g.atm, nz, ni);
-  WsView w = ws_view(ws, g, ni, B.ld);
-  const double* yb = y + g.z0 * ni;
-  const double r = ros2_r();
-  const double dtb = dt[b];
-  __shared__ double coefs[MAX_COEF];
-  load_coefs(net, coefs);
-  // rows j0-1 .. j0+2 of yk2 = y + k1/r (load_rows' expression) and their gas sums
-  for (int t = threadIdx.x; t < 4 * (ni + 1); t += blockDim.x) {
-    const int wr = t / (ni + 1), i = t % (ni + 1), jj = j0 - 1 + wr;
-    double v = 1.0;
-    if (i < ni) {
-      if (jj >= 0 && jj < nz) {
-        v = yb[(int64_t)jj * ni + i];
-        v = v + w.k1[(int64_t)jj * ni + i] / r;
-      } else {
-        v = 0.0;
-      }
-    }
-    y4[t] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    const int wr = threadIdx.x, jj = j0 - 1 + wr;
-    scal[wr] = (jj >= 0 && jj < nz) ? pairwise_sum_masked(y4 + wr * (ni + 1), a.gas, ni) : 0.0;
-  }
-  __syncthreads();
-  for (int l = 0; l < 2; ++l) {
-    if (l == 1 && !two) break;
-    LayerSmem L;
-    L.y3 = y4 + l * (ni + 1);
-    L.scal = scal + l;
-    L.diff = diff + l * ni;
-    L.diagd = nullptr;
-    layer_diffusion<2>(a, nz, ni, j0 + l, flags, L, nullptr, nullptr, false, l > 0);
-  }
-  {
-    const double* kcol = k + g.z0 * R + j0;
-    const double M0 = a.M[j0], M1 = two ? a.M[j0 + 1] : 0.0;
-    switch (net.T) {
-      case 1: rates_pair_rhs_t<1>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 2: rates_pair_rhs_t<2>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 3: rates_pair_rhs_t<3>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 4: rates_pair_rhs_t<4>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 5: rates_pair_rhs_t<5>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 6: rates_pair_rhs_t<6>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      case 7: rates_pair_rhs_t<7>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-      default: rates_pair_rhs_t<8>(net, y4 + (ni + 1), y4 + 2 * (ni + 1), kcol, nz, two, M0, M1, rate); break;
-    }
-  }
-  __syncthreads();
-  species_sums_pair(net, coefs, rate, part);
-  __syncthreads();
-  for (int t = threadIdx.x; t < 2 * ni; t += blockDim.x) {
-    const int l = t / ni, i = t - l * ni, j = j0 + l;
-    if (l == 1 && !two) break;
-    const double* pt = part + l * 2 * ni;
-    double v = (pt[2 * i + 1] - pt[2 * i]) + diff[l * ni + i];
-    const uint8_t* fm = fix_mask ? fix_mask + g.z0 * ni + (int64_t)j * ni : nullptr;
-    if (fm && fm[i]) v = 0.0;
-    const double k1v = w.k1[(int64_t)j * ni + i];
-    w.rmod[(int64_t)j * ni + i] = v - (2.0 / (r * dtb)) * k1v;
-  }
-}
-
-__global__ void __launch_bounds__(PAIR_THREADS, 2)
-stage1_pair_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
-                   const double* __restrict__ dt, const double* __restrict__ atm, int flags,
-                   const uint8_t* __restrict__ fix_mask, double* __restrict__ ws) {
-  extern __shared__ double smem[];
-  const int b = blockIdx.y, j0 = 2 * blockIdx.x;
-  Geo g = geo_of(B, b);
-  if (j0 >= g.nz) return;
-  const int ni = B.ni, nz = g.nz, ld = B.ld;
-  const bool two = j0 + 1 < nz;
-  PairSmem P = carve_pair(smem, ni, B.nr, net.T);
-  AtmRef a = atm_ref(atm + g.atm, nz, ni);
-  WsView w = ws_view(ws, g, ni, ld);
-  const double* yb = y + g.z0 * ni;
-  const double r = ros2_r();
-  const double c0 = 1.0 / (r * dt[b]);
-  __shared__ double coefs[MAX_COEF];
-  load_coefs(net, coefs);
-  // rows j0-1 .. j0+2 and their gas sums
-  for (int t = threadIdx.x; t < 4 * (ni + 1); t += blockDim.x) {
-    const int wr = t / (ni + 1), i = t % (ni + 1), jj = j0 - 1 + wr;
-    double v = 1.0;
-    if (i < ni) v = (jj >= 0 && jj < nz) ? yb[(int64_t)jj * ni + i] : 0.0;
-    P.y4[t] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    const int wr = threadIdx.x, jj = j0 - 1 + wr;
-    P.scal[wr] = (jj >= 0 && jj < nz) ? pairwise_sum_masked(P.y4 + wr * (ni + 1), a.gas, ni) : 0.0;
-  }
-  __syncthreads();
-  // diffusion of each layer (layer_diffusion on a one-layer view of the rows)
-  for (int l = 0; l < 2; ++l) {
-    if (l == 1 && !two) break;
-    LayerSmem L;
-    L.y3 = P.y4 + l * (ni + 1);
-    L.scal = P.scal + l;
-    L.diff = P.diff + l * ni;
-    L.diagd = P.diagd + l * ni;
-    layer_diffusion(a, nz, ni, j0 + l, flags, L, P.supb + l * ni, P.subb + l * ni, true, l > 0);
-  }
-  rates_pair(net, P.y4 + (ni + 1), P.y4 + 2 * (ni + 1), k + g.z0 * (B.nr + 1) + j0, nz, two, a.M[j0],
-             two ? a.M[j0 + 1] : 0.0, P.rate, P.drate);
-  __syncthreads();
-  species_sums_pair(net, coefs, P.rate, P.part);
-  double* blk0 = w.inv + (int64_t)j0 * ni * ld;
-  double* blk1 = blk0 + (int64_t)ni * ld;
-  const uint8_t* fm0 = fix_mask ? fix_mask + g.z0 * ni + (int64_t)j0 * ni : nullptr;
-  const uint8_t* fm1 = fm0 ? fm0 + ni : nullptr;
-  const double bot = (j0 == 0 && (flags & VB_USE_BOTFLUX)) ? 1.0 : 0.0;
-  jacobian_pair(net, coefs, P.drate, [&](int row, int col, double J0, double J1) {
-    double v = (row == col ? c0 : 0.0) - J0;
-    if (row == col) {
-      double dd = P.diagd[row];
-      if (j0 == 0) dd = dd + (bot != 0.0 ? -a.vdep[row] / a.dzi[0] : 0.0);
-      v = v + (-dd);
-    }
-    if (fm0 && fm0[row]) v = (row == col) ? c0 : 0.0;
-    blk0[(int64_t)row * ld + col] = v;
-    if (two) {
-      double v1 = (row == col ? c0 : 0.0) - J1;
-      if (row == col) v1 = v1 + (-P.diagd[ni + row]);
-      if (fm1 && fm1[row]) v1 = (row == col) ? c0 : 0.0;
-      blk1[(int64_t)row * ld + col] = v1;
-    }
-  }, min(2 * ni, (int)blockDim.x));
-  __syncthreads();   // the species sums
-  for (int t = threadIdx.x; t < 2 * ni; t += blockDim.x) {
-    const int l = t / ni, i = t - l * ni, j = j0 + l;
-    if (l == 1 && !two) break;
-    const double* part = P.part + l * 2 * ni;
-    const uint8_t* fm = l ? fm1 : fm0;
-    double v = (part[2 * i + 1] - part[2 * i]) + P.diff[l * ni + i];
-    const bool fixed = fm && fm[i];
-    if (fixed) v = 0.0;
-    w.rmod[(int64_t)j * ni + i] = v;
-    if (j < nz - 1) {
-      double s2 = -P.supb[l * ni + i];
-      if (fixed) s2 = 0.0;
-      w.supn[(int64_t)j * ni + i] = s2;
-    }
-    if (j > 0) {
-      double s2 = -P.subb[l * ni + i];
-      if (fixed) s2 = 0.0;
-      w.subn[(int64_t)(j - 1) * ni + i] = s2;
-    }
-  }
+__host__ __device__ inline size_t stage2_smem_bytes(int ni, int nr, int NL) {
+  return (size_t)NL * ((size_t)(nr + 1) + 2 * (size_t)ni + (ni + 1)) * sizeof(double);
 }
 
 // Stage-2 right-hand side: rmod[j] = rhs(yk2) - 2/(r dt) k1[j] with
-// yk2 = y + k1/r (jax_step.py:303-310). No drate buffer, so eight CTAs fit an
-// SM; occupancy, not per-thread ILP, hides the gathers' latency (measured on
-// B200, ni=69, nr=1400, 296 atmospheres: 3 / 4 / 5 / 6 CTAs per SM 2.22 /
-// 1.87 / 1.70 / 1.57 ms; 8 with rate constants loaded 2 deep instead of 6:
-// 1.53 ms, despite the spills at 32 registers).
-__global__ void __launch_bounds__(LAYER_THREADS, 8)
+// yk2 = y + k1/r (jax_step.py:303-310), of layers j .. j + NL - 1. No drate
+// buffer, so eight CTAs of one layer fit an SM; occupancy, not per-thread ILP,
+// hides the gathers' latency (measured on B200, ni=69, nr=1400, 296
+// atmospheres: 3 / 4 / 5 / 6 CTAs per SM 2.22 / 1.87 / 1.70 / 1.57 ms; 8 with
+// rate constants loaded 2 deep instead of 6: 1.53 ms, despite the spills at 32
+// registers).
+template <int NL>
+__global__ void __launch_bounds__(NL * LAYER_THREADS, 8 / NL)
 stage2_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
-              const double* __restrict__ dt, const double* __restrict__ atm, int flags,
+              const double* __restrict__ dt, const double* __restrict__ atm,
               const uint8_t* __restrict__ fix_mask, double* __restrict__ ws, double* __restrict__ resid) {
   extern __shared__ double smem[];
-  const int b = blockIdx.y, j = blockIdx.x;
+  const int b = blockIdx.y, j = NL * blockIdx.x;
   Geo g = geo_of(B, b);
   if (j >= g.nz) return;
   const int ni = B.ni, nz = g.nz;
-  LayerSmem L = carve(smem, ni, B.nr, net.T, false);
+  const int nl = min(NL, nz - j), last = nl - 1;   // layers here; a missing one repeats the last
+  double* rate = smem;                        // [nr+1][NL]
+  double* part = rate + NL * (B.nr + 1);      // [2 ni][NL]
+  double* yj = part + NL * 2 * ni;            // [NL][ni+1]
   AtmRef a = atm_ref(atm + g.atm, nz, ni);
   WsView w = ws_view(ws, g, ni, B.ld);
   const double* yb = y + g.z0 * ni;
@@ -951,69 +676,88 @@ stage2_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   const bool res = resid != nullptr;   // steady-state residual f(y) (steady_state_grad.py:116-130)
   const double dtb = res ? 1.0 : dt[b];
 
-  __shared__ double coefs[MAX_COEF];
+  __shared__ double coefs[MAX_COEF + 1];
   load_coefs(net, coefs);
-  // state row j (yk2 = y + k1/r, load_rows' expression; padding slot 1.0)
-  double* yj = L.y3 + (ni + 1);
-  for (int t = threadIdx.x; t <= ni; t += blockDim.x) {
-    double v = 1.0;
-    if (t < ni) {
-      v = yb[(int64_t)j * ni + t];
-      if (!res) v = v + w.k1[(int64_t)j * ni + t] / r;
+  // state rows (yk2 = y + k1/r; padding slot 1.0)
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    const int64_t q = (int64_t)(j + min(l, last)) * ni;
+    for (int t = threadIdx.x; t <= ni; t += blockDim.x) {
+      double v = 1.0;
+      if (t < ni) {
+        v = yb[q + t];
+        if (!res) v = v + w.k1[q + t] / r;
+      }
+      yj[l * (ni + 1) + t] = v;
     }
-    yj[t] = v;
   }
   __syncthreads();
-  layer_rates(net, yj, k + g.z0 * (B.nr + 1) + j, nz, a.M[j], L.rate, nullptr, false);
+  double M[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) M[l] = a.M[j + min(l, last)];
+  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, rate, nullptr, false);
   __syncthreads();
-  species_sums(net, coefs, L.rate, L.part);
+  species_sums<NL>(net, coefs, rate, part);
   __syncthreads();
   // rmod[j] (resid[j]) holds the row's diffusion term (diffusion_rows_kernel)
   const double* dif = res ? resid + g.z0 * ni : w.rmod;
-  for (int i = threadIdx.x; i < ni; i += blockDim.x) {
-    double v = (L.part[2 * i + 1] - L.part[2 * i]) + dif[(int64_t)j * ni + i];
+  for (int t = threadIdx.x; t < nl * ni; t += blockDim.x) {
+    const int l = t >= ni ? 1 : 0, i = t - l * ni;
+    const int64_t q = (int64_t)j * ni + t;
+    double v = (part[NL * (2 * i + 1) + l] - part[NL * 2 * i + l]) + dif[q];
     if (res) {
-      resid[g.z0 * ni + (int64_t)j * ni + i] = v;
+      resid[g.z0 * ni + q] = v;
       continue;
     }
-    if (fm && fm[i]) v = 0.0;
-    double k1v = w.k1[(int64_t)j * ni + i];
-    w.rmod[(int64_t)j * ni + i] = v - (2.0 / (r * dtb)) * k1v;
+    if (fm && fm[t]) v = 0.0;
+    w.rmod[q] = v - (2.0 / (r * dtb)) * w.k1[q];
   }
 }
 
 // Standalone chemistry: dydt (and optionally the Jacobian) of a uniform batch.
+__host__ __device__ inline size_t chem_smem_bytes(int ni, int nr, int T, bool jac) {
+  return ((size_t)(nr + 1) + 2 * (size_t)ni + (ni + 1) + (jac ? (size_t)(nr + 1) * T + 1 + (size_t)ni * ni : 0)) *
+         sizeof(double);
+}
+
 __global__ void __launch_bounds__(LAYER_THREADS)
 chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __restrict__ M,
             const double* __restrict__ k, double* __restrict__ dydt, double* __restrict__ jac) {
   extern __shared__ double smem[];
   const int b = blockIdx.y, j = blockIdx.x;
   const int ni = net.ni;
-  bool want_jac = jac != nullptr;
-  LayerSmem L = carve(smem, ni, net.nr, net.T, want_jac, want_jac);
+  const bool want_jac = jac != nullptr;
+  double* rate = smem;                            // [nr+1]
+  double* part = rate + (net.nr + 1);             // [2 ni]
+  double* yj = part + 2 * ni;                     // [ni+1]
+  double* drate = yj + (ni + 1);                  // [(nr+1)*T + 1]
+  double* J = drate + (net.nr + 1) * net.T + 1;   // [ni][ni]
   const double* yrow = y + ((int64_t)b * nz + j) * ni;
-  __shared__ double coefs[MAX_COEF];
+  __shared__ double coefs[MAX_COEF + 1];
   __shared__ int queue;
-  if (threadIdx.x == 0) queue = 0;
+  if (threadIdx.x == 0) {
+    queue = 0;
+    if (want_jac) drate[(net.nr + 1) * net.T] = 0.0;
+  }
   load_coefs(net, coefs);
-  for (int i = threadIdx.x; i <= ni; i += blockDim.x) L.y3[i] = i < ni ? yrow[i] : 1.0;
+  for (int i = threadIdx.x; i <= ni; i += blockDim.x) yj[i] = i < ni ? yrow[i] : 1.0;
   __syncthreads();
-  layer_rates(net, L.y3, k + (int64_t)b * (net.nr + 1) * nz + j, nz, M[(int64_t)b * nz + j], L.rate,
-              L.drate, want_jac);
+  const double Mj[1] = {M[(int64_t)b * nz + j]};
+  layer_rates<1>(net, yj, 0, k + (int64_t)b * (net.nr + 1) * nz + j, nz, 0, Mj, rate, drate, want_jac);
   __syncthreads();
   if (want_jac)
-    gather_layer(
-        net, coefs, L.rate, L.drate, true, &queue, L.part, [&](int row, double J) { L.jac[row * ni + row] = J; },
-        [&](int row, int col, double J) { L.jac[row * ni + col] = J; });
+    gather_layer<1>(
+        net, coefs, rate, drate, true, &queue, part, [&](int row, const double (&v)[1]) { J[row * ni + row] = v[0]; },
+        [&](int row, int col, const double (&v)[1]) { J[row * ni + col] = v[0]; });
   else
-    species_sums(net, coefs, L.rate, L.part);
+    species_sums<1>(net, coefs, rate, part);
   __syncthreads();
   if (dydt)
     for (int i = threadIdx.x; i < ni; i += blockDim.x)
-      dydt[((int64_t)b * nz + j) * ni + i] = L.part[2 * i + 1] - L.part[2 * i];
+      dydt[((int64_t)b * nz + j) * ni + i] = part[2 * i + 1] - part[2 * i];
   if (want_jac) {
     double* out = jac + ((int64_t)b * nz + j) * ni * ni;
-    for (int d = threadIdx.x; d < ni * ni; d += blockDim.x) out[d] = L.jac[d];
+    for (int d = threadIdx.x; d < ni * ni; d += blockDim.x) out[d] = J[d];
   }
 }
 
@@ -1024,14 +768,14 @@ diffusion_kernel(int nz, int ni, const double* __restrict__ y, const double* __r
                  double* __restrict__ sup_d, double* __restrict__ sub_d) {
   extern __shared__ double smem[];
   const int b = blockIdx.y, j = blockIdx.x;
-  LayerSmem L = carve(smem, ni, 0, 1, false);
+  LayerSmem L = carve(smem, ni);
   AtmRef a = atm_ref(atm + (int64_t)b * VB_ATM_DOUBLES(nz, ni), nz, ni);
   const double* yb = y + (int64_t)b * nz * ni;
-  load_rows<true>(yb, nullptr, a.gas, nz, ni, j, 1.0, false, L);
+  load_rows(yb, a.gas, nz, ni, j, L);
   __syncthreads();
   double* supo = sup_d ? sup_d + ((int64_t)b * (nz - 1) + j) * ni : nullptr;
   double* subo = sub_d ? sub_d + ((int64_t)b * (nz - 1) + (j - 1)) * ni : nullptr;
-  layer_diffusion(a, nz, ni, j, flags, L, supo, subo, true);
+  layer_diffusion(a, nz, ni, j, flags, L, supo, subo);
   __syncthreads();
   for (int i = threadIdx.x; i < ni; i += blockDim.x) {
     if (diff) diff[((int64_t)b * nz + j) * ni + i] = L.diff[i];
@@ -1085,7 +829,7 @@ diffusion_rows_kernel(Batch B, const double* __restrict__ y, const double* __res
   const AtmRef a = atm_ref(atm + g.atm, nz, ni);
   const WsView w = ws_view(ws, g, ni, B.ld);
   const double* yb = y + g.z0 * ni;
-  const bool yk2 = mode == 2 && !resid;   // stage 2: rows of yk2 = y + k1/r (load_rows' expression)
+  const bool yk2 = mode == 2 && !resid;   // stage 2: rows of yk2 = y + k1/r
   const double r = ros2_r();
   for (int t = threadIdx.x; t < NR * rs; t += blockDim.x) {
     const int rr = t / rs, i = t % rs, jj = jb - 1 + rr;
@@ -1244,7 +988,7 @@ lv_rates_kernel(NetDev net, Batch B, const double* __restrict__ y, const double*
 __global__ void __launch_bounds__(LV_LAYERS)
 lv_sums_kernel(NetDev net, Batch B, const double* __restrict__ dt, const uint8_t* __restrict__ fix_mask,
                double* __restrict__ ws) {
-  __shared__ double coefs[MAX_COEF];
+  __shared__ double coefs[MAX_COEF + 1];
   load_coefs(net, coefs);
   __syncthreads();
   const int i = blockIdx.x, b = blockIdx.y;
@@ -1284,14 +1028,18 @@ lv_sums_kernel(NetDev net, Batch B, const double* __restrict__ dt, const uint8_t
   }
 }
 
-// Reaction chunks per atmosphere of lv_rates_kernel: about two waves of
-// three 512-thread CTAs per SM, at least 8 reaction slots per chunk.
-static int lv_rate_chunks(const Batch& B) {
+static int sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
     sms = 148;
-  const int want = (6 * sms + B.count - 1) / B.count;
+  return sms;
+}
+
+// Reaction chunks per atmosphere of lv_rates_kernel: about two waves of
+// three 512-thread CTAs per SM, at least 8 reaction slots per chunk.
+static int lv_rate_chunks(const Batch& B) {
+  const int want = (6 * sm_count() + B.count - 1) / B.count;
   return std::max(1, std::min(want, (B.nr + 1) / 8));
 }
 
@@ -1322,62 +1070,70 @@ static cudaError_t launch_lv_stage2(const NetDev& net, const Batch& B, const dou
 }
 
 // ---------------------------------------------------------------- launchers
-// Stage-1 / stage-2 kernels of the Ros2 step (VbTuning.stage1_layers): one
-// layer per CTA by default (measured on B200 at 296 config-0 atmospheres, the
-// two-layer kernels make the step 13.08 ms against 12.81: the gather latency
-// is hidden better by more resident CTAs than by two chains per thread).
-static constexpr int kStage1DefaultLayers = 1;
+// Layers per CTA of the stage-1 assembly (VbTuning.stage1_layers, or by size).
+// Two layers read every gather word, descriptor and rate-constant sector once
+// for both, but halve the CTAs that hide each other's phases. Measured on
+// B200, one / two layers, stage 1 with the diffusion rows: networks whose
+// one-layer CTAs (a layer's drates) no longer fit four to an SM: 1.91 / 1.73 ms
+// (89 species, 2,000 reactions, 19,200 layers), 0.232 / 0.197 (128, 3,000,
+// 960 layers); that fit four but leave L1 under 40 KB: 2.02 / 1.98 (69, 1,400,
+// 35,520 layers) yet 0.149 / 0.152 at 1,920 layers; smaller ones 0.266 / 0.269
+// (64, 1,000) and 0.251 / 0.278 (30, 370, 256 atmospheres of 43 layers).
+static int stage1_layers(const NetDev& net, const Batch& B) {
+  if (B.stage1_layers) return B.stage1_layers;
+  const size_t per_sm = 228 * 1024, l1 = 40 * 1024;
+  const size_t cta = stage1_smem_bytes(B.ni, B.nr, net.T, 1) + (MAX_COEF + 1) * sizeof(double) + 1024;
+  if (stage1_smem_bytes(B.ni, B.nr, net.T, 2) > per_sm - 4096 || 4 * cta + l1 <= per_sm) return 1;
+  const int64_t least = 4 * cta > per_sm ? 4 : 16;   // layers per SM
+  return (int64_t)B.count * B.nz >= least * sm_count() ? 2 : 1;
+}
+
+template <int NL>
+static cudaError_t launch_stage1_t(const NetDev& net, const Batch& B, const double* y, const double* k,
+                                   const double* dt, const double* atm, int flags, const uint8_t* fm, double* ws,
+                                   cudaStream_t st, const double* adj_v) {
+  const size_t sm = stage1_smem_bytes(B.ni, B.nr, net.T, NL);
+  cudaError_t e = cudaFuncSetAttribute(stage1_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  stage1_kernel<NL><<<dim3((B.nz + NL - 1) / NL, B.count), NL * LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags,
+                                                                                         fm, ws, adj_v);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_stage1(const NetDev& net, const Batch& B, const double* y, const double* k,
                           const double* dt, const double* atm, int flags, const uint8_t* fm, double* ws,
                           cudaStream_t st, const double* adj_v) {
-  const int layers = B.stage1_layers ? B.stage1_layers : kStage1DefaultLayers;
-  if (!adj_v && layers == 2) {
-    size_t sm = pair_smem_bytes(B.ni, B.nr, net.T);
-    cudaError_t e = cudaFuncSetAttribute(stage1_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    dim3 grid((B.nz + 1) / 2, B.count);
-    stage1_pair_kernel<<<grid, PAIR_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags, fm, ws);
-    return cudaGetLastError();
-  }
   cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, nullptr, adj_v ? 1 : 0, st);
   if (e != cudaSuccess) return e;
-  size_t sm = layer_smem_bytes(B.ni, B.nr, net.T, true);
-  cudaFuncSetAttribute(stage1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  dim3 grid(B.nz, B.count);
-  stage1_kernel<<<grid, LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags, fm, ws, adj_v);
+  return stage1_layers(net, B) == 2 ? launch_stage1_t<2>(net, B, y, k, dt, atm, flags, fm, ws, st, adj_v)
+                                    : launch_stage1_t<1>(net, B, y, k, dt, atm, flags, fm, ws, st, adj_v);
+}
+
+template <int NL>
+static cudaError_t launch_stage2_t(const NetDev& net, const Batch& B, const double* y, const double* k,
+                                   const double* dt, const double* atm, const uint8_t* fm, double* ws,
+                                   cudaStream_t st, double* resid) {
+  const size_t sm = stage2_smem_bytes(B.ni, B.nr, NL);
+  cudaError_t e = cudaFuncSetAttribute(stage2_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  stage2_kernel<NL><<<dim3((B.nz + NL - 1) / NL, B.count), NL * LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, fm, ws,
+                                                                                         resid);
   return cudaGetLastError();
 }
 
 cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, const double* k,
                           const double* dt, const double* atm, int flags, const uint8_t* fm, double* ws,
                           cudaStream_t st, double* resid) {
-  const int layers = B.stage1_layers ? B.stage1_layers : kStage1DefaultLayers;
-  if (B.rates && !resid && layers != 2) {
-    cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, nullptr, 2, st);
-    if (e == cudaSuccess) e = launch_lv_stage2(net, B, y, k, dt, atm, fm, ws, st);
-    return e;
-  }
-  if (!resid && layers == 2) {
-    size_t sm = pair2_smem_bytes(B.ni, B.nr);
-    cudaError_t e = cudaFuncSetAttribute(stage2_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    dim3 grid((B.nz + 1) / 2, B.count);
-    stage2_pair_kernel<<<grid, PAIR_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags, fm, ws);
-    return cudaGetLastError();
-  }
   cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, resid, 2, st);
   if (e != cudaSuccess) return e;
-  size_t sm = layer_smem_bytes(B.ni, B.nr, net.T, false);
-  cudaFuncSetAttribute(stage2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  dim3 grid(B.nz, B.count);
-  stage2_kernel<<<grid, LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags, fm, ws, resid);
-  return cudaGetLastError();
+  if (!resid && B.stage1_layers == 2) return launch_stage2_t<2>(net, B, y, k, dt, atm, fm, ws, st, resid);
+  if (!resid && B.rates) return launch_lv_stage2(net, B, y, k, dt, atm, fm, ws, st);
+  return launch_stage2_t<1>(net, B, y, k, dt, atm, fm, ws, st, resid);
 }
 
 cudaError_t launch_chem(const NetDev& net, int batch, int nz, const double* y, const double* M,
                         const double* k, double* dydt, double* jac, cudaStream_t st) {
-  size_t sm = layer_smem_bytes(net.ni, net.nr, net.T, jac != nullptr, jac != nullptr);
+  size_t sm = chem_smem_bytes(net.ni, net.nr, net.T, jac != nullptr);
   cudaFuncSetAttribute(chem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid(nz, batch);
   chem_kernel<<<grid, LAYER_THREADS, sm, st>>>(net, nz, y, M, k, dydt, jac);
@@ -1387,7 +1143,7 @@ cudaError_t launch_chem(const NetDev& net, int batch, int nz, const double* y, c
 cudaError_t launch_diffusion(int batch, int nz, int ni, const double* y, const double* atm, int flags,
                              double* diff, double* diag_d, double* sup_d, double* sub_d,
                              cudaStream_t st) {
-  size_t sm = layer_smem_bytes(ni, 0, 1, false);
+  size_t sm = layer_smem_bytes(ni);
   dim3 grid(nz, batch);
   diffusion_kernel<<<grid, LAYER_THREADS, sm, st>>>(nz, ni, y, atm, flags, diff, diag_d, sup_d, sub_d);
   return cudaGetLastError();

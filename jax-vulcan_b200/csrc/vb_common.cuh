@@ -7,7 +7,7 @@
 
 namespace vb {
 
-constexpr int GL_SHORT = 4;   // longest Jacobian list with code of its own
+constexpr int GL_SHORT = 4;   // longest Jacobian list with code of its own (reason: vb_chem.cu, gather_short)
 constexpr int RX_TERMS = 6;   // reactant slots that fit a packed reaction word
 
 // Code of a stoichiometry: 0, 1, 2, or 3 for any other value.
@@ -32,7 +32,7 @@ struct NetDev {
   // bits give the coefficient: the top half of the double's high word where
   // every coefficient of the network is zero below it (coef_packed; whole and
   // half stoichiometries are), else its id in coef_tab (<= 256 distinct ones).
-  // The lists, in groups of 32 of falling term count (ties: increasing index):
+  // The lists, in groups of 32, by falling term count (ties: increasing index):
   // * the 2 ni species lists, t = 2 i (loss) or 2 i + 1 (production) of
   //   species i: the (r*T+s) slots whose reactant (loss) or product index is
   //   i, in increasing flat order (segment_sum order), with r_st or p_st;
@@ -41,17 +41,17 @@ struct NetDev {
   //   -r_st[r][o] (o < T) or p_st[r][o-T].
   // Groups [0, gl_sums) hold the species lists, [gl_sums, gl_diag) the
   // diagonal entries, [gl_diag, gl_long) the off-diagonal entries of more than
-  // GL_SHORT terms, and [gl_first[c], gl_first[c] + gl_count[c]) those of
-  // exactly c <= GL_SHORT terms (the last group of each kind padded with
-  // lanes whose descriptor is ~0). The words of a group are interleaved and
+  // GL_SHORT terms, [gl_long, gl_groups) the others, by increasing entry and
+  // each filled up to GL_SHORT terms with the index (nr+1)*T (a drate of 0) and
+  // a finite coefficient, which change no sum. The last group of a kind has
+  // lanes whose descriptor is ~0. The words of a group are interleaved and
   // padded (with 0) to its longest list: term k of lane l of group g at
   // gl_w[gl_base[g] + 32 k + l], so a warp that holds a group loads one line
   // per term.
-  const uint32_t* gl_base;       // [groups + 1]
-  const uint32_t* gl_desc;       // [32 groups]: count | t << 16, or count | row << 16 | col << 23
+  const uint32_t* gl_base;       // [gl_groups + 1]
+  const uint32_t* gl_desc;       // [32 gl_groups]: count | t << 16, or count | row << 16 | col << 23
   const uint32_t* gl_w;
-  int gl_sums, gl_diag, gl_long;
-  int gl_first[GL_SHORT + 1], gl_count[GL_SHORT + 1];
+  int gl_sums, gl_diag, gl_long, gl_groups;
   const double* coef_tab;        // [n_coef]
   int n_coef, coef_packed;
   // The species lists in natural order, for the layer-vectorized stage 2
@@ -62,7 +62,7 @@ struct NetDev {
 };
 
 constexpr int LAYER_THREADS = 256;
-constexpr int MAX_COEF = 256;   // distinct stoichiometric coefficients of a network
+constexpr int MAX_COEF = 256;   // distinct stoichiometric coefficients of a network (and 0.0 for filled-up lists)
 
 // Term word of a gather table: index (low 16 bits) and the coefficient's
 // high half-word or id.

@@ -127,7 +127,7 @@ struct AtmPtrAcc {
 
 // The atmosphere fields stencil row j reads, staged before any arithmetic:
 // the per-layer fields of layers j-1, j, j+1 in shared memory (lay[f][s],
-// f = Kzz dzi vz Hpi Ti Tco g, s = layer - (j-1); stage_row_layers) and one
+// f = Kzz dzi vz Hpi Ti Tco g, s = layer - (j-1)) and one
 // species' fields of layers j-1, j in registers. eddy_row_t and mol_row_t
 // read only those indices for row j (boundary rows included), so this
 // accessor returns the values AtmPtrAcc would, without their global-load
@@ -152,28 +152,8 @@ struct RowAcc {
   __device__ double alpha(int) const { return alpha_; }
 };
 
-// Fills lay[7][3] for row j (threads 0..20; layers outside [0, nz) read 0).
-__device__ inline void stage_row_layers(const AtmRef& a, int nz, int j, double* lay) {
-  if (threadIdx.x < 21) {
-    const int f = threadIdx.x / 3, m = j - 1 + (int)threadIdx.x % 3;
-    const double* src = f == 0 ? a.Kzz : f == 1 ? a.dzi : f == 2 ? a.vz : f == 3 ? a.Hpi : f == 4 ? a.Ti
-                      : f == 5 ? a.Tco : a.g;
-    lay[threadIdx.x] = (m >= 0 && m < nz) ? src[m] : 0.0;
-  }
-}
-
-// The staged per-layer fields only (lay[f][3] of row j; the eddy terms).
-__device__ inline RowAcc layer_acc(const double* lay, int j) {
-  RowAcc R{};
-  R.lay = lay;
-  R.j0 = j - 1;
-  R.base = j - 1;
-  R.S = 3;
-  return R;
-}
-
 // A species' fields of layers j-1 and j, loaded together (lay: per-layer
-// fields staged with f-stride S from layer base; a row's own stage: j-1, 3).
+// fields staged with f-stride S from layer base).
 __device__ inline RowAcc row_acc(const AtmRef& a, const double* lay, int ni, int j, int i, int base, int S) {
   RowAcc R;
   R.lay = lay;
