@@ -801,7 +801,8 @@ diffusion_kernel(int nz, int ni, const double* __restrict__ y, const double* __r
 //                      subn[j-1] = sub_d (steady_state_grad.py:153-175);
 //   mode 2 (stage 2):  rmod[j] = diff at yk2 = y + k1/r (with resid: resid[j]
 //                      = diff at y, the residual; ws unused).
-// Four CTAs per SM (64 registers, 32 bytes spilled): 0.239 ms per launch at
+// Four CTAs per SM (64 registers, 32 bytes spilled): 0.239 ms per launch, before
+// zero numerators were kept out of the divisions (0.117 since), at
 // 296 config-0 atmospheres on B200 against 0.261 with three (74 registers);
 // the items are chains of FP64 divisions, hidden by resident warps.
 constexpr int DIFF_THREADS = 256;
@@ -866,7 +867,7 @@ diffusion_rows_kernel(Batch B, const double* __restrict__ y, const double* __res
       E.base = jb - 1;
       E.S = NR;
       double A, Bc, C;
-      eddy_row_t<double>(E, nz, j, scal[l], scal[l + 1], scal[l + 2], A, Bc, C);
+      eddy_row_t(E, nz, j, scal[l], scal[l + 1], scal[l + 2], A, Bc, C);
       edd[3 * l] = A;
       edd[3 * l + 1] = Bc;
       edd[3 * l + 2] = C;
@@ -879,7 +880,7 @@ diffusion_rows_kernel(Batch B, const double* __restrict__ y, const double* __res
     const int l = q / ni, i = q % ni, j = jb + l;
     if (j >= nz) continue;
     double Am, Bm, Cm;
-    mol_row_t<double>(row_acc(a, lay, ni, j, i, jb - 1, NR), nz, j, i, scal[l], scal[l + 1], scal[l + 2], use_vm,
+    mol_row_t(row_acc(a, lay, ni, j, i, jb - 1, NR), nz, j, i, scal[l], scal[l + 1], scal[l + 2], use_vm,
                       use_set, Am, Bm, Cm);
     const double At = edd[3 * l] + Am;
     const double Bt = edd[3 * l + 1] + Bm;

@@ -82,8 +82,7 @@ __device__ __forceinline__ AtmRef atm_ref(const double* blob, int nz, int ni) {
   return a;
 }
 
-// Number types of the stencil formulas: double (the forward kernels) or
-// Dual (value + one derivative, for the adjoint's leaf cotangents).
+// Number type of a value with one derivative (the rate constants' d/dT).
 struct Dual {
   double v, d;
 };
@@ -104,8 +103,6 @@ __device__ __forceinline__ Dual operator/(Dual a, double b) { return {a.v / b, a
 __device__ __forceinline__ Dual operator/(double a, Dual b) { return {a / b.v, -a * b.d / (b.v * b.v)}; }
 __device__ __forceinline__ double value_of(double x) { return x; }
 __device__ __forceinline__ double value_of(Dual x) { return x.v; }
-template <typename T> __device__ __forceinline__ T pos_part_t(T v) { return (value_of(v) > 0.0 ? 1.0 : 0.0) * v; }
-template <typename T> __device__ __forceinline__ T neg_part_t(T v) { return (value_of(v) < 0.0 ? 1.0 : 0.0) * v; }
 
 // Plain reads of an atmosphere (the forward kernels).
 struct AtmPtrAcc {
@@ -172,110 +169,119 @@ __device__ inline RowAcc row_acc(const AtmRef& a, const double* lay, int ni, int
   return R;
 }
 
+// a / b. A zero numerator (no wind, no settling, no molecular diffusion) over a
+// finite nonzero b takes the product, whose value and sign are the quotient's,
+// instead of the division's out-of-range path: at 296 atmospheres of 69
+// species and 120 layers without molecular diffusion the rows kernel took
+// 0.239 ms with that path and 0.117 without.
+__device__ __forceinline__ double quot(double a, double b) {
+  return a == 0.0 && b != 0.0 && fabs(b) <= 1.7976931348623157e308 ? a * b : a / b;
+}
+
 // Eddy coefficients of stencil row j (reference jax_step.py:167-193).
-template <typename T, typename Acc>
-__device__ inline void eddy_row_t(const Acc& a, int nz, int j, double ysm, double ys0, double ysp, T& A, T& Bc,
-                                  T& C) {
+template <typename Acc>
+__device__ inline void eddy_row_t(const Acc& a, int nz, int j, double ysm, double ys0, double ysp, double& A, double& Bc,
+                                  double& C) {
   if (j == 0) {
     A = -1.0 / a.dzi(0) * (a.Kzz(0) / a.dzi(0)) * (ysp + ys0) / 2.0 / ys0;
-    A = A - pos_part_t(a.vz(0)) / a.dzi(0);
+    A = A - quot(pos_part(a.vz(0)), a.dzi(0));
     Bc = 1.0 / a.dzi(0) * (a.Kzz(0) / a.dzi(0)) * (ysp + ys0) / 2.0 / ysp;
-    Bc = Bc - neg_part_t(a.vz(0)) / a.dzi(0);
-    C = T{};
+    Bc = Bc - quot(neg_part(a.vz(0)), a.dzi(0));
+    C = 0.0;
   } else if (j == nz - 1) {
     int t = nz - 2;
     A = -1.0 / a.dzi(t) * (a.Kzz(t) / a.dzi(t)) * (ys0 + ysm) / 2.0 / ys0;
-    A = A + neg_part_t(a.vz(t)) / a.dzi(t);
+    A = A + quot(neg_part(a.vz(t)), a.dzi(t));
     C = 1.0 / a.dzi(t) * (a.Kzz(t) / a.dzi(t)) * (ys0 + ysm) / 2.0 / ysm;
-    C = C + pos_part_t(a.vz(t)) / a.dzi(t);
-    Bc = T{};
+    C = C + quot(pos_part(a.vz(t)), a.dzi(t));
+    Bc = 0.0;
   } else {
-    const auto dz_ave = 0.5 * (a.dzi(j - 1) + a.dzi(j));
+    const double dz_ave = 0.5 * (a.dzi(j - 1) + a.dzi(j));
     A = -1.0 / dz_ave *
         (a.Kzz(j) / a.dzi(j) * (ysp + ys0) / 2.0 + a.Kzz(j - 1) / a.dzi(j - 1) * (ys0 + ysm) / 2.0) / ys0;
     Bc = 1.0 / dz_ave * a.Kzz(j) / a.dzi(j) * (ysp + ys0) / 2.0 / ysp;
     C = 1.0 / dz_ave * a.Kzz(j - 1) / a.dzi(j - 1) * (ys0 + ysm) / 2.0 / ysm;
-    A = A - (pos_part_t(a.vz(j)) - neg_part_t(a.vz(j - 1))) / dz_ave;
-    Bc = Bc - neg_part_t(a.vz(j)) / dz_ave;
-    C = C + pos_part_t(a.vz(j - 1)) / dz_ave;
+    A = A - quot(pos_part(a.vz(j)) - neg_part(a.vz(j - 1)), dz_ave);
+    Bc = Bc - quot(neg_part(a.vz(j)), dz_ave);
+    C = C + quot(pos_part(a.vz(j - 1)), dz_ave);
   }
 }
 
 __device__ inline void eddy_row(const AtmRef& a, int nz, int j, double ysm, double ys0, double ysp,
                                 double& A, double& Bc, double& C) {
-  eddy_row_t<double>(AtmPtrAcc{a, 0}, nz, j, ysm, ys0, ysp, A, Bc, C);
+  eddy_row_t(AtmPtrAcc{a, 0}, nz, j, ysm, ys0, ysp, A, Bc, C);
 }
 
 // Gravity/thermal-diffusion factor of compute_diff_grav (jax_step.py:80-87):
 // -1/Hpi[h] + ms*g[gi]/(Navo*kb*Ti[h]) + alpha/Ti[h]*(Tco[t1]-Tco[t0])/dzi[h].
-template <typename T, typename Acc>
-__device__ __forceinline__ T grav_fac_t(const Acc& a, int i, int h, int gi, int t1, int t0) {
+template <typename Acc>
+__device__ __forceinline__ double grav_fac_t(const Acc& a, int i, int h, int gi, int t1, int t0) {
   return -1.0 / a.Hpi(h) + a.ms(i) * a.g(gi) / (NAVO * KB * a.Ti(h)) +
-         a.alpha(i) / a.Ti(h) * (a.Tco(t1) - a.Tco(t0)) / a.dzi(h);
+         quot(quot(a.alpha(i), a.Ti(h)) * (a.Tco(t1) - a.Tco(t0)), a.dzi(h));
 }
 
 // Molecular-diffusion coefficients of species i on stencil row j, including the
 // y-independent gravity / vm / settling pieces (jax_step.py:67-147, 195-218).
-template <typename T, typename Acc>
+template <typename Acc>
 __device__ inline void mol_row_t(const Acc& a, int nz, int j, int i, double ysm, double ys0, double ysp,
-                                 double use_vm, double use_set, T& A, T& Bc, T& C) {
+                                 double use_vm, double use_set, double& A, double& Bc, double& C) {
   if (j == 0) {
-    const T D0 = a.Dzz(0, i);
-    const T g0 = 1.0 / a.dzi(0) * D0 / 2.0 * grav_fac_t<T>(a, i, 0, 0, 1, 0);
-    const T vm0 = a.vm(0, i);
-    const T vs0 = a.vs(0, i);
-    const T b0_vm = -pos_part_t(vm0) / a.dzi(0);
-    const T b0_vm_B = -neg_part_t(vm0) / a.dzi(0);
-    const T b0_vs = -pos_part_t(vs0) / a.dzi(0);
-    const T b0_vs_B = -neg_part_t(vs0) / a.dzi(0);
-    const T bA = (1.0 - use_vm) * g0 + use_vm * b0_vm + use_set * b0_vs;
-    const T bB = (1.0 - use_vm) * g0 + use_vm * b0_vm_B + use_set * b0_vs_B;
-    A = -1.0 / a.dzi(0) * (D0 / a.dzi(0)) * (ysp + ys0) / 2.0 / ys0 + bA;
-    Bc = 1.0 / a.dzi(0) * (D0 / a.dzi(0)) * (ysp + ys0) / 2.0 / ysp + bB;
-    C = T{};
+    const double D0 = a.Dzz(0, i);
+    const double g0 = 1.0 / a.dzi(0) * D0 / 2.0 * grav_fac_t(a, i, 0, 0, 1, 0);
+    const double vm0 = a.vm(0, i);
+    const double vs0 = a.vs(0, i);
+    const double b0_vm = quot(-pos_part(vm0), a.dzi(0));
+    const double b0_vm_B = quot(-neg_part(vm0), a.dzi(0));
+    const double b0_vs = quot(-pos_part(vs0), a.dzi(0));
+    const double b0_vs_B = quot(-neg_part(vs0), a.dzi(0));
+    const double bA = (1.0 - use_vm) * g0 + use_vm * b0_vm + use_set * b0_vs;
+    const double bB = (1.0 - use_vm) * g0 + use_vm * b0_vm_B + use_set * b0_vs_B;
+    A = quot(-1.0 / a.dzi(0) * quot(D0, a.dzi(0)) * (ysp + ys0) / 2.0, ys0) + bA;
+    Bc = quot(1.0 / a.dzi(0) * quot(D0, a.dzi(0)) * (ysp + ys0) / 2.0, ysp) + bB;
+    C = 0.0;
   } else if (j == nz - 1) {
     const int t = nz - 2;
-    const T Dt = a.Dzz(t, i);
-    const T gt = -1.0 / a.dzi(t) * Dt / 2.0 * grav_fac_t<T>(a, i, t, nz - 1, nz - 1, nz - 2);
-    const T vmt = a.vm(nz - 1, i);
-    const T vst = a.vs(t, i);
-    const T bt_vm = neg_part_t(vmt) / a.dzi(t);
-    const T bt_vm_C = pos_part_t(vmt) / a.dzi(t);
-    const T bt_vs = neg_part_t(vst) / a.dzi(t);
-    const T bt_vs_C = pos_part_t(vst) / a.dzi(t);
-    const T bA = (1.0 - use_vm) * gt + use_vm * bt_vm + use_set * bt_vs;
-    const T bC = (1.0 - use_vm) * gt + use_vm * bt_vm_C + use_set * bt_vs_C;
-    A = -1.0 / a.dzi(t) * (Dt / a.dzi(t)) * (ys0 + ysm) / 2.0 / ys0 + bA;
-    C = 1.0 / a.dzi(t) * (Dt / a.dzi(t)) * (ys0 + ysm) / 2.0 / ysm + bC;
-    Bc = T{};
+    const double Dt = a.Dzz(t, i);
+    const double gt = -1.0 / a.dzi(t) * Dt / 2.0 * grav_fac_t(a, i, t, nz - 1, nz - 1, nz - 2);
+    const double vmt = a.vm(nz - 1, i);
+    const double vst = a.vs(t, i);
+    const double bt_vm = quot(neg_part(vmt), a.dzi(t));
+    const double bt_vm_C = quot(pos_part(vmt), a.dzi(t));
+    const double bt_vs = quot(neg_part(vst), a.dzi(t));
+    const double bt_vs_C = quot(pos_part(vst), a.dzi(t));
+    const double bA = (1.0 - use_vm) * gt + use_vm * bt_vm + use_set * bt_vs;
+    const double bC = (1.0 - use_vm) * gt + use_vm * bt_vm_C + use_set * bt_vs_C;
+    A = quot(-1.0 / a.dzi(t) * quot(Dt, a.dzi(t)) * (ys0 + ysm) / 2.0, ys0) + bA;
+    C = quot(1.0 / a.dzi(t) * quot(Dt, a.dzi(t)) * (ys0 + ysm) / 2.0, ysm) + bC;
+    Bc = 0.0;
   } else {
-    const T dz_ave = 0.5 * (a.dzi(j - 1) + a.dzi(j));
-    const T Dj = a.Dzz(j, i);
-    const T Dm = a.Dzz(j - 1, i);
-    const T gj = grav_fac_t<T>(a, i, j, j, j + 1, j);
-    const T gjm = grav_fac_t<T>(a, i, j - 1, j, j, j - 1);
-    const T gjpb = grav_fac_t<T>(a, i, j, j + 1, j + 1, j);
-    const T gjmc = grav_fac_t<T>(a, i, j - 1, j - 1, j, j - 1);
-    const T inv2 = 1.0 / (2.0 * dz_ave);
-    const T Ag = inv2 * (Dj * gj - Dm * gjm);
-    const T Bg = inv2 * Dj * gjpb;
-    const T Cg = -inv2 * Dm * gjmc;
-    const T vmj = a.vm(j, i), vmm = a.vm(j - 1, i);
-    const T vsj = a.vs(j, i), vsm = a.vs(j - 1, i);
-    const T Avm = -(pos_part_t(vmj) - neg_part_t(vmm)) / dz_ave;
-    const T Bvm = -neg_part_t(vmj) / dz_ave;
-    const T Cvm = pos_part_t(vmm) / dz_ave;
-    const T Avs = -(pos_part_t(vsj) - neg_part_t(vsm)) / dz_ave;
-    const T Bvs = -neg_part_t(vsj) / dz_ave;
-    const T Cvs = pos_part_t(vsm) / dz_ave;
-    const T Ax = (1.0 - use_vm) * Ag + use_vm * Avm + use_set * Avs;
-    const T Bx = (1.0 - use_vm) * Bg + use_vm * Bvm + use_set * Bvs;
-    const T Cx = (1.0 - use_vm) * Cg + use_vm * Cvm + use_set * Cvs;
-    A = -1.0 / dz_ave * (Dj / a.dzi(j) * (ysp + ys0) / 2.0 + Dm / a.dzi(j - 1) * (ys0 + ysm) / 2.0) / ys0;
+    const double dz_ave = 0.5 * (a.dzi(j - 1) + a.dzi(j));
+    const double Dj = a.Dzz(j, i);
+    const double Dm = a.Dzz(j - 1, i);
+    const double gj = grav_fac_t(a, i, j, j, j + 1, j);
+    const double gjm = grav_fac_t(a, i, j - 1, j, j, j - 1);
+    const double gjpb = grav_fac_t(a, i, j, j + 1, j + 1, j);
+    const double gjmc = grav_fac_t(a, i, j - 1, j - 1, j, j - 1);
+    const double inv2 = 1.0 / (2.0 * dz_ave);
+    const double Ag = inv2 * (Dj * gj - Dm * gjm);
+    const double Bg = inv2 * Dj * gjpb;
+    const double Cg = -inv2 * Dm * gjmc;
+    const double vmj = a.vm(j, i), vmm = a.vm(j - 1, i);
+    const double vsj = a.vs(j, i), vsm = a.vs(j - 1, i);
+    const double Avm = quot(-(pos_part(vmj) - neg_part(vmm)), dz_ave);
+    const double Bvm = quot(-neg_part(vmj), dz_ave);
+    const double Cvm = quot(pos_part(vmm), dz_ave);
+    const double Avs = quot(-(pos_part(vsj) - neg_part(vsm)), dz_ave);
+    const double Bvs = quot(-neg_part(vsj), dz_ave);
+    const double Cvs = quot(pos_part(vsm), dz_ave);
+    const double Ax = (1.0 - use_vm) * Ag + use_vm * Avm + use_set * Avs;
+    const double Bx = (1.0 - use_vm) * Bg + use_vm * Bvm + use_set * Bvs;
+    const double Cx = (1.0 - use_vm) * Cg + use_vm * Cvm + use_set * Cvs;
+    A = quot(-1.0 / dz_ave * (quot(Dj, a.dzi(j)) * (ysp + ys0) / 2.0 + quot(Dm, a.dzi(j - 1)) * (ys0 + ysm) / 2.0), ys0);
     A = A + Ax;
-    Bc = 1.0 / dz_ave * Dj / a.dzi(j) * (ysp + ys0) / 2.0 / ysp;
+    Bc = quot(quot(1.0 / dz_ave * Dj, a.dzi(j)) * (ysp + ys0) / 2.0, ysp);
     Bc = Bc + Bx;
-    C = 1.0 / dz_ave * Dm / a.dzi(j - 1) * (ys0 + ysm) / 2.0 / ysm;
+    C = quot(quot(1.0 / dz_ave * Dm, a.dzi(j - 1)) * (ys0 + ysm) / 2.0, ysm);
     C = C + Cx;
   }
 }
@@ -283,7 +289,7 @@ __device__ inline void mol_row_t(const Acc& a, int nz, int j, int i, double ysm,
 __device__ inline void mol_row(const AtmRef& a, int nz, int ni, int j, int i, double ysm, double ys0,
                                double ysp, double use_vm, double use_set, double& A, double& Bc,
                                double& C) {
-  mol_row_t<double>(AtmPtrAcc{a, ni}, nz, j, i, ysm, ys0, ysp, use_vm, use_set, A, Bc, C);
+  mol_row_t(AtmPtrAcc{a, ni}, nz, j, i, ysm, ys0, ysp, use_vm, use_set, A, Bc, C);
 }
 
 }  // namespace vb
