@@ -221,6 +221,15 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   add_lists(brief, [](uint32_t) { return (size_t)vb::GL_SHORT; },
             [&](uint32_t d, size_t i) { return i < jac_len(d) ? jac_word(d, i) : filler; }, jac_tag);
   if (gw.empty()) gw.push_back(0u);
+  std::vector<int32_t> any;
+  for (int r = 0; r < R; ++r)
+    for (int s = 0; s < T; ++s)
+      if (vb::st_code(r_st[(int64_t)r * T + s]) == 3u) {
+        any.push_back(r);
+        break;
+      }
+  const int n_any = (int)any.size();
+  if (any.empty()) any.push_back(0);
   std::vector<uint64_t> rx(R, 0);
   if (T <= vb::RX_TERMS)
     for (int r = 0; r < R; ++r) {
@@ -250,7 +259,7 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
       {three, (size_t)R, 0},         {gbase.data(), gbase.size() * 4, 0},
       {gdesc.data(), gdesc.size() * 4, 0}, {gw.data(), gw.size() * 4, 0},
       {coefs.data(), coefs.size() * 8, 0}, {snp.data(), snp.size() * 4, 0}, {snw.data(), snw.size() * 4, 0},
-      {rx.data(), rx.size() * 8, 0}};
+      {rx.data(), rx.size() * 8, 0}, {any.data(), any.size() * 4, 0}};
   size_t total = 0;
   for (auto& p : parts) { p.off = total; total += (p.bytes + 255) & ~(size_t)255; }
   void* base = nullptr;
@@ -283,6 +292,8 @@ int vb_net_create(int ni, int nr, int T, const int64_t* r_idx, const int64_t* p_
   d.sum_nptr = (const int32_t*)(b + parts[9].off);
   d.sum_nw = (const uint32_t*)(b + parts[10].off);
   d.rx = (const uint64_t*)(b + parts[11].off);
+  d.any_list = (const int32_t*)(b + parts[12].off);
+  d.n_any = n_any;
   net->base = base;
   net->bytes = total;
   *out = net;

@@ -128,10 +128,18 @@ __device__ __forceinline__ double rate_terms_p(const double (&yr)[TT], const Slo
   return rt;
 }
 
-// A stoichiometry other than 0, 1 and 2 in the slot: out of line, so that pow
-// takes neither registers nor instruction cache from the rest.
+// Whether a slot has a stoichiometry other than 0, 1 and 2.
 template <int TT>
-__device__ __noinline__ double rate_terms_any(const double* y, Slot S, double kr, double M, bool jac, double* dout) {
+__device__ __forceinline__ bool any_powers(const Slot& S) {
+  constexpr uint32_t LOW = 0x5555u & ((1u << (2 * TT)) - 1u);
+  return (S.codes & (S.codes >> 1) & LOW) != 0;
+}
+
+// rate_terms_p of such a slot: out of line, so that pow takes neither
+// registers nor instruction cache from the rest.
+template <int TT>
+__device__ __noinline__ double rate_terms_any(const double* y, const Slot& S, double kr, double M, bool jac,
+                                              double* dout) {
   double yr[TT], d[TT];
 #pragma unroll
   for (int s = 0; s < TT; ++s) yr[s] = y[s];
@@ -139,22 +147,6 @@ __device__ __noinline__ double rate_terms_any(const double* y, Slot S, double kr
   if (jac) {
 #pragma unroll
     for (int s = 0; s < TT; ++s) dout[s] = d[s];
-  }
-  return rt;
-}
-
-template <int TT>
-__device__ __forceinline__ double rate_terms(const double (&yr)[TT], const Slot& S, double kr, double M, bool jac,
-                                             double (&d)[TT]) {
-  constexpr uint32_t LOW = 0x5555u & ((1u << (2 * TT)) - 1u);
-  if ((S.codes & (S.codes >> 1) & LOW) == 0) return rate_terms_p<TT, WholePowers>(yr, S, kr, M, jac, d);
-  double y[TT], dd[TT];
-#pragma unroll
-  for (int s = 0; s < TT; ++s) y[s] = yr[s];
-  const double rt = rate_terms_any<TT>(y, S, kr, M, jac, dd);
-  if (jac) {
-#pragma unroll
-    for (int s = 0; s < TT; ++s) d[s] = dd[s];
   }
   return rt;
 }
@@ -186,7 +178,7 @@ __device__ __forceinline__ void st_vals(double* p, int i, const double (&v)[NL])
 
 // Rates (and drates) of reaction slot r with TT terms; yrow: the layers' state
 // rows, ystride apart.
-template <int TT, int NL>
+template <int TT, int NL, bool ANY>
 __device__ inline void rate_slot(const Slot& S, int r, const double* yrow, int ystride, const double (&kr)[NL],
                                  const double (&M)[NL], double* rate, double* drate, bool jac) {
   double rt[NL], d[NL][TT];
@@ -195,7 +187,10 @@ __device__ inline void rate_slot(const Slot& S, int r, const double* yrow, int y
     double yr[TT];
 #pragma unroll
     for (int s = 0; s < TT; ++s) yr[s] = yrow[l * ystride + slot_species<TT>(S, s)];
-    rt[l] = rate_terms<TT>(yr, S, kr[l], M[l], jac, d[l]);
+    if (ANY)
+      rt[l] = rate_terms_any<TT>(yr, S, kr[l], M[l], jac, d[l]);
+    else
+      rt[l] = rate_terms_p<TT, WholePowers>(yr, S, kr[l], M[l], jac, d[l]);
   }
   st_vals<NL>(rate, r, rt);
   if (jac) {
@@ -209,27 +204,50 @@ __device__ inline void rate_slot(const Slot& S, int r, const double* yrow, int y
   }
 }
 
-// Rate constants of RU consecutive passes, loaded before any arithmetic so the
-// strided L2 loads overlap (L2 only: the column of k would flush the gather
-// tables from L1). kcol: the first layer's column; zs: the second's offset.
+// Warps take blocks of 32 RU slots from a queue (zeroed before the barrier
+// ahead of this), after the slots that need pow: one costs about 12,000 cycles
+// (a long chain in code seldom in the instruction cache), which held up its
+// warp's share and with it the layer. Rate constants of a block are loaded
+// before any arithmetic so the strided L2 loads overlap (L2 only: the column
+// of k would flush the gather tables from L1). kcol: the first layer's
+// column; zs: the second's offset.
 template <int TT, int NL, int RU>
 __device__ inline void rates_t(const NetDev& net, const double* yrow, int ystride, const double* kcol,
-                               int64_t kstride, int zs, const double (&M)[NL], double* rate, double* drate, bool jac) {
-  for (int r0 = threadIdx.x; r0 <= net.nr; r0 += RU * blockDim.x) {
+                               int64_t kstride, int zs, const double (&M)[NL], int* queue, double* rate,
+                               double* drate, bool jac) {
+  const int lane = threadIdx.x & 31, n_any = (net.n_any + 31) / 32;
+  while (true) {
+    int q = 0;
+    if (lane == 0) q = atomicAdd(queue, 1);
+    q = __shfl_sync(0xffffffffu, q, 0);
+    if (q < n_any) {
+      if (32 * q + lane < net.n_any) {
+        const int r = net.any_list[32 * q + lane];
+        double kr[NL];
+#pragma unroll
+        for (int l = 0; l < NL; ++l) kr[l] = __ldcg(kcol + (int64_t)r * kstride + l * zs);
+        rate_slot<TT, NL, true>(load_slot<TT>(net, r), r, yrow, ystride, kr, M, rate, drate, jac);
+      }
+      __syncwarp();
+      continue;
+    }
+    const int r0 = 32 * RU * (q - n_any);
+    if (r0 > net.nr) break;
     double kv[RU][NL];
     Slot S[RU];
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
+      const int r = min(r0 + 32 * u + lane, net.nr);
 #pragma unroll
-      for (int l = 0; l < NL; ++l) kv[u][l] = r <= net.nr ? __ldcg(kcol + (int64_t)r * kstride + l * zs) : 0.0;
-      if (TT <= RX_TERMS) S[u] = load_slot<TT>(net, min(r, net.nr));
+      for (int l = 0; l < NL; ++l) kv[u][l] = __ldcg(kcol + (int64_t)r * kstride + l * zs);
+      if (TT <= RX_TERMS) S[u] = load_slot<TT>(net, r);
     }
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
-      const int r = r0 + u * blockDim.x;
-      if (TT > RX_TERMS && r <= net.nr) S[u] = load_slot<TT>(net, r);
-      if (r <= net.nr) rate_slot<TT, NL>(S[u], r, yrow, ystride, kv[u], M, rate, drate, jac);
+      const int r = r0 + 32 * u + lane;
+      if (TT > RX_TERMS) S[u] = load_slot<TT>(net, min(r, net.nr));
+      if (r <= net.nr && !any_powers<TT>(S[u]))
+        rate_slot<TT, NL, false>(S[u], r, yrow, ystride, kv[u], M, rate, drate, jac);
     }
   }
 }
@@ -238,30 +256,30 @@ __device__ inline void rates_t(const NetDev& net, const double* yrow, int ystrid
 // (chem.py:92-99); with jac, also drate[r][s] (chem.py:156-182).
 template <int NL>
 __device__ inline void layer_rates(const NetDev& net, const double* yrow, int ystride, const double* kcol,
-                                   int64_t kstride, int zs, const double (&M)[NL], double* rate, double* drate,
-                                   bool jac) {
-  constexpr int D = NL == 2 ? 3 : 6, DW = NL == 2 ? 2 : 4;
+                                   int64_t kstride, int zs, const double (&M)[NL], int* queue, double* rate,
+                                   double* drate, bool jac) {
+  constexpr int D = 3, DW = 2;
   if (!jac) {   // the right-hand-side kernels run at full occupancy: fewer loads in flight per thread
     switch (net.T) {
-      case 1: rates_t<1, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 2: rates_t<2, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 3: rates_t<3, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 4: rates_t<4, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 5: rates_t<5, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 6: rates_t<6, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      case 7: rates_t<7, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-      default: rates_t<8, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+      case 1: rates_t<1, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 2: rates_t<2, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 3: rates_t<3, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 4: rates_t<4, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 5: rates_t<5, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 6: rates_t<6, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      case 7: rates_t<7, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+      default: rates_t<8, NL, 2>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
     }
   }
   switch (net.T) {
-    case 1: rates_t<1, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 2: rates_t<2, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 3: rates_t<3, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 4: rates_t<4, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 5: rates_t<5, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 6: rates_t<6, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    case 7: rates_t<7, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
-    default: rates_t<8, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, rate, drate, jac); return;
+    case 1: rates_t<1, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 2: rates_t<2, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 3: rates_t<3, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 4: rates_t<4, NL, D>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 5: rates_t<5, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 6: rates_t<6, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    case 7: rates_t<7, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
+    default: rates_t<8, NL, DW>(net, yrow, ystride, kcol, kstride, zs, M, queue, rate, drate, jac); return;
   }
 }
 
@@ -287,9 +305,10 @@ __device__ __forceinline__ void group_words(const uint32_t* wp, int len, uint32_
 
 // Sums of a lane's list of cnt terms, in list order; len: the group's longest.
 // w holds the first GW words; each half is reloaded GW terms ahead as it is used.
-template <bool PK, int NL>
-__device__ __forceinline__ void gather_list(const double* coef, const double* src, const uint32_t* wp, int len,
-                                            int cnt, uint32_t (&w)[GW], double (&acc)[NL]) {
+// load(i): the values at index i.
+template <bool PK, int NL, typename Load>
+__device__ __forceinline__ void gather_list(const double* coef, Load load, const uint32_t* wp, int len, int cnt,
+                                            uint32_t (&w)[GW], double (&acc)[NL]) {
   constexpr int H = GW / 2;
 #pragma unroll
   for (int l = 0; l < NL; ++l) acc[l] = 0.0;
@@ -302,7 +321,7 @@ __device__ __forceinline__ void gather_list(const double* coef, const double* sr
       double c[H];
 #pragma unroll
       for (int u = 0; u < H; ++u) {
-        v[u] = ld_vals<NL>(src, (int)(w[h * H + u] & 0xffffu));
+        v[u] = load((int)(w[h * H + u] & 0xffffu));
         c[u] = term_coef<PK>(coef, w[h * H + u]);
       }
 #pragma unroll
@@ -328,7 +347,7 @@ __device__ __forceinline__ void gather_group(const NetDev& net, const double* co
   const uint32_t* wp = net.gl_w + b0 + (threadIdx.x & 31);
   uint32_t w[GW];
   group_words(wp, len, w);
-  gather_list<PK, NL>(coef, src, wp, len, (int)(desc & 0xffffu), w, acc);
+  gather_list<PK, NL>(coef, [&](int i) { return ld_vals<NL>(src, i); }, wp, len, (int)(desc & 0xffffu), w, acc);
 }
 
 // Up to GB groups of short entries, from group g (n of them exist): all words
@@ -533,8 +552,9 @@ __host__ __device__ inline size_t stage1_smem_bytes(int ni, int nr, int T, int N
 // 2.92 with the queue alone; 2.46 with code without counts for the short lists
 // and packed reaction words (406 M); 2.35 with pow out of line; 2.02 with the
 // short entries in storage order; 1.98 with two layers per CTA, where 512
-// threads beat 384 (2.20 against 2.07 at that point) and 256 (2.44). What is
-// left is the wavefronts of the scattered shared-memory reads.
+// threads beat 384 (2.20 against 2.07 at that point) and 256 (2.44); 1.86 with
+// the rows kernel's zero numerators; 1.78 with the slots that need pow ahead of
+// the others. What is left is the wavefronts of the scattered shared-memory reads.
 template <int NL>
 __global__ void __launch_bounds__(NL * LAYER_THREADS, 4 / NL)
 stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
@@ -561,8 +581,8 @@ stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   const double c0 = adj ? 0.0 : 1.0 / (r * dt[b]);
 
   __shared__ double coefs[MAX_COEF + 1];
-  __shared__ int queue;
-  if (threadIdx.x == 0) queue = 0;
+  __shared__ int queue, slots;
+  if (threadIdx.x == 0) queue = slots = 0;
   if (threadIdx.x < NL) drate[NL * (B.nr + 1) * net.T + threadIdx.x] = 0.0;
   load_coefs(net, coefs);
   // state rows (the rates; padding slot 1.0) and diag_d, written with the rows'
@@ -577,7 +597,7 @@ stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   double M[NL];
 #pragma unroll
   for (int l = 0; l < NL; ++l) M[l] = a.M[j + min(l, last)];
-  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, rate, drate, true);
+  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, &slots, rate, drate, true);
   __syncthreads();
   // One phase for the species sums and the Jacobian gather. The gather writes
   // each block entry in its final form.
@@ -677,6 +697,8 @@ stage2_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   const double dtb = res ? 1.0 : dt[b];
 
   __shared__ double coefs[MAX_COEF + 1];
+  __shared__ int slots;
+  if (threadIdx.x == 0) slots = 0;
   load_coefs(net, coefs);
   // state rows (yk2 = y + k1/r; padding slot 1.0)
 #pragma unroll
@@ -695,7 +717,7 @@ stage2_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* _
   double M[NL];
 #pragma unroll
   for (int l = 0; l < NL; ++l) M[l] = a.M[j + min(l, last)];
-  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, rate, nullptr, false);
+  layer_rates<NL>(net, yj, ni + 1, k + g.z0 * (B.nr + 1) + j, nz, last, M, &slots, rate, nullptr, false);
   __syncthreads();
   species_sums<NL>(net, coefs, rate, part);
   __syncthreads();
@@ -734,16 +756,16 @@ chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __re
   double* J = drate + (net.nr + 1) * net.T + 1;   // [ni][ni]
   const double* yrow = y + ((int64_t)b * nz + j) * ni;
   __shared__ double coefs[MAX_COEF + 1];
-  __shared__ int queue;
+  __shared__ int queue, slots;
   if (threadIdx.x == 0) {
-    queue = 0;
+    queue = slots = 0;
     if (want_jac) drate[(net.nr + 1) * net.T] = 0.0;
   }
   load_coefs(net, coefs);
   for (int i = threadIdx.x; i <= ni; i += blockDim.x) yj[i] = i < ni ? yrow[i] : 1.0;
   __syncthreads();
   const double Mj[1] = {M[(int64_t)b * nz + j]};
-  layer_rates<1>(net, yj, 0, k + (int64_t)b * (net.nr + 1) * nz + j, nz, 0, Mj, rate, drate, want_jac);
+  layer_rates<1>(net, yj, 0, k + (int64_t)b * (net.nr + 1) * nz + j, nz, 0, Mj, &slots, rate, drate, want_jac);
   __syncthreads();
   if (want_jac)
     gather_layer<1>(
@@ -978,7 +1000,8 @@ lv_rates_kernel(NetDev net, Batch B, const double* __restrict__ y, const double*
           double yr[TT], d[TT];
 #pragma unroll
           for (int s = 0; s < TT; ++s) yr[s] = yT[slot_species<TT>(sl, s) * S + zl];
-          const double rt = rate_terms<TT>(yr, sl, kv[u], M, false, d);
+          const double rt = any_powers<TT>(sl) ? rate_terms_any<TT>(yr, sl, kv[u], M, false, d)
+                                               : rate_terms_p<TT, WholePowers>(yr, sl, kv[u], M, false, d);
           if (on) rate[(int64_t)rr * nzb + z] = rt;
         }
       }
@@ -1027,6 +1050,160 @@ lv_sums_kernel(NetDev net, Batch B, const double* __restrict__ dt, const uint8_t
     if (fix_mask && fix_mask[g.z0 * ni + q]) v = 0.0;
     w.rmod[q] = v - (2.0 / (r * dt[b])) * w.k1[q];
   }
+}
+
+// ---------------------------------------------------------------- stage 2 by tiles of layers
+// The stage-2 right-hand side of TZ consecutive layers of one atmosphere: the
+// layers are the fastest lanes, so rate constants are read by sectors, a term
+// is one word for eight lanes and eight neighbouring rates, and the rates
+// never leave shared memory. The same terms in the same order as
+// stage2_kernel's. The warps take quadruples of species lists (in the order of
+// the groups, longest first) from a queue. Bound by the latency of the rate
+// constants and of the longest lists at two CTAs per SM: 0.39 ms at 296
+// atmospheres of 69 species and 120 layers, against 0.28 + 0.24 of the two
+// thread-per-layer passes, which write and read every rate in global memory;
+// 0.52 before the slots that need pow went ahead of the others.
+constexpr int TZ = 8;
+constexpr int TZ_THREADS = 512;
+
+__host__ __device__ inline size_t tz_smem_bytes(int ni, int nr) {
+  return (size_t)TZ * ((size_t)(nr + 1) + (ni + 1) + 2 * (size_t)ni) * sizeof(double);
+}
+
+template <bool PK>
+__device__ __forceinline__ void tz_sums(const NetDev& net, const double* coef, const double* rate, int* queue,
+                                        double* part) {
+  const int lane = threadIdx.x & 31, z = lane % TZ;
+  while (true) {
+    int q = 0;
+    if (lane == 0) q = atomicAdd(queue, 1);
+    q = 4 * __shfl_sync(0xffffffffu, q, 0);
+    if (q >= 2 * net.ni) break;
+    q += lane / TZ;
+    const uint32_t desc = net.gl_desc[q];
+    const bool on = desc != ~0u;
+    const int cnt = on ? (int)(desc & 0xffffu) : 0;
+    const int len = __shfl_sync(0xffffffffu, cnt, 0);   // the first list is the longest
+    const uint32_t* wp = net.gl_w + net.gl_base[q >> 5] + (q & 31);
+    uint32_t w[GW];
+    group_words(wp, len, w);
+    double acc[1];
+    gather_list<PK, 1>(coef, [&](int i) { return Vals<1>{{rate[i * TZ + z]}}; }, wp, len, cnt, w, acc);
+    if (on) part[(desc >> 16) * TZ + z] = acc[0];
+  }
+}
+
+template <int TT>
+__global__ void __launch_bounds__(TZ_THREADS, 2)
+stage2_tile_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
+                   const double* __restrict__ dt, const double* __restrict__ atm,
+                   const uint8_t* __restrict__ fix_mask, double* __restrict__ ws) {
+  extern __shared__ double smem[];
+  constexpr int RU = 4;   // rate constants loaded ahead
+  const int b = blockIdx.y, j0 = TZ * blockIdx.x;
+  const Geo g = geo_of(B, b);
+  if (j0 >= g.nz) return;
+  const int ni = B.ni, R = B.nr + 1, nl = min(TZ, g.nz - j0);
+  double* rate = smem;            // [R][TZ]
+  double* yT = rate + R * TZ;     // [ni+1][TZ]
+  double* part = yT + (ni + 1) * TZ;   // [2 ni][TZ]
+  const WsView w = ws_view(ws, g, ni, B.ld);
+  const AtmRef a = atm_ref(atm + g.atm, g.nz, ni);
+  const double* yb = y + (g.z0 + j0) * ni;
+  const double* k1 = w.k1 + (int64_t)j0 * ni;
+  const double r = ros2_r();
+  __shared__ double coefs[MAX_COEF + 1];
+  __shared__ int queue, slots;
+  if (threadIdx.x == 0) queue = slots = 0;
+  load_coefs(net, coefs);
+  for (int e = threadIdx.x; e < nl * ni; e += blockDim.x) {
+    const int z = e / ni, i = e - z * ni;
+    yT[i * TZ + z] = yb[e] + k1[e] / r;   // stage2_kernel's expression
+  }
+  if (threadIdx.x < TZ) yT[ni * TZ + threadIdx.x] = 1.0;
+  __syncthreads();
+  // warps take blocks of RU quadruples of slots, after those that need pow (rates_t)
+  const int lane = threadIdx.x & 31, z = lane % TZ, sub = lane / TZ, n_any = (net.n_any + 3) / 4;
+  const bool on = z < nl;
+  const double M = a.M[j0 + (on ? z : 0)];
+  const double* kb = k + g.z0 * R + j0 + (on ? z : 0);
+  while (true) {
+    int q = 0;
+    if (lane == 0) q = atomicAdd(&slots, 1);
+    q = __shfl_sync(0xffffffffu, q, 0);
+    const bool any = q < n_any;
+    const int r0 = any ? 0 : 4 * RU * (q - n_any);
+    if (r0 >= R) break;
+    if (any) {
+      if (4 * q + sub < net.n_any) {
+        const int rr = net.any_list[4 * q + sub];
+        const Slot S = load_slot<TT>(net, rr);
+        double yr[TT], d[TT];
+#pragma unroll
+        for (int s = 0; s < TT; ++s) yr[s] = yT[slot_species<TT>(S, s) * TZ + z];
+        rate[rr * TZ + z] = rate_terms_any<TT>(yr, S, __ldcg(kb + (int64_t)rr * g.nz), M, false, d);
+      }
+      __syncwarp();
+      continue;
+    }
+    double kv[RU];
+    Slot S[RU];
+#pragma unroll
+    for (int u = 0; u < RU; ++u) {
+      const int rr = min(r0 + 4 * u + sub, R - 1);
+      kv[u] = __ldcg(kb + (int64_t)rr * g.nz);
+      if (TT <= RX_TERMS) S[u] = load_slot<TT>(net, rr);
+    }
+#pragma unroll
+    for (int u = 0; u < RU; ++u) {
+      const int rr = r0 + 4 * u + sub;
+      if (TT > RX_TERMS) S[u] = load_slot<TT>(net, min(rr, R - 1));
+      if (rr < R && !any_powers<TT>(S[u])) {
+        double yr[TT], d[TT];
+#pragma unroll
+        for (int s = 0; s < TT; ++s) yr[s] = yT[slot_species<TT>(S[u], s) * TZ + z];
+        rate[rr * TZ + z] = rate_terms_p<TT, WholePowers>(yr, S[u], kv[u], M, false, d);
+      }
+    }
+  }
+  __syncthreads();
+  if (net.coef_packed)
+    tz_sums<true>(net, coefs, rate, &queue, part);
+  else
+    tz_sums<false>(net, coefs, rate, &queue, part);
+  __syncthreads();
+  const uint8_t* fm = fix_mask ? fix_mask + (g.z0 + j0) * ni : nullptr;
+  double* rmod = w.rmod + (int64_t)j0 * ni;   // holds the rows' diffusion terms (diffusion_rows_kernel)
+  const double c = 2.0 / (r * dt[b]);
+  for (int e = threadIdx.x; e < nl * ni; e += blockDim.x) {
+    const int zz = e / ni, i = e - zz * ni;
+    double v = (part[(2 * i + 1) * TZ + zz] - part[2 * i * TZ + zz]) + rmod[e];
+    if (fm && fm[e]) v = 0.0;
+    rmod[e] = v - c * k1[e];
+  }
+}
+
+static cudaError_t launch_stage2_tiles(const NetDev& net, const Batch& B, const double* y, const double* k,
+                                       const double* dt, const double* atm, const uint8_t* fm, double* ws,
+                                       cudaStream_t st) {
+  const size_t sm = tz_smem_bytes(B.ni, B.nr);
+  dim3 grid((B.nz + TZ - 1) / TZ, B.count);
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto kern) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess) kern<<<grid, TZ_THREADS, sm, st>>>(net, B, y, k, dt, atm, fm, ws);
+  };
+  switch (net.T) {
+    case 1: go(stage2_tile_kernel<1>); break;
+    case 2: go(stage2_tile_kernel<2>); break;
+    case 3: go(stage2_tile_kernel<3>); break;
+    case 4: go(stage2_tile_kernel<4>); break;
+    case 5: go(stage2_tile_kernel<5>); break;
+    case 6: go(stage2_tile_kernel<6>); break;
+    case 7: go(stage2_tile_kernel<7>); break;
+    default: go(stage2_tile_kernel<8>); break;
+  }
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 static int sm_count() {
@@ -1128,6 +1305,13 @@ cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, co
   cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, resid, 2, st);
   if (e != cudaSuccess) return e;
   if (!resid && B.stage1_layers == 2) return launch_stage2_t<2>(net, B, y, k, dt, atm, fm, ws, st, resid);
+  // Tiles where their rates fit shared memory and two CTAs per SM have work;
+  // fewer layers leave SMs idle that the reaction chunks of the thread-per-layer
+  // passes fill. Measured on B200, thread per layer / tiles, stage 2 with the
+  // diffusion rows: 0.63 / 0.51 ms (296 atmospheres of 69 species, 120 layers),
+  // 0.72 / 0.51 (128 of 89, 150 layers), 0.083 / 0.041 (33 of 45, 97 layers).
+  if (!resid && tz_smem_bytes(B.ni, B.nr) <= 220 * 1024 && (int64_t)B.count * ((B.nz + TZ - 1) / TZ) >= 2 * sm_count())
+    return launch_stage2_tiles(net, B, y, k, dt, atm, fm, ws, st);
   if (!resid && B.rates) return launch_lv_stage2(net, B, y, k, dt, atm, fm, ws, st);
   return launch_stage2_t<1>(net, B, y, k, dt, atm, fm, ws, st, resid);
 }

@@ -27,6 +27,9 @@ struct NetDev {
   // Reaction slot in one word (T <= RX_TERMS): reactant index s in byte s, its
   // stoichiometry's code (st_code) at bits 48 + 2 s, the three-body flag at bit 60.
   const uint64_t* rx;            // [nr+1]
+  // Reactions with a stoichiometry of code 3 (their powers take pow).
+  const int32_t* any_list;       // [n_any]
+  int n_any;
   // Gather tables, one 32-bit word per term: the low 16 bits index a rate
   // (species lists: reaction r) or a drate slot (Jacobian: r*T+s), the high 16
   // bits give the coefficient: the top half of the double's high word where

@@ -102,3 +102,26 @@ def test_step_layers_per_block(ni, third):
     assert all(torch.equal(a, b) for a, b in zip(one, two))
     sol, _ = oracle.ros2_step(c.y, c.k, c.dt, c.atm, net.tables)[:2]
     assert np.allclose(one[0].cpu().numpy().reshape(sol.shape), sol, rtol=1e-9, atol=1e-9 * np.abs(sol).max())
+
+
+@pytest.mark.parametrize("ni,change", [(12, None), (33, "coefficient"), (33, "power"), (69, "power")])
+def test_stage2_tiles(ni, change):
+    """A batch of enough layers takes the tiled stage 2 (whole and part tiles of
+    eight layers); every atmosphere equals its own step, which does not."""
+    net = syn.make_network(11 + ni, ni, 5 * ni)
+    if change == "coefficient":
+        net.tables.product_stoich[1, 0] = 1.0 / 3.0
+    if change == "power":
+        net.tables.reactant_stoich[2, 0] = 3.0
+        net.tables.reactant_stoich[4, 0] = 0.5
+    dn = chem.to_device(net.tables)
+    cases = [syn.make_case(seed=20 + nz, net=net, nz=nz, mild=True, k_range=(-12.0, 4.0), dt=1e-5)
+             for nz in (3, 7, 8, 9, 16, 17)]
+    many = cases * 50
+    step = jstep.RaggedRos2Step(dn, [jstep.atm_from_dict(c.atm) for c in many])
+    y, k = step.pack([c.y for c in many], [c.k for c in many])
+    sol, delta, _ = step(y, k, torch.full((len(many),), 1e-5, dtype=torch.float64, device="cuda"))
+    alone = [[t.clone() for t in jstep.jax_ros2_step(c.y, c.k, 1e-5, jstep.atm_from_dict(c.atm), dn)] for c in cases]
+    for b, (s, d) in enumerate(zip(step.unpack(sol), step.unpack(delta))):
+        s1, d1 = alone[b % len(cases)]
+        assert torch.equal(s, s1) and torch.equal(d, d1), b
