@@ -79,8 +79,10 @@ int vb_net_destroy(VbNet* net);
  * reference, whose XLA compiler picks its own): set by the project's
  * autotuner (jax-vulcan_b200/autotune.py), which times the candidates on the
  * device per network and batch; 0 in a field = the automatic choice.
- *   factor_kernel: 1 blocked Gauss-Jordan on the tensor cores, 2 scalar
- *                  Gauss-Jordan, 3 scalar Gauss-Jordan pipelined per column
+ *   factor_kernel: 1 blocked Gauss-Jordan on the tensor cores, 2 Gauss-Jordan
+ *                  by panels of eight columns, one block barrier per panel
+ *                  (the default; FP64 trailing updates on the tensor cores),
+ *                  3 scalar Gauss-Jordan pipelined per column
  *                  panel, 4 scalar Gauss-Jordan with two atmospheres per CTA
  *                  (uniform batches of 65-72 species; else as 2) (0: the
  *                  process default, vb_set_factor_kernel)
@@ -94,10 +96,10 @@ int vb_net_destroy(VbNet* net);
  *                  and joined with events, so the call stays stream-ordered
  *                  on the caller's stream), so one half's assembly overlaps
  *                  the other half's factor; 0 or 1 = one stream
- *   stage1_layers: layers per CTA of the stage-1 and stage-2 assembly, 1 or
- *                  2 (two share every gather-table word and rate-constant
- *                  sector; 0 = by size in stage 1, thread-per-layer or 1 in
- *                  stage 2) */
+ *   stage1_layers: layers per CTA of the stage-1 assembly, 1 or 2 (two share
+ *                  every gather-table word and rate-constant sector; 0 = by
+ *                  size), and 2 also of the stage-2 assembly of batches too
+ *                  small for its tiles of eight layers */
 typedef struct VbTuning {
   int32_t factor_kernel, factor_ctas, sweep_stages, streams, stage1_layers, reserved;
 } VbTuning;
@@ -117,8 +119,9 @@ size_t vb_ros2_workspace_bytes(int batch, int nz, int ni, const int64_t* zoff_ho
  * count of a ragged batch), the step assembles the stage-2 right-hand side
  * with one thread per layer (the rate of every reaction and layer staged in
  * that region, then every species sum formed from coalesced rows of layers)
- * instead of one CTA per layer; the results are identical. nr+1 doubles per
- * layer. */
+ * instead of one CTA per layer, where the batch is too small for tiles of
+ * eight layers per CTA (two CTAs per SM) or their rates exceed shared memory;
+ * the results are identical. nr+1 doubles per layer. */
 size_t vb_ros2_assembly_bytes(const VbNet* net, int batch, int nz);
 int vb_ros2_step(const VbNet* net, int batch, int nz, const int64_t* zoff,
                  const double* y, const double* k, const double* dt,
@@ -130,7 +133,7 @@ int vb_ros2_step(const VbNet* net, int batch, int nz, const int64_t* zoff,
  * vb_ros2_step, with the demotion inside. The LHS blocks are assembled in
  * FP64 (kept for the residual); each Schur-updated block is row-equilibrated
  * (exact powers of two) and inverted in FP32 by the process's factor kernel
- * (vb_set_factor_kernel: scalar Gauss-Jordan by default; the blocked kernel
+ * (vb_set_factor_kernel: Gauss-Jordan by panels by default; the blocked kernel
  * runs its rank-8 trailing updates on the TF32 tensor cores, each operand
  * split into a TF32 head and tail, three products); each stage solve
  * LHS k = rhs (jax_step.py:300-311) starts from the FP32 factors and is
@@ -184,14 +187,17 @@ int vb_set_pipeline_wait_limit(long long polls);
  * overrides it for that network): 0 = blocked Gauss-Jordan, one warp per
  * 8-column panel, the panel's pivot steps inside the warp and the rank-8
  * trailing updates on the FP64 tensor cores (mma.sync m8n8k4); 1 (default) =
- * scalar Gauss-Jordan, one block barrier per pivot step; 2 = the same scalar
+ * Gauss-Jordan by panels of eight columns, one block barrier per panel: a
+ * panel's owner warp and the next panel's run its pivot steps while the others
+ * apply the panel before (FP64 on the tensor cores, whose multiply-adds are
+ * those of the scalar elimination in its order; FP32 scalar); 2 = the scalar
  * elimination pipelined: the warp owning a column panel runs its pivot steps
  * back to back and publishes each (pivot row, multipliers) through a
  * shared-memory ring signalled by mbarriers, the other warps apply the steps
  * as they arrive (bounded waits; no block barrier per step); 3 = the scalar
  * elimination with two atmospheres per CTA, their pivot chains interleaved
  * in the same warps under one barrier per step (FP64 factor of uniform
- * batches of 65-72 species; the scalar kernel elsewhere). All replace the
+ * batches of 65-72 species; kernel 1 elsewhere). All replace the
  * reference's lu_factor + lu_solve(LU, I) pair (solver.py:46-48). */
 int vb_set_factor_kernel(int variant);
 

@@ -4,9 +4,9 @@
 //   * the stage-1 kernel: rhs(y) and the LHS blocks c0*I - J - diag(diff)
 //     (reference jax_step.py:263-298, chem.py:83-214), and
 //   * the stage-2 kernel: rhs(yk2) - 2/(r dt) k1 (jax_step.py:303-310).
-// One CTA per (layer, atmosphere). Compiled with --fmad=false: the gathers sum
-// in the segment_sum order of the reference, so the RHS and the Jacobian are
-// bit-identical to the reference's.
+// One CTA per layer, pair or tile of layers of an atmosphere. Compiled with
+// --fmad=false: the gathers sum in the segment_sum order of the reference, so
+// the RHS and the Jacobian are bit-identical to the reference's.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1304,7 +1304,6 @@ cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, co
                           cudaStream_t st, double* resid) {
   cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, resid, 2, st);
   if (e != cudaSuccess) return e;
-  if (!resid && B.stage1_layers == 2) return launch_stage2_t<2>(net, B, y, k, dt, atm, fm, ws, st, resid);
   // Tiles where their rates fit shared memory and two CTAs per SM have work;
   // fewer layers leave SMs idle that the reaction chunks of the thread-per-layer
   // passes fill. Measured on B200, thread per layer / tiles, stage 2 with the
@@ -1312,6 +1311,7 @@ cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, co
   // 0.72 / 0.51 (128 of 89, 150 layers), 0.083 / 0.041 (33 of 45, 97 layers).
   if (!resid && tz_smem_bytes(B.ni, B.nr) <= 220 * 1024 && (int64_t)B.count * ((B.nz + TZ - 1) / TZ) >= 2 * sm_count())
     return launch_stage2_tiles(net, B, y, k, dt, atm, fm, ws, st);
+  if (!resid && B.stage1_layers == 2) return launch_stage2_t<2>(net, B, y, k, dt, atm, fm, ws, st, resid);
   if (!resid && B.rates) return launch_lv_stage2(net, B, y, k, dt, atm, fm, ws, st);
   return launch_stage2_t<1>(net, B, y, k, dt, atm, fm, ws, st, resid);
 }

@@ -98,7 +98,7 @@ struct Batch {
   int ld;             // row stride of stored inverse blocks (ni rounded up to even)
   const int64_t* zoff;  // [count+1] prefix sums of layers, or nullptr (uniform)
   // launch shapes chosen by the network's tuning (VbTuning; 0 = automatic)
-  int factor_kernel = 0;   // 1 blocked tensor-core, 2 scalar Gauss-Jordan, 3 pipelined
+  int factor_kernel = 0;   // 1 blocked tensor-core, 2 by panels, 3 pipelined, 4 paired
   int factor_ctas = 0;     // CTAs per SM of the factor (1 or 2, where both fit)
   int sweep_stages = 0;    // bulk-copy ring depth of the sweeps (1..3)
   int stage1_layers = 0;   // layers per stage-1 CTA (1 or 2)

@@ -43,7 +43,7 @@ void set_wait_limit(long long polls);
 void set_pipe_wait_limit(long long polls);
 long long wait_limit();
 // FP64 factor kernel: 0 = blocked Gauss-Jordan with FP64 tensor-core trailing
-// updates, 1 = scalar Gauss-Jordan.
+// updates, 1 = Gauss-Jordan by panels (the default), 2 = pipelined, 3 = paired.
 void set_factor_variant(int v);
 cudaError_t launch_chem(const NetDev&, int batch, int nz, const double* y, const double* M, const double* k,
                         double* dydt, double* jac, cudaStream_t);

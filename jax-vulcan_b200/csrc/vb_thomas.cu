@@ -1616,7 +1616,7 @@ static cudaError_t launch_gj_t(const Batch& B, double* ws, int32_t* status, int 
 // FP32: scalar), 2 = scalar Gauss-Jordan pipelined per column panel
 // (no block barrier per step), 3 = scalar Gauss-Jordan with two atmospheres'
 // chains interleaved per CTA (FP64 factor of uniform batches of 65-72
-// species; the scalar kernel elsewhere). A network's tuning (factor_kernel
+// species; kernel 1 elsewhere). A network's tuning (factor_kernel
 // 1..4 = variant 0..3) overrides it.
 static int g_factor_variant = 1;
 void set_factor_variant(int v) { g_factor_variant = v; }

@@ -101,13 +101,14 @@ class Ros2Step:
     def __init__(self, net: NetworkArrays, atm: AtmStatic, batch: int | None = None, mixed: bool = False,
                  max_refine: int = 3, tol: float = 1e-12, assembly: bool = True):
         """``mixed=True``: the mixed-precision step (``vb_ros2_step_mixed``:
-        FP32 row-equilibrated factor on the TF32 tensor cores, FP64 refinement
+        FP32 row-equilibrated factor, FP64 refinement
         of both stages, at most ``max_refine`` passes to ``tol``, FP64
         fallback); ``self.passes`` then holds the passes run per atmosphere.
         ``assembly``: allocate the rate region of the layer-vectorized
         stage 2 (``vb_ros2_assembly_bytes``: nr+1 doubles per layer), so the
-        stage-2 right-hand side is formed with a thread per layer; False: the
-        per-layer stage-2 kernel (same results, less memory)."""
+        stage-2 right-hand side is formed with a thread per layer where the
+        batch is too small for tiles of eight layers per CTA; False: the
+        per-layer stage-2 kernel there (same results, less memory)."""
         self.net = net
         self.mixed = bool(mixed)
         self.max_refine = int(max_refine)
