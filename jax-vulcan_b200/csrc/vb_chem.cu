@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(NL * LAYER_THREADS, 4 / NL)
 stage1_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
               const double* __restrict__ dt, const double* __restrict__ atm, int flags,
               const uint8_t* __restrict__ fix_mask, double* __restrict__ ws, const double* __restrict__ adj_v) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int b = blockIdx.y, j = NL * blockIdx.x;
   Geo g = geo_of(B, b);
   if (j >= g.nz) return;
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(NL * LAYER_THREADS, 8 / NL)
 stage2_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
               const double* __restrict__ dt, const double* __restrict__ atm,
               const uint8_t* __restrict__ fix_mask, double* __restrict__ ws, double* __restrict__ resid) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int b = blockIdx.y, j = NL * blockIdx.x;
   Geo g = geo_of(B, b);
   if (j >= g.nz) return;
@@ -745,7 +745,7 @@ __host__ __device__ inline size_t chem_smem_bytes(int ni, int nr, int T, bool ja
 __global__ void __launch_bounds__(LAYER_THREADS)
 chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __restrict__ M,
             const double* __restrict__ k, double* __restrict__ dydt, double* __restrict__ jac) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int b = blockIdx.y, j = blockIdx.x;
   const int ni = net.ni;
   const bool want_jac = jac != nullptr;
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(LAYER_THREADS)
 diffusion_kernel(int nz, int ni, const double* __restrict__ y, const double* __restrict__ atm,
                  int flags, double* __restrict__ diff, double* __restrict__ diag_d,
                  double* __restrict__ sup_d, double* __restrict__ sub_d) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int b = blockIdx.y, j = blockIdx.x;
   LayerSmem L = carve(smem, ni);
   AtmRef a = atm_ref(atm + (int64_t)b * VB_ATM_DOUBLES(nz, ni), nz, ni);
@@ -838,7 +838,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 4)
 diffusion_rows_kernel(Batch B, const double* __restrict__ y, const double* __restrict__ atm, int flags,
                       const uint8_t* __restrict__ fix_mask, double* __restrict__ ws, double* __restrict__ resid,
                       int mode) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   constexpr int LB = DIFF_LAYERS, NR = LB + 2;
   const int b = blockIdx.y, jb = blockIdx.x * LB;
   Geo g = geo_of(B, b);
@@ -957,7 +957,7 @@ template <int TT>
 __global__ void __launch_bounds__(LV_RATE_THREADS, 2)
 lv_rates_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
                 const double* __restrict__ atm, double* __restrict__ ws) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   constexpr int RU = 4;   // rate constants loaded ahead
   const int b = blockIdx.y;
   const Geo g = geo_of(B, b);
@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(TZ_THREADS, 2)
 stage2_tile_kernel(NetDev net, Batch B, const double* __restrict__ y, const double* __restrict__ k,
                    const double* __restrict__ dt, const double* __restrict__ atm,
                    const uint8_t* __restrict__ fix_mask, double* __restrict__ ws) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   constexpr int RU = 4;   // rate constants loaded ahead
   const int b = blockIdx.y, j0 = TZ * blockIdx.x;
   const Geo g = geo_of(B, b);
@@ -1203,7 +1203,7 @@ static cudaError_t launch_stage2_tiles(const NetDev& net, const Batch& B, const 
     case 7: go(stage2_tile_kernel<7>); break;
     default: go(stage2_tile_kernel<8>); break;
   }
-  return e == cudaSuccess ? cudaGetLastError() : e;
+  return cudaGetLastError();
 }
 
 static int sm_count() {
@@ -1272,7 +1272,7 @@ static cudaError_t launch_stage1_t(const NetDev& net, const Batch& B, const doub
                                    cudaStream_t st, const double* adj_v) {
   const size_t sm = stage1_smem_bytes(B.ni, B.nr, net.T, NL);
   cudaError_t e = cudaFuncSetAttribute(stage1_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) return cudaGetLastError();   // too large a layer; leaves no error behind
   stage1_kernel<NL><<<dim3((B.nz + NL - 1) / NL, B.count), NL * LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, flags,
                                                                                          fm, ws, adj_v);
   return cudaGetLastError();
@@ -1293,7 +1293,7 @@ static cudaError_t launch_stage2_t(const NetDev& net, const Batch& B, const doub
                                    cudaStream_t st, double* resid) {
   const size_t sm = stage2_smem_bytes(B.ni, B.nr, NL);
   cudaError_t e = cudaFuncSetAttribute(stage2_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) return cudaGetLastError();
   stage2_kernel<NL><<<dim3((B.nz + NL - 1) / NL, B.count), NL * LAYER_THREADS, sm, st>>>(net, B, y, k, dt, atm, fm, ws,
                                                                                          resid);
   return cudaGetLastError();
