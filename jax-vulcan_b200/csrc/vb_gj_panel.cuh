@@ -14,16 +14,18 @@ namespace vb {
 // (FP32), the lowest row among those (threshold partial pivoting with threshold
 // 1 - 2^-13; strict partial pivoting takes the exact maximum, at the price of a
 // second reduction, ballots and shuffles on the pivot chain). The magnitude
-// bits are shifted out of the sign and raised by one exponent unit, which
-// takes infinities and NaN around to the bottom of the order (such a layer is
-// non-finite whatever row it takes) in one integer instruction: testing for NaN
-// with a double comparison per row cost 160 of a step's 475 cycles. Rows that
-// may not pivot (pivoted, padding) take key 0, below every candidate (row <=
-// 127, so a candidate's low byte is >= 128).
+// bits are shifted out of the sign and raised so that infinity, the largest,
+// takes the top value; NaN wraps around below zero's and is brought to it (a
+// NaN counts as magnitude 0). Two integer instructions: testing for NaN with a
+// double comparison per row cost 160 of a step's 475 cycles. Rows that may not
+// pivot (pivoted, padding) take key 0, below every candidate (row <= 127, so a
+// candidate's low byte is >= 128).
 __device__ __forceinline__ unsigned pivot_mag(double v) {
-  return ((unsigned)__double2hiint(v) << 1) + 0x00200000u;
+  return max(((unsigned)__double2hiint(v) << 1) + 0x001fff00u, 0x001fff00u);
 }
-__device__ __forceinline__ unsigned pivot_mag(float v) { return (__float_as_uint(v) << 1) + 0x01000000u; }
+__device__ __forceinline__ unsigned pivot_mag(float v) {
+  return max((__float_as_uint(v) << 1) + 0x00ffff00u, 0x00ffff00u);
+}
 template <typename R>
 __device__ __forceinline__ unsigned pivot_key32(R v, int row) {
   return (pivot_mag(v) & 0xffffff00u) | (unsigned)(255 - row);
