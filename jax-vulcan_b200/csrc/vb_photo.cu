@@ -219,11 +219,6 @@ tau_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const
   }
 }
 
-// a / b for a finite nonzero b. A zero numerator (opaque layers: no beam, no
-// flux) takes the product, whose value and sign are the quotient's, instead of
-// the division's out-of-range path.
-__device__ __forceinline__ double quot(double a, double b) { return a == 0.0 ? a * b : a / b; }
-
 struct TwoStream {
   double chi, xi, phi, gp, gm;
 };
