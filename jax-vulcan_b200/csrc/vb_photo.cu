@@ -17,6 +17,8 @@
 // element-wise expressions do.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "vb_common.cuh"
 #include "vb_launch.cuh"
 
@@ -39,9 +41,9 @@ static_assert(sizeof(VbConvState) % sizeof(double) == 0, "VbConvState size");
 // 32 bins a tile: the recursion, which one warp runs while the others wait,
 // serves 32 bins at a time; the flux tile's seven rows per layer then fill one
 // SM's shared memory at nz = 120. nz=120, 2500 bins, 40 branches (B200, us,
-// before -> now): tau 1 atmosphere 376 -> 21, 64: 420 -> 241; flux 580 -> 30,
-// 1420 -> 952 (about 220 FP64 instructions per layer and bin; the recursion's
-// share is a quarter); J (below) 62 -> 24, 640 -> 272.
+// before -> now, launches back to back): tau 1 atmosphere 261 -> 11, 64: 403 ->
+// 208; flux 449 -> 27, 1412 -> 967 (about 220 FP64 instructions per layer and
+// bin; the recursion's share is a quarter); J (below) 33 -> 21, 570 -> 267.
 constexpr size_t PHOTO_SMEM_MAX = 220 * 1024;
 
 // Cross sections of the tile's bins (absorbers, then scatterers; 0 outside nbin)
@@ -179,7 +181,7 @@ tau_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const double
 }
 
 // The same with a thread per bin and column: columns whose tile does not fit
-// shared memory.
+// shared memory, and many short ones (short_columns).
 __global__ void __launch_bounds__(PHOTO_THREADS)
 tau_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ y, const double* __restrict__ dz,
            double* __restrict__ tau, const int32_t* __restrict__ due, double* __restrict__ achg) {
@@ -306,10 +308,10 @@ __host__ __device__ inline size_t flux_smem_bytes(const VbPhoto& P, int nz) {
 // the weights' tile lies over the rows xi and 1/chi until the coefficients are formed
 template <int PB>
 constexpr int FLUX_MAX_SPECIES = 2 * PB;
-constexpr int FLUX_THREADS = 512;
+constexpr int FLUX_THREADS = 512;   // of an SM: 128 registers each
 
 template <int PB, int PT>
-__global__ void __launch_bounds__(PT, PB == 32 ? 1 : 2)
+__global__ void __launch_bounds__(PT, FLUX_THREADS / PT)
 flux_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, const double* __restrict__ ymix,
             const double* du_prev, double* __restrict__ aflux, double* __restrict__ sflux,
             double* __restrict__ dd, double* du, const int32_t* __restrict__ due, double flux_atol,
@@ -501,8 +503,7 @@ flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, co
   double* ddb = dd + zb;
   double* dub = du + zb;
   double* ab = aflux + (int64_t)b * nz * nbin;
-  const StreamConst sc(P);
-  const double mu_ang = sc.mu;
+  const double mu_ang = -1.0 * P.mu_zenith;
   const double top = P.sflux_top[bin];
   // albedo of every layer, parked in the sflux rows until the up recursion
   // hands each row its direct beam (the sums over absorbers run once per
@@ -516,7 +517,7 @@ flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, co
   for (int j = nz - 1; j >= 0; --j) {
     const double t0 = tb[(int64_t)j * nbin + bin], t1 = tb[(int64_t)(j + 1) * nbin + bin];
     const double s_lo = top * exp(t0 / mu_ang);
-    TwoStream c = two_stream(P, sc, sb[(int64_t)j * nbin + bin], t0 - t1);
+    TwoStream c = two_stream(P, StreamConst(P), sb[(int64_t)j * nbin + bin], t0 - t1);
     const double dir0 = s_lo * (-mu_ang);
     const double dir1 = s_hi * (-mu_ang);
     const double i_d = c.phi * c.gm * dir1 - (c.chi * c.gm + c.xi * c.gp) * dir0;
@@ -534,7 +535,7 @@ flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, co
   for (int j = 1; j <= nz; ++j) {
     const double t0 = tb[(int64_t)(j - 1) * nbin + bin], t1 = tb[(int64_t)j * nbin + bin];
     const double s_up = top * exp(t1 / mu_ang);
-    TwoStream c = two_stream(P, sc, sb[(int64_t)(j - 1) * nbin + bin], t0 - t1);
+    TwoStream c = two_stream(P, StreamConst(P), sb[(int64_t)(j - 1) * nbin + bin], t0 - t1);
     const double dir0 = s_lo * (-mu_ang);
     const double dir1 = s_up * (-mu_ang);
     const double i_u = c.phi * c.gp * dir0 - (c.xi * c.gm + c.chi * c.gp) * dir1;
@@ -682,45 +683,104 @@ j_kernel(int batch, int nz, int nr, int lt, VbPhoto P, const double* __restrict_
   }
 }
 
+static int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Threads of a tile's CTA: 512 where one tile takes an SM's shared memory or
+// the grid has no second one for it, else fewer, down to 128, until the tiles
+// that an SM holds share its threads (sm_threads). With 512 for every tile a
+// short column idles most of them (64 layers in flight) and the tiles of an SM
+// run one after another. 2500 bins, 512 threads / this rule, us: flux of 64
+// atmospheres of 20 layers 323 / 160, 43 layers 443 / 344, of 64 1233 / 980 at
+// 126 (16 bins); tau of 64 of 20 layers 102 / 51, 90 layers 218 / 153.
+static int tile_threads(size_t smem, int64_t tiles, int sms, int sm_threads) {
+  const int64_t per_sm = std::min<int64_t>(227 * 1024 / (smem + 1024), (tiles + sms - 1) / sms);
+  int t = 512;
+  while (t > 128 && t * per_sm > sm_threads) t /= 2;
+  return t;
+}
+
+// Whether a thread per bin and column is faster: a tile costs the same however
+// short its column (a table of cross sections, five barriers, 16 layers a pass
+// of 128 threads), a column's thread in proportion, so the line rises with the
+// square of the layers. Flux, 2500 bins, us, tiles (128 threads) / columns: 2
+// layers 4 atmospheres 7.5 / 10.5 and 8: 13.0 / 10.6, 4 layers 16: 21.0 / 18.9, 6
+// layers 16: 24.8 / 27.2 and 32: 41.0 / 32.5, 8 layers 16: 26.5 / 34 and 64: 79 / 74,
+// 10 layers 48: 71.7 / 67.1 and 128: 198 / 175, 14 layers 96: 171 / 176 and 256:
+// 452 / 417, 18 layers 128: 297 / 311 and 256: 576 / 543, 20 layers 256: 602 / 615.
+// Tau: 2 layers 8: 5.6 / 7.3 and 16: 9.6 / 7.4, 4 layers 16: 10.8 / 11.9 and 32:
+// 16.3 / 12.3, 7 layers 48: 23.4 / 21.9, 8 layers 128: 54.9 / 53.0, 10 layers 256:
+// 111 / 115.
+static bool short_columns(int nz, int64_t tiles, int sms, bool flux) {
+  const int64_t per_sm = flux ? std::max(nz + 2, nz * nz * (nz < 16 ? 5 : 6) / 20) : std::max(8, nz * nz / 2);
+  return nz < (flux ? 20 : 10) && tiles >= sms * per_sm;
+}
+
 cudaError_t launch_photo_tau(int batch, int nz, int ni, const VbPhoto& P, const double* y, const double* dz,
                              double* tau, const int32_t* due, double* achg, cudaStream_t st) {
-  constexpr int PB = 32, PT = 512;
+  constexpr int PB = 32;
   const size_t sm = tau_smem_bytes<PB>(P, nz);
-  if (sm <= PHOTO_SMEM_MAX) {
-    cudaError_t e = cudaFuncSetAttribute(tau_kernel<PB, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const dim3 grid((P.nbin + PB - 1) / PB, batch);
+  const int64_t tiles = (int64_t)grid.x * batch;
+  const int sms = sm_count();
+  auto tiled = [&](auto kern, int threads) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    dim3 grid((P.nbin + PB - 1) / PB, batch);
-    tau_kernel<PB, PT><<<grid, PT, sm, st>>>(nz, ni, P, y, dz, tau, due, achg);
-  } else {
-    dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
-    tau_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, y, dz, tau, due, achg);
+    kern<<<grid, threads, sm, st>>>(nz, ni, P, y, dz, tau, due, achg);
+    return cudaGetLastError();
+  };
+  if (sm <= PHOTO_SMEM_MAX && !short_columns(nz, tiles, sms, false)) {
+    switch (tile_threads(sm, tiles, sms, 1024)) {
+      case 128: return tiled(tau_kernel<PB, 128>, 128);
+      case 256: return tiled(tau_kernel<PB, 256>, 256);
+      default: return tiled(tau_kernel<PB, 512>, 512);
+    }
   }
+  dim3 grid1((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
+  tau_column_kernel<<<grid1, PHOTO_THREADS, 0, st>>>(nz, ni, P, y, dz, tau, due, achg);
   return cudaGetLastError();
+}
+
+template <int PB>
+static cudaError_t launch_flux_tiles(int batch, int nz, int ni, const VbPhoto& P, const double* tau,
+                                     const double* ymix, const double* du_prev, double* aflux, double* sflux,
+                                     double* dd, double* du, const int32_t* due, double flux_atol, double* achg,
+                                     cudaStream_t st) {
+  const size_t sm = flux_smem_bytes<PB>(P, nz);
+  const dim3 grid((P.nbin + PB - 1) / PB, batch);
+  auto launch = [&](auto kern, int threads) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, threads, sm, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg);
+    return cudaGetLastError();
+  };
+  switch (tile_threads(sm, (int64_t)grid.x * batch, sm_count(), FLUX_THREADS)) {
+    case 128: return launch(flux_kernel<PB, 128>, 128);
+    case 256: return launch(flux_kernel<PB, 256>, 256);
+    default: return launch(flux_kernel<PB, 512>, 512);
+  }
 }
 
 cudaError_t launch_photo_flux(int batch, int nz, int ni, const VbPhoto& P, const double* tau, const double* ymix,
                               const double* du_prev, double* aflux, double* sflux, double* dd, double* du,
                               const int32_t* due, double flux_atol, double* achg, cudaStream_t st) {
-  auto tiled = [&](auto kern, int pb, int threads, size_t sm) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    dim3 grid((P.nbin + pb - 1) / pb, batch);
-    kern<<<grid, threads, sm, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg);
-    return cudaGetLastError();
-  };
   const int species = P.n_abs + P.n_abs_T + P.n_scat;
-  {
-    // 32 bins up to 120 layers or so, 16 up to 240
+  // 32 bins up to 120 layers or so, 16 up to 240
+  if (!short_columns(nz, (int64_t)((P.nbin + 31) / 32) * batch, sm_count(), true)) {
     if (species <= FLUX_MAX_SPECIES<32> && flux_smem_bytes<32>(P, nz) <= PHOTO_SMEM_MAX)
-      return tiled(flux_kernel<32, FLUX_THREADS>, 32, FLUX_THREADS, flux_smem_bytes<32>(P, nz));
+      return launch_flux_tiles<32>(batch, nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg,
+                                   st);
     if (species <= FLUX_MAX_SPECIES<16> && flux_smem_bytes<16>(P, nz) <= PHOTO_SMEM_MAX)
-      return tiled(flux_kernel<16, 512>, 16, 512, flux_smem_bytes<16>(P, nz));
+      return launch_flux_tiles<16>(batch, nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg,
+                                   st);
   }
-  {
-    dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
-    flux_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due,
-                                                       flux_atol, achg);
-  }
+  dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
+  flux_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due,
+                                                     flux_atol, achg);
   return cudaGetLastError();
 }
 
@@ -730,9 +790,7 @@ cudaError_t launch_photo_j(int batch, int nz, int nr, const VbPhoto& P, const do
   // layers per block: JT when the batch fills the GPU with tiles, else one
   // layer per block (more blocks for a small batch); fewer when the flux rows
   // would not fit 200 KB of shared memory
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   int lt = ((int64_t)batch * ((nz + J_ROWS - 1) / J_ROWS) >= 2 * (int64_t)sms) ? J_ROWS : 1;
   while (lt > 1 && (size_t)lt * P.nbin * sizeof(double) > 200 * 1024) --lt;
   if ((size_t)lt * P.nbin * sizeof(double) > 200 * 1024) return cudaErrorInvalidValue;
