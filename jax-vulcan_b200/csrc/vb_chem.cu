@@ -742,13 +742,19 @@ __host__ __device__ inline size_t chem_smem_bytes(int ni, int nr, int T, bool ja
          sizeof(double);
 }
 
-__global__ void __launch_bounds__(LAYER_THREADS)
+// The right-hand side has a kernel of its own: with the Jacobian's registers two
+// CTAs fit an SM, and a layer of a small network is one round of dependent
+// loads, which only other CTAs hide. Right-hand side of 60 layers (B200, us, one
+// kernel for both / four / six / eight CTAs per SM): 64 atmospheres of 12 species
+// 63 / 35 / 28 / 29, 200 of 30: 232 / 127 / 103 / 114, 64 of 89: 110 / 82 / 65 / 68,
+// one of 69: 9.1 / 8.7 / 8.8 / 10.0.
+template <bool JAC>
+__global__ void __launch_bounds__(LAYER_THREADS, JAC ? 2 : 6)
 chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __restrict__ M,
             const double* __restrict__ k, double* __restrict__ dydt, double* __restrict__ jac) {
   extern __shared__ __align__(16) double smem[];
   const int b = blockIdx.y, j = blockIdx.x;
   const int ni = net.ni;
-  const bool want_jac = jac != nullptr;
   double* rate = smem;                            // [nr+1]
   double* part = rate + (net.nr + 1);             // [2 ni]
   double* yj = part + 2 * ni;                     // [ni+1]
@@ -759,15 +765,15 @@ chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __re
   __shared__ int queue, slots;
   if (threadIdx.x == 0) {
     queue = slots = 0;
-    if (want_jac) drate[(net.nr + 1) * net.T] = 0.0;
+    if (JAC) drate[(net.nr + 1) * net.T] = 0.0;
   }
   load_coefs(net, coefs);
   for (int i = threadIdx.x; i <= ni; i += blockDim.x) yj[i] = i < ni ? yrow[i] : 1.0;
   __syncthreads();
   const double Mj[1] = {M[(int64_t)b * nz + j]};
-  layer_rates<1>(net, yj, 0, k + (int64_t)b * (net.nr + 1) * nz + j, nz, 0, Mj, &slots, rate, drate, want_jac);
+  layer_rates<1>(net, yj, 0, k + (int64_t)b * (net.nr + 1) * nz + j, nz, 0, Mj, &slots, rate, drate, JAC);
   __syncthreads();
-  if (want_jac)
+  if (JAC)
     gather_layer<1>(
         net, coefs, rate, drate, true, &queue, part, [&](int row, const double (&v)[1]) { J[row * ni + row] = v[0]; },
         [&](int row, int col, const double (&v)[1]) { J[row * ni + col] = v[0]; });
@@ -777,7 +783,7 @@ chem_kernel(NetDev net, int nz, const double* __restrict__ y, const double* __re
   if (dydt)
     for (int i = threadIdx.x; i < ni; i += blockDim.x)
       dydt[((int64_t)b * nz + j) * ni + i] = part[2 * i + 1] - part[2 * i];
-  if (want_jac) {
+  if (JAC) {
     double* out = jac + ((int64_t)b * nz + j) * ni * ni;
     for (int d = threadIdx.x; d < ni * ni; d += blockDim.x) out[d] = J[d];
   }
@@ -1319,9 +1325,10 @@ cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, co
 cudaError_t launch_chem(const NetDev& net, int batch, int nz, const double* y, const double* M,
                         const double* k, double* dydt, double* jac, cudaStream_t st) {
   size_t sm = chem_smem_bytes(net.ni, net.nr, net.T, jac != nullptr);
-  cudaFuncSetAttribute(chem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  auto kern = jac ? chem_kernel<true> : chem_kernel<false>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid(nz, batch);
-  chem_kernel<<<grid, LAYER_THREADS, sm, st>>>(net, nz, y, M, k, dydt, jac);
+  kern<<<grid, LAYER_THREADS, sm, st>>>(net, nz, y, M, k, dydt, jac);
   return cudaGetLastError();
 }
 
