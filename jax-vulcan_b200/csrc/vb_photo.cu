@@ -562,7 +562,7 @@ flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, co
 }
 
 // J-rates of a tile of actinic-flux rows, all branches: JT layers of one
-// atmosphere, or (ATM) one layer of JT atmospheres that share the branch
+// atmosphere, or (ATM) one layer of JT due atmospheres that share the branch
 // tables, so a temperature-dependent branch's row of that layer serves all of
 // them as the others' rows serve every tile. The flux rows are staged once in
 // shared memory and each warp takes up to JB branches at a time, so a staged
@@ -572,22 +572,61 @@ flux_column_kernel(int nz, int ni, VbPhoto P, const double* __restrict__ tau, co
 // (photo.py:316-349), then the k row (photo.py:465-478). With a branch at a time
 // and tiles of layers, shared and L2 loads (two per product) bounded the
 // kernel: 64 atmospheres, 120 layers, 2500 bins, 40 branches 640 us -> 272.
+// A tile holds due atmospheres only (due_rows): a run whose atmospheres are due
+// at different times would otherwise pay for four where one is due (update of 64
+// atmospheres with 16 due 570 us -> 452, with all 1511 -> 1502).
 constexpr int J_THREADS = 256;
 constexpr int JW = J_THREADS / 32;
 constexpr int J_ROWS = 4, J_BRANCHES = 5;   // of a full tile; a small batch takes single rows and branches
+
+// The due atmospheres of ranks r0 .. r0 + JT - 1, by increasing index, into
+// rows; returns how many there are (below 1: none). A thread takes a run of
+// consecutive atmospheres; the block's prefix of the counts gives the ranks.
+template <int JT>
+__device__ inline int due_rows(const int32_t* __restrict__ due, int batch, int r0, int* rows) {
+  __shared__ int sums[JW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (batch + J_THREADS - 1) / J_THREADS;
+  const int a0 = min((int)threadIdx.x * per, batch), a1 = min(a0 + per, batch);
+  int n = 0;
+  for (int a = a0; a < a1; ++a) n += due[a] != 0;
+  int incl = n;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  int rank = incl - n, total = 0;
+#pragma unroll
+  for (int q = 0; q < JW; ++q) {
+    rank += q < warp ? sums[q] : 0;
+    total += sums[q];
+  }
+  if (rank < r0 + JT && rank + n > r0)
+    for (int a = a0; a < a1; ++a)
+      if (due[a] != 0) {
+        if (rank >= r0 && rank < r0 + JT) rows[rank - r0] = a;
+        ++rank;
+      }
+  __syncthreads();
+  return min(JT, total - r0);
+}
 
 template <bool ATM, int JT, int JB>
 __global__ void __launch_bounds__(J_THREADS, 2)
 j_kernel(int batch, int nz, int nr, int lt, VbPhoto P, const double* __restrict__ aflux, double* __restrict__ J_br,
          double* __restrict__ J_br_T, double* __restrict__ k, const int32_t* __restrict__ due) {
   extern __shared__ double fs[];   // [lt][nbin]
+  __shared__ int rows[ATM ? JT : 1];   // the tile's atmospheres
   const int b0 = ATM ? blockIdx.y * lt : blockIdx.y, j0 = ATM ? blockIdx.x : blockIdx.x * lt;
-  const int nl = ATM ? min(lt, batch - b0) : min(lt, nz - j0);
-  auto atm_of = [&](int l) { return ATM ? b0 + l : b0; };
+  if (!ATM && due && due[b0] == 0) return;
+  int nl = ATM ? min(lt, batch - b0) : min(lt, nz - j0);
+  if (ATM && due) nl = due_rows<JT>(due, batch, b0, rows);
+  if (nl <= 0) return;
+  auto atm_of = [&](int l) { return !ATM ? b0 : due ? rows[l] : b0 + l; };
   auto layer_of = [&](int l) { return ATM ? j0 : j0 + l; };
-  bool any = due == nullptr;
-  for (int l = 0; l < (ATM ? nl : 1) && !any; ++l) any = due[atm_of(l)] != 0;
-  if (!any) return;
   const int nbin = P.nbin, d12 = P.din12;
   for (int l = 0; l < nl; ++l) {
     const double* f = aflux + ((int64_t)atm_of(l) * nz + layer_of(l)) * nbin;
@@ -604,7 +643,8 @@ j_kernel(int batch, int nz, int nr, int lt, VbPhoto P, const double* __restrict_
     for (int u = 0; u < JB; ++u) {
       const int br = min(br0 + u * step, nb - 1);   // past the last branch: a repeat nobody reads
       const bool is_T = br >= P.n_br;
-      c0[u] = is_T ? P.cross_J_T + (int64_t)b0 * P.T_stride_J + ((int64_t)(br - P.n_br) * nz + j0) * nbin
+      // (a tile of atmospheres shares its tables: T_stride_J = 0)
+      c0[u] = is_T ? P.cross_J_T + (ATM ? 0 : b0 * P.T_stride_J) + ((int64_t)(br - P.n_br) * nz + j0) * nbin
                    : P.cross_J + (int64_t)br * nbin;
       cstep[u] = is_T && !ATM ? nbin : 0;
     }
@@ -652,7 +692,7 @@ j_kernel(int batch, int nz, int nr, int lt, VbPhoto P, const double* __restrict_
           a2 = sum[1][u][l];
         }
     const int u = lane / JT, l = lane % JT, br = br0 + u * step;
-    if (u < JB && l < nl && br < nb && (!due || due[atm_of(l)])) {
+    if (u < JB && l < nl && br < nb) {
       const bool is_T = br >= P.n_br;
       const int brl = is_T ? br - P.n_br : br, b = atm_of(l), j = layer_of(l);
       const double* f = fs + l * nbin;
