@@ -6,7 +6,9 @@ chosen by timing: for every network group of a batch (its species count,
 reaction count, atmosphere count and layer total), each candidate
 ``VbTuning`` (factor kernel, factor CTAs per SM where both variants exist,
 depth of the sweeps' bulk-copy ring) is applied to the network and the
-group's Ros2 step is timed with CUDA events on the device; the fastest is
+group's Ros2 step is timed with CUDA events on the device, next to the
+automatic choice (every field 0), which no candidate equals: its ring is as
+deep as shared memory allows and its assembly goes by size. The fastest is
 kept. Choices are cached in a JSON file keyed by the group's shape and the
 GPU name, and ``MultiNetworkBatch(tuning=...)`` applies a cache before it
 captures its graph.
@@ -74,32 +76,51 @@ def time_call(fn, reps: int = 5, warm: int = 2) -> float:
     return e0.elapsed_time(e1) / reps
 
 
-def tune_group(group: dict, reps: int = 5, split: bool = False) -> tuple[dict, dict]:
-    """Best tuning of one group (dict with step, y, k, dt, sol, delta: a
-    MultiNetworkBatch group or a uniform Ros2Step batch) -> (tuning,
-    {candidate label: ms})."""
+def automatic(split: bool = False):
+    """Tunings with the shapes left to the library; ``split``: also on two streams."""
+    yield dict.fromkeys(FIELDS, 0)
+    if split:
+        yield dict(dict.fromkeys(FIELDS, 0), streams=2)
+
+
+def _tune(group: dict, reps: int, split: bool):
+    """(best tuning, its ms, {candidate label: ms}, ms of the best automatic tuning)."""
     step = group["step"]
     net = step.net
-    timings, best, best_ms = {}, None, float("inf")
+
+    def ms_of(tuning):
+        set_tuning(net, tuning)
+        return time_call(lambda: step(group["y"], group["k"], group["dt"], out=(group["sol"], group["delta"])), reps)
+
+    auto = [(ms_of(t), t) for t in automatic(split)]
+    auto_ms, best = min(auto, key=lambda p: p[0])
+    best_ms, timings = auto_ms, {}
     for cand in candidates(net.ni, split):
-        set_tuning(net, cand)
-        ms = time_call(lambda: step(group["y"], group["k"], group["dt"], out=(group["sol"], group["delta"])), reps)
+        ms = ms_of(cand)
         timings[json.dumps(cand, sort_keys=True)] = ms
         if ms < best_ms:
             best, best_ms = cand, ms
     set_tuning(net, best)
+    return best, best_ms, timings, auto_ms
+
+
+def tune_group(group: dict, reps: int = 5, split: bool = False) -> tuple[dict, dict]:
+    """Best tuning of one group (dict with step, y, k, dt, sol, delta: a
+    MultiNetworkBatch group or a uniform Ros2Step batch) -> (tuning,
+    {candidate label: ms})."""
+    best, _, timings, _ = _tune(group, reps, split)
     return best, timings
 
 
 def tune_batch(batch, cache_path: str | None = None, reps: int = 5) -> dict:
     """Tune every group of a MultiNetworkBatch (before capture); returns
-    {group key: {"tuning": ..., "ms": ..., "candidates": ...}} and, with
-    cache_path, merges it into that JSON file."""
+    {group key: {"tuning": ..., "ms": ..., "automatic_ms": ..., "candidates":
+    ...}} and, with cache_path, merges it into that JSON file."""
     out = {}
     for g in batch.groups:
-        best, timings = tune_group(g, reps)
+        best, best_ms, timings, auto_ms = _tune(g, reps, False)
         key = group_key(g["step"].net, g["step"].batch, g["step"].layers)
-        out[key] = {"tuning": best, "ms": min(timings.values()), "candidates": timings}
+        out[key] = {"tuning": best, "ms": best_ms, "automatic_ms": auto_ms, "candidates": timings}
     if cache_path:
         cache = load_cache(cache_path)
         cache.update(out)
