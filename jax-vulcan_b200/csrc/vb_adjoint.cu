@@ -106,32 +106,51 @@ vjp_transport_kernel(Batch B, const double* __restrict__ y, const double* __rest
 
 // ---- cotangents of every transport leaf of the atmosphere blob
 // One stencil row's diffusion term (jax_step.py:67-246) of species i in flux
-// form, F = E / dz with
-//   E = (K2+D2)/d2 q2 - (K1+D1)/d1 q1 + c (D2 P2 - D1 P1) + advection terms,
-//   q2 = (ysp+ys0)/2 (yp/ysp - y0/ys0),   q1 = (ys0+ysm)/2 (y0/ys0 - ym/ysm),
-//   P2 = (-1/H2 + alpha/T2 (Tp-T0)/d2) (y0+yp) + ms/(Navo kb T2) (g0 y0 + gp yp)
-// (2: the interface above, j; 1: the one below, j-1; c = 1/2, 0 with vm; the
-// end rows have one interface, its spacing as dz and their own gravity in both
-// terms), differentiated by hand in every leaf at once: one evaluation per
-// (row, species) instead of one per leaf element, row and species.
+// form is (F of its upper interface - F of its lower one) / dz, with
+//   F = (K+D)/d q + c D P + advection terms,   q = (y1s+y0s)/2 (y1/y1s - y0/y0s),
+//   P = (-1/H + alpha/T (T1-T0)/d) (y0+y1) + ms/(Navo kb T) (g0 y0 + g1 y1)
+// (0, 1: the layers below and above the interface; c = 1/2, 0 with vm; the end
+// rows have one interface, its spacing as dz and their own gravity in both
+// terms). Differentiated by hand in every leaf at once: one evaluation per
+// (interface, species). An interface enters the two rows with opposite sign, so
+// its leaves take the difference lambda_0/dz_0 - lambda_1/dz_1, formed first
+// (RowPair): lambda is nearly conserved from layer to layer where the chemistry
+// is slow, and the difference of the rows' products, each rounded, lost its
+// digits (alpha against long double from the same lambda, median relative error:
+// 2.8e-12 at 69 species and 17 layers with the rows apart, 1.2e-12 with dual
+// numbers, 1.7e-13 so).
 //
-// CTA per block of VA_ROWS layers of an atmosphere, a warp per stencil row that
-// enters them (two more than the layers), lanes over species: the layer fields'
-// derivatives are summed over species in the warp, the species' own go to
-// shared memory, and every leaf element then adds the two or three rows it
-// enters, in a fixed order. FP64 arithmetic bound (about 20 divisions a row and
-// species). ni=69, nz=120, 64 atmospheres (B200): a thread per leaf element
-// with dual numbers 12.8 ms (4 to 120 rows times up to 69 species each, 21.6 M
-// evaluations), the two kernels below 0.077 and 0.064 ms (0.66 M evaluations of the rows).
+// CTA per block of VA_ROWS layers of an atmosphere, a warp per interface that
+// enters their leaves (two more than the layers), lanes over species: the layer
+// fields' derivatives are summed over species in the warp, the species' own are
+// written at once, and every layer element then adds the one to three
+// interfaces it enters, in a fixed order. FP64 arithmetic bound. ni=69, nz=120,
+// 64 atmospheres (B200), both kernels: a thread per leaf element with dual
+// numbers 12.8 ms (4 to 120 rows times up to 69 species each, 21.6 M
+// evaluations), a warp per row 0.130 ms, now 0.089 (0.53 M evaluations).
 constexpr int VA_ROWS = 8;
 constexpr int VA_WARPS = VA_ROWS + 2;
-constexpr int VA_SLOTS = 16;   // layer-field derivatives of a row (VaSlot)
-enum VaSlot { S_K2, S_K1, S_D2, S_D1, S_V2, S_V1, S_H2, S_H1, S_T2, S_T1, S_TM, S_T0, S_TP, S_GM, S_G0, S_GP };
-constexpr int VA_SPEC = 6;     // species' own: Dzz, vm, vs at j and at j-1
+// layer-field derivatives of an interface: Kzz, vz, Hpi, Ti, the spacing (not
+// through dz), the temperature of the layer above (minus that of the one below),
+// gravity of the layers below and above, lambda F / dz of the rows below and above
+enum VaSlot { S_K, S_V, S_H, S_T, S_D, S_TCO, S_G0, S_G1, S_R0, S_R1, VA_SLOTS };
+
+// The rows j and j + 1 that an interface enters: their dz, and
+// lambda_j / dz_j - lambda_{j+1} / dz_{j+1} to a few roundings of its value.
+struct RowPair {
+  double rz0, rz1, rho, err;   // 1/dz of both, dz_j / dz_{j+1} and what it rounded off (over dz_{j+1})
+  __device__ RowPair(const double* dzi, int nz, int j) {
+    const double d = dzi[j], h0 = j == 0 ? d : 0.5 * (dzi[j - 1] + d), h1 = j == nz - 2 ? d : 0.5 * (d + dzi[j + 1]);
+    rz0 = 1.0 / h0;
+    rz1 = 1.0 / h1;
+    rho = h0 / h1;
+    err = fma(-rho, h1, h0) * rz1;
+  }
+  __device__ double diff(double l0, double l1) const { return (fma(-rho, l1, l0) - err * l1) * rz0; }
+};
 
 __host__ __device__ inline size_t vjp_atm_smem_bytes(int ni) {
-  return ((size_t)(VA_ROWS + 4) * ni + ni + (VA_ROWS + 4) + VA_WARPS * VA_SLOTS + (size_t)VA_WARPS * VA_SPEC * ni) *
-         sizeof(double);
+  return ((size_t)(VA_ROWS + 3) * ni + ni + (VA_ROWS + 3) + VA_WARPS * VA_SLOTS) * sizeof(double);
 }
 
 __global__ void __launch_bounds__(VA_WARPS * 32)
@@ -145,147 +164,107 @@ vjp_atm_rows_kernel(Batch B, const double* __restrict__ y, const double* __restr
   const AtmRef a = atm_ref(atm + g.atm, nz, ni);
   const double* yb = y + g.z0 * ni;
   const double* lb = lam + g.z0 * ni;
-  double* yr = sm;                                  // [VA_ROWS + 4][ni]: layers m0-2 ..
-  double* gas = yr + (VA_ROWS + 4) * ni;
-  double* ysum = gas + ni;                          // [VA_ROWS + 4]
-  double* S = ysum + VA_ROWS + 4;                   // [VA_WARPS][VA_SLOTS]: rows m0-1 ..
-  double* P = S + VA_WARPS * VA_SLOTS;              // [VA_WARPS][VA_SPEC][ni]
+  double* yr = sm;                                  // [VA_ROWS + 3][ni]: layers m0-1 ..
+  double* gas = yr + (VA_ROWS + 3) * ni;
+  double* ysum = gas + ni;                          // [VA_ROWS + 3]
+  double* S = ysum + VA_ROWS + 3;                   // [VA_WARPS][VA_SLOTS]: interfaces m0-1 ..
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < (VA_ROWS + 4) * ni; e += VA_WARPS * 32) {
-    const int jj = m0 - 2 + e / ni;
-    yr[e] = (jj >= 0 && jj < nz) ? yb[(int64_t)(m0 - 2) * ni + e] : 0.0;
+  for (int e = threadIdx.x; e < (VA_ROWS + 3) * ni; e += VA_WARPS * 32) {
+    const int jj = m0 - 1 + e / ni;
+    yr[e] = (jj >= 0 && jj < nz) ? yb[(int64_t)(m0 - 1) * ni + e] : 0.0;
   }
   for (int i = threadIdx.x; i < ni; i += VA_WARPS * 32) gas[i] = a.gas[i];
   __syncthreads();
   // gas sums of the rows (0 outside the column, as the forward kernels)
-  if (threadIdx.x < VA_ROWS + 4) {
-    const int jj = m0 - 2 + (int)threadIdx.x;
+  if (threadIdx.x < VA_ROWS + 3) {
+    const int jj = m0 - 1 + (int)threadIdx.x;
     ysum[threadIdx.x] = (jj >= 0 && jj < nz) ? pairwise_sum_masked(yr + threadIdx.x * ni, gas, ni) : 0.0;
-  }
-  __syncthreads();
-  {
-    const int j = m0 - 1 + warp;
-    const bool row = j >= 0 && j < nz, up = row && j < nz - 1, dn = row && j > 0;
-    double acc[VA_SLOTS] = {};
-    if (row) {
-      const double use_vm = (flags & VB_USE_VM_MOL) ? 1.0 : 0.0, use_set = (flags & VB_USE_SETTLING) ? 1.0 : 0.0;
-      const double c = 0.5 * (1.0 - use_vm);
-      const double* y0r = yr + (warp + 1) * ni;
-      const double ys0 = ysum[warp + 1], ysm = ysum[warp], ysp = ysum[warp + 2];
-      const double d2 = up ? a.dzi[j] : 0.0, d1 = dn ? a.dzi[j - 1] : 0.0;
-      const double rz = (up && dn) ? 1.0 / (0.5 * (d1 + d2)) : 1.0 / (up ? d2 : d1);
-      const double drz = (up && dn) ? -0.5 * rz : -rz;   // d(1/dz)/d(spacing) = drz / dz
-      const double K2 = up ? a.Kzz[j] : 0.0, K1 = dn ? a.Kzz[j - 1] : 0.0;
-      const double v2 = up ? a.vz[j] : 0.0, v1 = dn ? a.vz[j - 1] : 0.0;
-      const double rH2 = up ? 1.0 / a.Hpi[j] : 0.0, rH1 = dn ? 1.0 / a.Hpi[j - 1] : 0.0;
-      const double rT2 = up ? 1.0 / a.Ti[j] : 0.0, rT1 = dn ? 1.0 / a.Ti[j - 1] : 0.0;
-      const double rd2 = up ? 1.0 / d2 : 0.0, rd1 = dn ? 1.0 / d1 : 0.0;
-      const double T0 = a.Tco[j];
-      const double t2 = up ? (a.Tco[j + 1] - T0) * rd2 : 0.0, t1 = dn ? (T0 - a.Tco[j - 1]) * rd1 : 0.0;
-      const double g0 = a.g[j], gp = (up && dn) ? a.g[j + 1] : g0, gm = (up && dn) ? a.g[j - 1] : g0;
-      const double S2 = 0.5 * (ysp + ys0), S1 = 0.5 * (ys0 + ysm);
-      for (int i = lane; i < ni; i += 32) {
-        const double y0 = y0r[i], yp = y0r[ni + i], ym = y0r[i - ni];
-        const double L = lb[(int64_t)j * ni + i], w = L * rz;
-        const double al = a.alpha[i], mk = a.ms[i] / (NAVO * KB);
-        double E = 0.0, sp[VA_SPEC] = {};
-        // derivative of an advection term of interface speed v: upwind from below / above
-        auto wind = [](double v, double below, double above) { return v > 0.0 ? below : (v < 0.0 ? above : 0.0); };
-        if (up) {
-          const double D2 = a.Dzz[(int64_t)j * ni + i], vm = a.vm[(int64_t)j * ni + i], vs = a.vs[(int64_t)j * ni + i];
-          const double q = S2 * (yp / ysp - y0 / ys0), s = y0 + yp, gy = g0 * y0 + gp * yp;
-          const double th = al * rT2 * t2, Pm = (th - rH2) * s + mk * rT2 * gy;
-          const double wc = w * c * D2, th_w = wc * al * rT2 * rd2 * s, gw = wc * mk * rT2;
-          E += (K2 + D2) * rd2 * q + c * D2 * Pm;
-          acc[S_K2] += w * q * rd2;
-          sp[0] = w * (q * rd2 + c * Pm);
-          acc[S_H2] += wc * s * rH2 * rH2;
-          acc[S_T2] -= wc * (th * s + mk * rT2 * gy) * rT2;
-          acc[S_TP] += th_w;
-          acc[S_T0] -= th_w;
-          acc[S_G0] += gw * y0;
-          acc[dn ? S_GP : S_G0] += gw * yp;
-          acc[S_D2] -= w * (K2 + D2) * rd2 * rd2 * q + wc * th * rd2 * s;
-          const double ez = -wind(v2, y0, yp), em = -wind(vm, y0, yp), es = -wind(vs, y0, yp);
-          acc[S_V2] += w * ez;
-          sp[2] = use_vm * w * em;
-          sp[4] = use_set * w * es;
-          E += v2 * ez + use_vm * vm * em + use_set * vs * es;
-        }
-        if (dn) {
-          const int64_t mv = (int64_t)(up ? j - 1 : j) * ni + i;   // the top row reads its own vm
-          const double D1 = a.Dzz[(int64_t)(j - 1) * ni + i], vm = a.vm[mv], vs = a.vs[(int64_t)(j - 1) * ni + i];
-          const double q = S1 * (y0 / ys0 - ym / ysm), s = y0 + ym, gy = g0 * y0 + gm * ym;
-          const double th = al * rT1 * t1, Pm = (th - rH1) * s + mk * rT1 * gy;
-          const double wc = w * c * D1, th_w = wc * al * rT1 * rd1 * s, gw = wc * mk * rT1;
-          E -= (K1 + D1) * rd1 * q + c * D1 * Pm;
-          acc[S_K1] -= w * q * rd1;
-          sp[1] = -w * (q * rd1 + c * Pm);
-          acc[S_H1] -= wc * s * rH1 * rH1;
-          acc[S_T1] += wc * (th * s + mk * rT1 * gy) * rT1;
-          acc[S_TM] += th_w;
-          acc[S_T0] -= th_w;
-          acc[S_G0] -= gw * y0;
-          acc[up ? S_GM : S_G0] -= gw * ym;
-          acc[S_D1] += w * (K1 + D1) * rd1 * rd1 * q + wc * th * rd1 * s;
-          const double ez = wind(v1, ym, y0), em = wind(vm, ym, y0), es = wind(vs, ym, y0);
-          acc[S_V1] += w * ez;
-          sp[up ? 3 : 2] += use_vm * w * em;
-          sp[5] = use_set * w * es;
-          E += v1 * ez + use_vm * vm * em + use_set * vs * es;
-        }
-        const double dF = L * drz * rz * E;
-        if (up) acc[S_D2] += dF;
-        if (dn) acc[S_D1] += dF;
-        if (j == 0 && (flags & VB_USE_BOTFLUX)) acc[S_D2] -= L * (a.bot[i] - y0 * a.vdep[i]) * rd2 * rd2;
-        if (j == nz - 1 && (flags & VB_USE_TOPFLUX)) acc[S_D1] -= L * a.top[i] * rd1 * rd1;
-#pragma unroll
-        for (int q = 0; q < VA_SPEC; ++q) P[(warp * VA_SPEC + q) * ni + i] = sp[q];
-      }
-    } else {
-      for (int e = lane; e < VA_SPEC * ni; e += 32) P[warp * VA_SPEC * ni + e] = 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < VA_SLOTS; ++q) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < VA_SLOTS; ++q) S[warp * VA_SLOTS + q] = acc[q];
-    }
   }
   __syncthreads();
   const AtmOff o = atm_offsets(nz, ni);
   double* out = g_atm + g.atm;
-  for (int e = threadIdx.x; e < 7 * VA_ROWS; e += VA_WARPS * 32) {
-    const int f = e / VA_ROWS, l = e % VA_ROWS, m = m0 + l;
-    const double* s = S + l * VA_SLOTS;   // row m - 1; rows m and m + 1 follow
-    if (f < 5) {
-      const int64_t off[5] = {o.Kzz, o.dzi, o.vz, o.Hpi, o.Ti};
-      if (m < nz - 1) out[off[f] + m] = -(s[VA_SLOTS + 2 * f] + s[2 * VA_SLOTS + 2 * f + 1]);
-    } else if (m < nz) {
-      const int q = f == 5 ? S_TM : S_GM;   // j-1, j, j+1 of the field
-      out[(f == 5 ? o.Tco : o.g) + m] = -(s[q + 2] + s[VA_SLOTS + q + 1] + s[2 * VA_SLOTS + q]);
+  {
+    const int q = m0 - 1 + warp;
+    double acc[VA_SLOTS] = {};
+    if (q >= 0 && q < nz - 1) {
+      const bool lo = q == 0, hi = q == nz - 2, mine = q >= m0 && q < m0 + VA_ROWS;
+      const double use_vm = (flags & VB_USE_VM_MOL) ? 1.0 : 0.0, use_set = (flags & VB_USE_SETTLING) ? 1.0 : 0.0;
+      const double c = 0.5 * (1.0 - use_vm);
+      const double *y0r = yr + warp * ni, *l0r = lb + (int64_t)q * ni;
+      const double ys0 = ysum[warp], ys1 = ysum[warp + 1], half = 0.5 * (ys1 + ys0);
+      const RowPair rows(a.dzi, nz, q);
+      const double rd = 1.0 / a.dzi[q], K = a.Kzz[q], v = a.vz[q], rH = 1.0 / a.Hpi[q], rT = 1.0 / a.Ti[q];
+      const double t = (a.Tco[q + 1] - a.Tco[q]) * rd, g0 = a.g[q], g1 = a.g[q + 1];
+      // derivative of an advection term of interface speed v: upwind from below / above
+      auto wind = [](double v, double below, double above) { return v > 0.0 ? below : (v < 0.0 ? above : 0.0); };
+      for (int i = lane; i < ni; i += 32) {
+        const int64_t at = (int64_t)q * ni + i;
+        const double y0 = y0r[i], y1 = y0r[ni + i], l0 = l0r[i], l1 = l0r[ni + i];
+        const double w0 = l0 * rows.rz0, w1 = l1 * rows.rz1, w = rows.diff(l0, l1);
+        const double D = a.Dzz[at], al = a.alpha[i], mk = a.ms[i] / (NAVO * KB) * rT;
+        const double vm0 = a.vm[at], vm1 = hi ? a.vm[at + ni] : vm0, vs = a.vs[at];   // the top row reads its own vm
+        const double qd = half * (y1 / ys1 - y0 / ys0), s = y0 + y1;
+        const double th = al * rT * t, Bt = th * s + mk * (g0 * y0 + g1 * y1), Pm = Bt - rH * s;
+        const double e0 = lo ? mk * (g0 - g1) * y1 : 0.0, e1 = hi ? mk * (g1 - g0) * y0 : 0.0;   // end rows' gravity
+        const double cD = c * D, cor = w0 * e0 - w1 * e1, wc = w * cD, gw = cD * mk;
+        const double ez = -wind(v, y0, y1), em0 = -wind(vm0, y0, y1), em1 = -wind(vm1, y0, y1), es = -wind(vs, y0, y1);
+        acc[S_K] += w * qd * rd;
+        acc[S_V] += w * ez;
+        acc[S_H] += wc * s * rH * rH;
+        acc[S_T] -= (wc * Bt + cD * cor) * rT;
+        acc[S_D] -= w * (K + D) * rd * rd * qd + wc * th * rd * s;
+        acc[S_TCO] += wc * al * rT * rd * s;
+        acc[S_G0] += gw * ((hi ? w0 : w) * y0 + (lo ? w0 * y1 : 0.0));
+        acc[S_G1] += gw * ((lo ? -w1 : w) * y1 - (hi ? w1 * y0 : 0.0));
+        const double F = (K + D) * rd * qd + v * ez + use_set * vs * es;
+        acc[S_R0] += w0 * (F + cD * (Pm + e0) + use_vm * vm0 * em0);
+        acc[S_R1] -= w1 * (F + cD * (Pm + e1) + use_vm * vm1 * em1);
+        if (lo && (flags & VB_USE_BOTFLUX)) acc[S_D] -= l0 * (a.bot[i] - y0 * a.vdep[i]) * rd * rd;
+        if (hi && (flags & VB_USE_TOPFLUX)) acc[S_D] -= l1 * a.top[i] * rd * rd;
+        if (mine) {
+          out[o.Dzz + at] = -(w * (qd * rd + c * Pm) + c * cor);
+          out[o.vs + at] = -(use_set * w * es);
+          out[o.vm + at] = -(use_vm * (hi ? w0 : w) * em0);
+          if (hi) out[o.vm + at + ni] = use_vm * w1 * em1;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < VA_SLOTS; ++k) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int k = 0; k < VA_SLOTS; ++k) S[warp * VA_SLOTS + k] = acc[k];
     }
   }
-  for (int e = threadIdx.x; e < VA_ROWS * ni; e += VA_WARPS * 32) {
-    const int l = e / ni, i = e - l * ni, m = m0 + l;
-    if (m >= nz) break;
-    const double* r0 = P + (l + 1) * VA_SPEC * ni + i;   // row m
-    const double* r1 = r0 + VA_SPEC * ni;                // row m + 1
-    const int64_t at = (int64_t)m * ni + i;
-    if (m < nz - 1) {
-      out[o.Dzz + at] = -(r0[0] + r1[ni]);
-      out[o.vs + at] = -(r0[4 * ni] + r1[5 * ni]);
+  __syncthreads();
+  for (int e = threadIdx.x; e < 7 * VA_ROWS; e += VA_WARPS * 32) {
+    const int f = e / VA_ROWS, l = e % VA_ROWS, m = m0 + l;
+    const double *s0 = S + l * VA_SLOTS, *s1 = s0 + VA_SLOTS, *s2 = s1 + VA_SLOTS;   // interfaces m - 1, m, m + 1
+    if (f < 4) {
+      const int64_t off[4] = {o.Kzz, o.vz, o.Hpi, o.Ti};
+      if (m < nz - 1) out[off[f] + m] = -s1[f];
+    } else if (f == 4) {
+      // the spacing itself, and as the dz (or half of it) of rows m and m + 1
+      if (m < nz - 1) {
+        const double c0 = m == 0 ? 1.0 / a.dzi[0] : 0.5 / (0.5 * (a.dzi[m - 1] + a.dzi[m]));
+        const double c1 = m == nz - 2 ? 1.0 / a.dzi[m] : 0.5 / (0.5 * (a.dzi[m] + a.dzi[m + 1]));
+        out[o.dzi + m] = -(s1[S_D] - c0 * (s0[S_R1] + s1[S_R0]) - c1 * (s1[S_R1] + s2[S_R0]));
+      }
+    } else if (m < nz) {
+      if (f == 5)
+        out[o.Tco + m] = -(s0[S_TCO] - s1[S_TCO]);
+      else
+        out[o.g + m] = -(s0[S_G1] + s1[S_G0]);
     }
-    out[o.vm + at] = -(r0[2 * ni] + r1[3 * ni]);
   }
 }
 
 // The leaves with one element per species: ms and alpha (summed over the
-// column), the boundary fluxes and the deposition velocity. CTA per atmosphere,
-// warps over rows, lanes over species.
+// column's interfaces), the boundary fluxes and the deposition velocity. CTA
+// per atmosphere, warps over interfaces, lanes over species.
 __global__ void __launch_bounds__(VJP_THREADS)
 vjp_atm_species_kernel(Batch B, const double* __restrict__ y, const double* __restrict__ atm, int flags,
                        const double* __restrict__ lam, double* __restrict__ g_atm) {
@@ -301,21 +280,16 @@ vjp_atm_species_kernel(Batch B, const double* __restrict__ y, const double* __re
   const double c = (flags & VB_USE_VM_MOL) ? 0.0 : 0.5;
   for (int i = lane; i < ni; i += 32) {
     double gms = 0.0, gal = 0.0;
-    for (int j = warp; j < nz; j += NWARP) {
-      const bool up = j < nz - 1, dn = j > 0;
-      const double d2 = up ? a.dzi[j] : 0.0, d1 = dn ? a.dzi[j - 1] : 0.0;
-      const double dz = (up && dn) ? 0.5 * (d1 + d2) : (up ? d2 : d1);
-      const double w = c * lb[(int64_t)j * ni + i] / dz, y0 = yb[(int64_t)j * ni + i], g0 = a.g[j];
-      if (up) {
-        const double yp = yb[(int64_t)(j + 1) * ni + i], D = w * a.Dzz[(int64_t)j * ni + i] / a.Ti[j];
-        gms += D * (g0 * y0 + (dn ? a.g[j + 1] : g0) * yp);
-        gal += D * ((a.Tco[j + 1] - a.Tco[j]) / d2) * (y0 + yp);
-      }
-      if (dn) {
-        const double ym = yb[(int64_t)(j - 1) * ni + i], D = w * a.Dzz[(int64_t)(j - 1) * ni + i] / a.Ti[j - 1];
-        gms -= D * (g0 * y0 + (up ? a.g[j - 1] : g0) * ym);
-        gal -= D * ((a.Tco[j] - a.Tco[j - 1]) / d1) * (y0 + ym);
-      }
+    for (int q = warp; q < nz - 1; q += NWARP) {
+      const int64_t at = (int64_t)q * ni + i;
+      const RowPair rows(a.dzi, nz, q);
+      const double y0 = yb[at], y1 = yb[at + ni], l0 = lb[at], l1 = lb[at + ni], w = rows.diff(l0, l1);
+      const double D = c * a.Dzz[at] / a.Ti[q], g0 = a.g[q], g1 = a.g[q + 1];
+      // the end rows' own gravity in both terms
+      const double e0 = q == 0 ? l0 * rows.rz0 * (g0 - g1) * y1 : 0.0;
+      const double e1 = q == nz - 2 ? l1 * rows.rz1 * (g1 - g0) * y0 : 0.0;
+      gms += D * (w * (g0 * y0 + g1 * y1) + (e0 - e1));
+      gal += D * ((a.Tco[q + 1] - a.Tco[q]) / a.dzi[q]) * (y0 + y1) * w;
     }
     red[0][warp][i] = gms;
     red[1][warp][i] = gal;
