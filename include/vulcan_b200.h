@@ -121,7 +121,8 @@ size_t vb_ros2_workspace_bytes(int batch, int nz, int ni, const int64_t* zoff_ho
  * that region, then every species sum formed from coalesced rows of layers)
  * instead of one CTA per layer, where the batch is too small for tiles of
  * eight layers per CTA (two CTAs per SM) or their rates exceed shared memory;
- * the results are identical. nr+1 doubles per layer. */
+ * the results are identical. nr+1 doubles per layer; 0 where the batch, and
+ * its halves on two streams, go by tiles and would not use it. */
 size_t vb_ros2_assembly_bytes(const VbNet* net, int batch, int nz);
 int vb_ros2_step(const VbNet* net, int batch, int nz, const int64_t* zoff,
                  const double* y, const double* k, const double* dt,

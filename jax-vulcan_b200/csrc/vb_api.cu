@@ -347,22 +347,31 @@ static vb::Batch make_batch(const VbNet* net, int batch, int nz, const int64_t* 
   return B;
 }
 
-// The launch sequence of one Ros2 step (jax_step.py:249-315) on one stream.
+// 0 where the stage 2 of the batch, and of its halves on two streams, goes by
+// tiles, which keep the rates in shared memory.
 size_t vb_ros2_assembly_bytes(const VbNet* net, int batch, int nz) {
   if (!net || batch < 1 || nz < 1) return 0;
+  vb::Batch half{};
+  half.count = batch > 1 ? batch / 2 : 1;
+  half.nz = nz;
+  half.ni = net->dev.ni;
+  half.nr = net->dev.nr;
+  if (vb::stage2_tiles(half)) return 0;
   return (size_t)batch * nz * vb::rates_region_doubles(net->dev.nr) * sizeof(double);
 }
 
-// The rate region of the layer-vectorized stage 2 in a vb_ros2_step
-// workspace (after the step's own bytes, on a 256-byte boundary), or nullptr
-// when the workspace does not hold it (the per-layer stage-2 kernel runs then).
-static double* assembly_region(const VbNet* net, int batch, int nz, void* ws, size_t ws_bytes) {
-  const size_t off = (vb_ros2_workspace_bytes(batch, nz, net->dev.ni, nullptr) + 255) & ~(size_t)255;
+// The rate region of the layer-vectorized stage 2 in a step's workspace, after
+// the step's own bytes on a 256-byte boundary, or nullptr when there is none
+// (the batch does not use it, or the workspace does not hold it and the
+// per-layer stage-2 kernel runs).
+static double* assembly_region(const VbNet* net, int batch, int nz, void* ws, size_t ws_bytes, size_t own) {
+  const size_t off = (own + 255) & ~(size_t)255;
   const size_t need = vb_ros2_assembly_bytes(net, batch, nz);
-  if (ws_bytes < off || ws_bytes - off < need) return nullptr;
+  if (need == 0 || ws_bytes < off || ws_bytes - off < need) return nullptr;
   return reinterpret_cast<double*>(static_cast<char*>(ws) + off);
 }
 
+// The launch sequence of one Ros2 step (jax_step.py:249-315) on one stream.
 static int ros2_sequence(const VbNet* net, const vb::Batch& B, const double* y, const double* k, const double* dt,
                          const double* atm, int32_t flags, const uint8_t* fix_mask, double* sol, double* delta,
                          int32_t* status, double* ws, cudaStream_t st) {
@@ -437,7 +446,8 @@ int vb_ros2_step(const VbNet* net, int batch, int nz, const int64_t* zoff, const
     return fail(VB_ERR_ARG, "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
   double* ws = (double*)workspace;
-  double* rates = assembly_region(net, batch, nz, workspace, ws_bytes);
+  double* rates = assembly_region(net, batch, nz, workspace, ws_bytes,
+                                  vb_ros2_workspace_bytes(batch, nz, net->dev.ni, nullptr));
   VB_CHECK(cudaMemsetAsync(status, 0, sizeof(int32_t) * batch, st), "status reset");
   if (net->tune.streams != 2 || zoff || batch < 2) {
     vb::Batch B = make_batch(net, batch, nz, zoff);
@@ -512,13 +522,7 @@ int vb_ros2_step_mixed(const VbNet* net, int batch, int nz, const int64_t* zoff,
   cudaStream_t st = (cudaStream_t)stream;
   vb::Batch B = make_batch(net, batch, nz, zoff);
   char* base = (char*)workspace;
-  // the optional rate region of the thread-per-layer stage 2, after the
-  // mixed step's own bytes on a 256-byte boundary
-  {
-    const size_t off = (L.total + 255) & ~(size_t)255;
-    if (ws_bytes >= off && ws_bytes - off >= vb_ros2_assembly_bytes(net, batch, nz))
-      B.rates = reinterpret_cast<double*>(base + off);
-  }
+  B.rates = assembly_region(net, batch, nz, workspace, ws_bytes, L.total);
   double* ws = (double*)base;
   void* mxr = base + L.mx;
   int32_t* mode = (int32_t*)(base + L.mode);

@@ -1305,18 +1305,21 @@ static cudaError_t launch_stage2_t(const NetDev& net, const Batch& B, const doub
   return cudaGetLastError();
 }
 
+// Tiles where their rates fit shared memory and two CTAs per SM have work;
+// fewer layers leave SMs idle that the reaction chunks of the thread-per-layer
+// passes fill. Measured on B200, thread per layer / tiles, stage 2 with the
+// diffusion rows: 0.63 / 0.51 ms (296 atmospheres of 69 species, 120 layers),
+// 0.72 / 0.51 (128 of 89, 150 layers), 0.083 / 0.041 (33 of 45, 97 layers).
+bool stage2_tiles(const Batch& B) {
+  return tz_smem_bytes(B.ni, B.nr) <= 220 * 1024 && (int64_t)B.count * ((B.nz + TZ - 1) / TZ) >= 2 * sm_count();
+}
+
 cudaError_t launch_stage2(const NetDev& net, const Batch& B, const double* y, const double* k,
                           const double* dt, const double* atm, int flags, const uint8_t* fm, double* ws,
                           cudaStream_t st, double* resid) {
   cudaError_t e = launch_diffusion_rows(B, y, atm, flags, fm, ws, resid, 2, st);
   if (e != cudaSuccess) return e;
-  // Tiles where their rates fit shared memory and two CTAs per SM have work;
-  // fewer layers leave SMs idle that the reaction chunks of the thread-per-layer
-  // passes fill. Measured on B200, thread per layer / tiles, stage 2 with the
-  // diffusion rows: 0.63 / 0.51 ms (296 atmospheres of 69 species, 120 layers),
-  // 0.72 / 0.51 (128 of 89, 150 layers), 0.083 / 0.041 (33 of 45, 97 layers).
-  if (!resid && tz_smem_bytes(B.ni, B.nr) <= 220 * 1024 && (int64_t)B.count * ((B.nz + TZ - 1) / TZ) >= 2 * sm_count())
-    return launch_stage2_tiles(net, B, y, k, dt, atm, fm, ws, st);
+  if (!resid && stage2_tiles(B)) return launch_stage2_tiles(net, B, y, k, dt, atm, fm, ws, st);
   if (!resid && B.stage1_layers == 2) return launch_stage2_t<2>(net, B, y, k, dt, atm, fm, ws, st, resid);
   if (!resid && B.rates) return launch_lv_stage2(net, B, y, k, dt, atm, fm, ws, st);
   return launch_stage2_t<1>(net, B, y, k, dt, atm, fm, ws, st, resid);

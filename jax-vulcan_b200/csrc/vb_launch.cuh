@@ -25,6 +25,8 @@ cudaError_t launch_stage1(const NetDev&, const Batch&, const double* y, const do
                           const double* adj_v = nullptr);
 // resid != nullptr: write the residual f(y) = chem + diffusion to resid [B][nz][ni]
 // instead of the stage-2 right-hand side.
+// Whether the batch's stage 2 goes by tiles of layers (which use no rate region).
+bool stage2_tiles(const Batch& B);
 cudaError_t launch_stage2(const NetDev&, const Batch&, const double* y, const double* k, const double* dt,
                           const double* atm, int flags, const uint8_t* fix_mask, double* ws, cudaStream_t,
                           double* resid = nullptr);

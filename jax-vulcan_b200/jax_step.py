@@ -105,10 +105,10 @@ class Ros2Step:
         of both stages, at most ``max_refine`` passes to ``tol``, FP64
         fallback); ``self.passes`` then holds the passes run per atmosphere.
         ``assembly``: allocate the rate region of the layer-vectorized
-        stage 2 (``vb_ros2_assembly_bytes``: nr+1 doubles per layer), so the
-        stage-2 right-hand side is formed with a thread per layer where the
-        batch is too small for tiles of eight layers per CTA; False: the
-        per-layer stage-2 kernel there (same results, less memory)."""
+        stage 2 (``vb_ros2_assembly_bytes``: nr+1 doubles per layer, none where
+        the batch goes by tiles of eight layers per CTA), so the stage-2
+        right-hand side of a smaller batch is formed with a thread per layer;
+        False: the per-layer stage-2 kernel there (same results, less memory)."""
         self.net = net
         self.mixed = bool(mixed)
         self.max_refine = int(max_refine)
@@ -125,9 +125,9 @@ class Ros2Step:
         L = _lib.lib()
         size = L.vb_ros2_mixed_workspace_bytes if self.mixed else L.vb_ros2_workspace_bytes
         self.ws_bytes = int(size(self.batch, self.nz, ni, None))
-        if assembly:
-            self.ws_bytes = ((self.ws_bytes + 255) & ~255) + int(
-                L.vb_ros2_assembly_bytes(net.handle, self.batch, self.nz))
+        region = int(L.vb_ros2_assembly_bytes(net.handle, self.batch, self.nz)) if assembly else 0
+        if region:
+            self.ws_bytes = ((self.ws_bytes + 255) & ~255) + region
         self.ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device="cuda")
         self.status = torch.zeros(self.batch, dtype=torch.int32, device="cuda")
         self.passes = torch.zeros(self.batch, dtype=torch.int32, device="cuda")
@@ -221,9 +221,9 @@ class RaggedRos2Step:
         self.blob = torch.cat(blobs).contiguous()
         L = _lib.lib()
         self.ws_bytes = int(L.vb_ros2_workspace_bytes(self.batch, self.nz_max, ni, self.zoff_host.ctypes.data))
-        if assembly:
-            self.ws_bytes = ((int(L.vb_ros2_workspace_bytes(self.batch, self.nz_max, ni, None)) + 255) & ~255) + \
-                int(L.vb_ros2_assembly_bytes(net.handle, self.batch, self.nz_max))
+        region = int(L.vb_ros2_assembly_bytes(net.handle, self.batch, self.nz_max)) if assembly else 0
+        if region:
+            self.ws_bytes = ((int(L.vb_ros2_workspace_bytes(self.batch, self.nz_max, ni, None)) + 255) & ~255) + region
         self.ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device="cuda")
         self.status = torch.zeros(self.batch, dtype=torch.int32, device="cuda")
 
