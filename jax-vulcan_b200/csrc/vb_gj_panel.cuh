@@ -30,6 +30,14 @@ template <typename R>
 __device__ __forceinline__ unsigned pivot_key32(R v, int row) {
   return (pivot_mag(v) & 0xffffff00u) | (unsigned)(255 - row);
 }
+// Largest key of a lane's rows (two at a time: one instruction).
+template <int N>
+__device__ __forceinline__ unsigned key_max(const unsigned (&k)[N]) {
+  unsigned m = k[0];
+#pragma unroll
+  for (int r = 1; r + 1 < N; r += 2) m = __vimax3_u32(m, k[r], k[r + 1]);
+  return N % 2 == 0 ? max(m, k[N - 1]) : m;
+}
 __device__ __forceinline__ int pivot_row(unsigned kmax) { return 255 - (int)(kmax & 255u); }
 
 // Zero with the sign of v.
@@ -209,12 +217,10 @@ __device__ __forceinline__ void panel_factor_atmosphere(int nz, int n, int ld, c
     for (int c2 = 0; c2 < CPWP; ++c2) prow[c2] = R(0);
 #pragma unroll 1
     for (int s = 0; s < cnt; ++s) {
-      unsigned kr[RPL], km = 0u;
+      unsigned kr[RPL];
 #pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        kr[r] = (pivot_mag(t[r]) & msk[r]) | cc[r];
-        km = max(km, kr[r]);
-      }
+      for (int r = 0; r < RPL; ++r) kr[r] = (pivot_mag(t[r]) & msk[r]) | cc[r];
+      const unsigned km = key_max(kr);
       const unsigned kx = __reduce_max_sync(FULL, km);
       R vb = t[0];   // this lane's candidate
 #pragma unroll
@@ -654,12 +660,10 @@ __device__ __forceinline__ void dmma_factor_atmosphere(int nz, int n, int ld, co
     double lv = 0.0;
 #pragma unroll 1
     for (int s = 0; s < cnt; ++s) {
-      unsigned kr[RPL], km = 0u;
+      unsigned kr[RPL];
 #pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        kr[r] = (pivot_mag(XR(r, 0)) & msk[r]) | cc[r];
-        km = max(km, kr[r]);
-      }
+      for (int r = 0; r < RPL; ++r) kr[r] = (pivot_mag(XR(r, 0)) & msk[r]) | cc[r];
+      const unsigned km = key_max(kr);
       const unsigned kx = __reduce_max_sync(FULL, km);
       double vb = XR(0, 0);   // this lane's candidate
 #pragma unroll
