@@ -244,12 +244,23 @@ def oracle_check(net, cases, sol, delta, status, k1, k2, samples):
             "stage_backward_error_max": bwd, "schur_block_cond_max": conds}
 
 
-def launches_per_step(torch, tuned, B, nz):
-    """Launches of the package's kernels in one batched FP64 step."""
-    parts = 2 if tuned.get("streams") == 2 else 1
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    one_kernel = tuned.get("stage1_layers") == 2 or (B // parts) * -(-nz // 8) >= 2 * sms
-    return parts * (8 if one_kernel else 9)
+def kernel_launches(torch, fn):
+    """Kernel launches of one fn() on the current stream's device, counted in a
+    capture of it (a captured step holds the package's kernels and memory sets)."""
+    from cuda.bindings import runtime as rt
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        fn()
+    handle = rt.cudaGraph_t(init_value=graph.raw_cuda_graph())
+
+    def ok(res):
+        if res[0] != rt.cudaError_t.cudaSuccess:
+            raise RuntimeError(f"graph query: {res[0]}")
+        return res[1:]
+
+    n = ok(rt.cudaGraphGetNodes(handle))[-1]
+    nodes = ok(rt.cudaGraphGetNodes(handle, n))[0]
+    return sum(ok(rt.cudaGraphNodeGetType(v))[0] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for v in nodes)
 
 
 def fp64_peak_tflops(lib, torch, stream):
@@ -319,7 +330,7 @@ def run_config2(args, torch):
                        "groups": len(batch.groups), "l2": "inputs larger than L2, no flush"},
             "sequential_single_instance": {"value": n / (seq_ms * 1e-3), "unit": UNIT, "ms_per_pass": seq_ms},
             "speedup_vs_sequential": seq_ms / ms, "gpu_launches": args.steps * sum(
-                launches_per_step(torch, {}, len(g["idx"]), max(items[i][2].shape[0] for i in g["idx"]))
+                kernel_launches(torch, lambda g=g: g["step"](g["y"], g["k"], g["dt"], out=(g["sol"], g["delta"])))
                 for g in batch.groups),
             "tuning": {k: {"tuning": v["tuning"], "ms": v["ms"], "candidates_ms": v["candidates"]}
                        for k, v in batch.tuned.items()},
@@ -732,6 +743,7 @@ def main():
     # the measured region
     at = pkg("autotune")
     tuned, tune_ms = at.tune_group(dict(step=step, y=y, k=k, dt=dt, sol=sol, delta=delta), reps=3, split=True)
+    launches = kernel_launches(torch, one)
     for _ in range(args.warmup):
         one()
     torch.cuda.synchronize()
@@ -767,7 +779,7 @@ def main():
 
     # the two FP64 factor kernels on the same batch (per-launch event split)
     variants = {}
-    for vid, vname in ((2, "scalar_gauss_jordan"), (3, "pipelined_gauss_jordan"), (4, "paired_gauss_jordan"),
+    for vid, vname in ((2, "panel_gauss_jordan"), (3, "pipelined_gauss_jordan"), (4, "paired_gauss_jordan"),
                        (1, "blocked_dmma")):
         at.set_tuning(dn, dict(tuned, streams=1, factor_kernel=vid))
         for _ in range(args.warmup):
@@ -952,7 +964,7 @@ def main():
             # per step: diffusion rows, stage 1, factor, back sweep, diffusion rows,
             # stage 2 (one kernel by tiles of eight layers; rates and sums in batches
             # too small for tiles), forward sweep, back sweep (twice with two streams)
-            "gpu_launches": launches_per_step(torch, tuned, B, Y.shape[1]) * args.steps,
+            "gpu_launches": launches * args.steps,
             "roofline": {"bound": "fp64", "kernel": "factor (Gauss-Jordan inverse with threshold partial pivoting of "
                                                     "each layer block, serial in z, one CTA per atmosphere)",
                          "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
@@ -970,9 +982,9 @@ def main():
             "factor_variants": dict(variants, note="blocked_dmma: one warp per 8-column panel, "
                                                    "pivot steps inside the warp, rank-8 trailing updates on "
                                                    "the FP64 tensor cores (mma.sync m8n8k4); "
-                                                   "scalar_gauss_jordan (default): by panels of eight "
+                                                   "panel_gauss_jordan (default): by panels of eight "
                                                    "columns, one block barrier per panel, the same "
-                                                   "multiply-adds as the scalar elimination, on the "
+                                                   "multiply-adds as a scalar elimination, on the "
                                                    "FP64 tensor cores"),
             "single_instance_fp64": {"value": 1.0 / (single_ms * 1e-3), "unit": UNIT, "ms_per_step": single_ms},
             "status_ok": check["status_ok"],
