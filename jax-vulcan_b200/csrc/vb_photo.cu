@@ -789,7 +789,7 @@ template <int PB>
 static cudaError_t launch_flux_tiles(int batch, int nz, int ni, const VbPhoto& P, const double* tau,
                                      const double* ymix, const double* du_prev, double* aflux, double* sflux,
                                      double* dd, double* du, const int32_t* due, double flux_atol, double* achg,
-                                     cudaStream_t st) {
+                                     int sms, cudaStream_t st) {
   const size_t sm = flux_smem_bytes<PB>(P, nz);
   const dim3 grid((P.nbin + PB - 1) / PB, batch);
   auto launch = [&](auto kern, int threads) {
@@ -798,7 +798,7 @@ static cudaError_t launch_flux_tiles(int batch, int nz, int ni, const VbPhoto& P
     kern<<<grid, threads, sm, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg);
     return cudaGetLastError();
   };
-  switch (tile_threads(sm, (int64_t)grid.x * batch, sm_count(), FLUX_THREADS)) {
+  switch (tile_threads(sm, (int64_t)grid.x * batch, sms, FLUX_THREADS)) {
     case 128: return launch(flux_kernel<PB, 128>, 128);
     case 256: return launch(flux_kernel<PB, 256>, 256);
     default: return launch(flux_kernel<PB, 512>, 512);
@@ -808,15 +808,15 @@ static cudaError_t launch_flux_tiles(int batch, int nz, int ni, const VbPhoto& P
 cudaError_t launch_photo_flux(int batch, int nz, int ni, const VbPhoto& P, const double* tau, const double* ymix,
                               const double* du_prev, double* aflux, double* sflux, double* dd, double* du,
                               const int32_t* due, double flux_atol, double* achg, cudaStream_t st) {
-  const int species = P.n_abs + P.n_abs_T + P.n_scat;
+  const int species = P.n_abs + P.n_abs_T + P.n_scat, sms = sm_count();
   // 32 bins up to 120 layers or so, 16 up to 240
-  if (!short_columns(nz, (int64_t)((P.nbin + 31) / 32) * batch, sm_count(), true)) {
+  if (!short_columns(nz, (int64_t)((P.nbin + 31) / 32) * batch, sms, true)) {
     if (species <= FLUX_MAX_SPECIES<32> && flux_smem_bytes<32>(P, nz) <= PHOTO_SMEM_MAX)
       return launch_flux_tiles<32>(batch, nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg,
-                                   st);
+                                   sms, st);
     if (species <= FLUX_MAX_SPECIES<16> && flux_smem_bytes<16>(P, nz) <= PHOTO_SMEM_MAX)
       return launch_flux_tiles<16>(batch, nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due, flux_atol, achg,
-                                   st);
+                                   sms, st);
   }
   dim3 grid((P.nbin + PHOTO_THREADS - 1) / PHOTO_THREADS, batch);
   flux_column_kernel<<<grid, PHOTO_THREADS, 0, st>>>(nz, ni, P, tau, ymix, du_prev, aflux, sflux, dd, du, due,
