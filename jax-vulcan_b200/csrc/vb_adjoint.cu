@@ -306,9 +306,11 @@ vjp_atm_species_kernel(Batch B, const double* __restrict__ y, const double* __re
     }
     out[o.ms + i] = -gms / (NAVO * KB);
     out[o.alpha + i] = -gal;
-    out[o.top + i] = (flags & VB_USE_TOPFLUX) ? -lb[(int64_t)(nz - 1) * ni + i] / a.dzi[nz - 2] : 0.0;
-    out[o.bot + i] = (flags & VB_USE_BOTFLUX) ? -lb[i] / a.dzi[0] : 0.0;
-    out[o.vdep + i] = (flags & VB_USE_BOTFLUX) ? lb[i] * yb[i] / a.dzi[0] : 0.0;
+    // (no boundary flux: 0 lambda, so that a lambda that is not finite shows here too)
+    const double lt = lb[(int64_t)(nz - 1) * ni + i], l0 = lb[i];
+    out[o.top + i] = (flags & VB_USE_TOPFLUX) ? -lt / a.dzi[nz - 2] : -(0.0 * lt);
+    out[o.bot + i] = (flags & VB_USE_BOTFLUX) ? -l0 / a.dzi[0] : -(0.0 * l0);
+    out[o.vdep + i] = (flags & VB_USE_BOTFLUX) ? l0 * yb[i] / a.dzi[0] : -(0.0 * l0);
   }
 }
 
