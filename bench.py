@@ -289,8 +289,9 @@ def run_config2(args, torch):
     nets, cases = syn.config2_batch(seed=2, batch=args.batch or 256)
     dev = {id(n): chem.to_device(n.tables) for n in nets.values()}
     items = [(dev[id(c.net)], jstep.atm_from_dict(c.atm), c.y, c.k, c.dt) for c in cases]
-    # launch shapes per network group chosen by the autotuner on this GPU (timed
-    # candidates: factor kernel, factor CTAs per SM, sweep ring depth)
+    # launch shapes per network group chosen by the autotuner on this GPU (the
+    # automatic shapes and timed candidates: factor kernel, factor CTAs per SM,
+    # sweep ring depth, layers per assembly CTA)
     batch = jstep.MultiNetworkBatch(items, tuning="tune")
     batch.capture()
     for _ in range(args.warmup):
@@ -777,7 +778,7 @@ def main():
     check = oracle_check(net, cases, sol, delta, step.status, *step.stages(), samples=(0, B - 1)) \
         if rank == 0 else None
 
-    # the two FP64 factor kernels on the same batch (per-launch event split)
+    # the FP64 factor kernels on the same batch (per-launch event split)
     variants = {}
     for vid, vname in ((2, "panel_gauss_jordan"), (3, "pipelined_gauss_jordan"), (4, "paired_gauss_jordan"),
                        (1, "blocked_dmma")):
@@ -930,8 +931,9 @@ def main():
     # algorithmic bytes of the factor: read each D_j, write each inverse (ni^2 doubles each)
     fac_bytes = B * nz * 2.0 * ni * ni * 8
     # DRAM read + write bytes of one factor launch measured by ncu, per atmosphere,
-    # scaled to the batch: 160 atmospheres, 775.3 MB read + 697.2 MB written
-    fac_traffic = (775.31e6 + 697.17e6) / 160 * B
+    # scaled to the batch: the panel factor, 160 atmospheres, 773.7 MB read +
+    # 694.7 MB written
+    fac_traffic = (773.72e6 + 694.66e6) / 160 * B
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -969,8 +971,8 @@ def main():
                                                     "each layer block, serial in z, one CTA per atmosphere)",
                          "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                          "frac": achieved / peak64 if peak64 else None, "traffic": fac_traffic,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one factor "
-                                           "launch of the same layout, per atmosphere, scaled to the batch",
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of "
+                                           "the panel factor, per atmosphere, scaled to the batch",
                          "peak_source": "measured live: FP64 FMA probe kernel (vb_fp64_probe); "
                                         "MEASURED_PEAKS.json has no FP64 figure",
                          "algorithmic": f"2*ni^3 flops per layer block x {nz} layers x {B} atmospheres",

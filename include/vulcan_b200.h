@@ -77,8 +77,9 @@ int vb_net_create(int ni, int nr, int max_terms,
 int vb_net_destroy(VbNet* net);
 /* Launch shapes of the steps run with a network (no counterpart in the
  * reference, whose XLA compiler picks its own): set by the project's
- * autotuner (jax-vulcan_b200/autotune.py), which times the candidates on the
- * device per network and batch; 0 in a field = the automatic choice.
+ * autotuner (jax-vulcan_b200/autotune.py), which times the automatic choice and
+ * the candidates on the device per network and batch; 0 in a field = the
+ * automatic choice.
  *   factor_kernel: 1 blocked Gauss-Jordan on the tensor cores, 2 Gauss-Jordan
  *                  by panels of eight columns, one block barrier per panel
  *                  (the default; FP64 trailing updates on the tensor cores),
@@ -89,7 +90,8 @@ int vb_net_destroy(VbNet* net);
  *   factor_ctas:   CTAs per SM of the factor, 1 or 2 (honoured for 65-72
  *                  species, the shape with both variants compiled)
  *   sweep_stages:  depth of the sweeps' bulk-copy ring, 1..3 (lowered when
- *                  the ring does not fit in shared memory)
+ *                  the ring does not fit in shared memory; 0: as deep as
+ *                  fits, up to eight)
  *   streams:       2 = vb_ros2_step runs the two halves of a uniform batch
  *                  on the caller's stream and a second stream of the
  *                  library's (created on first use, one per device; forked

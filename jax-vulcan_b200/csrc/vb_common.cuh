@@ -100,7 +100,7 @@ struct Batch {
   // launch shapes chosen by the network's tuning (VbTuning; 0 = automatic)
   int factor_kernel = 0;   // 1 blocked tensor-core, 2 by panels, 3 pipelined, 4 paired
   int factor_ctas = 0;     // CTAs per SM of the factor (1 or 2, where both fit)
-  int sweep_stages = 0;    // bulk-copy ring depth of the sweeps (1..3)
+  int sweep_stages = 0;    // bulk-copy ring depth of the sweeps (1..3; 0: as deep as fits)
   int stage1_layers = 0;   // layers per stage-1 CTA (1 or 2)
   // rate region of the layer-vectorized stage 2 (rates_region_doubles per
   // layer), or nullptr: the per-layer stage-2 kernel

@@ -556,8 +556,9 @@ struct DGJ {
 // instructions of one warp, issued in order), 370 beside the other warps of
 // the block, 600 with two blocks on the SM. Factor of nz=120, ni=69 (B200, ms,
 // one block barrier per step before, this kernel now): one atmosphere 3.07,
-// 2.10; 148 (one per SM) 3.21, 2.11; 296 (two per SM) 5.64, 3.65; ni=89,
-// nz=150, 128 atmospheres 6.03, 4.13; ni=30, nz=43, one 0.349, 0.242.
+// 2.12 (34.7K cycles a layer); 148 (one per SM) 3.21, 2.13; 296 (two per SM)
+// 5.64, 3.70; ni=89, nz=150, 128 atmospheres 6.03, 4.12; ni=30, nz=43, one 0.349,
+// 0.242.
 // WIDE: registers for both halves of a panel's update at once (one block on the
 // SM).
 template <int NT, bool DPF, bool WIDE>

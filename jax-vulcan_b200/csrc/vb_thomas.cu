@@ -863,9 +863,11 @@ gj_pair_kernel(Batch B, double* __restrict__ ws, int32_t* __restrict__ status, i
   gj_factor_pair<RPL, CPW, NW>(B.nz, B.ni, B.ld, P, tr != 0, smem_raw, wlim);
 }
 
-// out == nullptr: the inverses replace the blocks in the workspace (FP64
-// path); otherwise they go to out (layer-major, ni x ld per layer) and the
-// FP64 blocks stay. only != nullptr: atmospheres with only[b] == 0 are skipped.
+// The factor kernels. out == nullptr: the inverses replace the blocks in the
+// workspace (FP64 path); otherwise they go to out (layer-major, ni x ld per
+// layer) and the FP64 blocks stay. only != nullptr: atmospheres with only[b] ==
+// 0 are skipped.
+
 // FP64, panels of 8 columns with DMMA trailing updates (one warp per panel).
 template <int NT, int MB, bool DPF>
 __global__ void __launch_bounds__(NT * 32, MB)
@@ -1695,8 +1697,6 @@ cudaError_t launch_factor32(const Batch& B, double* ws, void* mxr, int32_t* stat
   return launch_bgj32_t<16, 16, 1, false>(B, ws, mxr, status32, st);
 }
 
-
-
 template <int NT, int MB, bool DPF>
 static cudaError_t launch_dgj_t(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
                                 double* out, const int32_t* only) {
@@ -1709,9 +1709,13 @@ static cudaError_t launch_dgj_t(const Batch& B, double* ws, int32_t* status, int
 }
 
 // The FP64 Gauss-Jordan factor: one warp per panel of 8 columns, the smallest
-// instantiated count that holds ni. Up to 72 species two CTAs share an SM when
+// instantiated count that holds ni. A block runs ceil(ni / 8) panels whatever the
+// count, its spare warps only meet the barriers (factor and two solves of 32
+// atmospheres of 30 layers, ms: 40 species 0.36, 41 0.39, 48 0.43, all with six
+// warps; 88 1.01, 96 1.13 with twelve). Up to 72 species two CTAs share an SM when
 // the batch has more atmospheres than SMs (registers capped for it), else one
-// (no cap); larger blocks leave shared memory for one.
+// (no cap); larger blocks leave shared memory for one, and above 96 species not
+// for the prefetched block (97 species 1.87).
 static cudaError_t launch_dgj(const Batch& B, double* ws, int32_t* status, int with_rhs, int tr, cudaStream_t st,
                               double* out, const int32_t* only) {
   if (B.ni <= 24) return launch_dgj_t<3, 4, true>(B, ws, status, with_rhs, tr, st, out, only);

@@ -101,9 +101,10 @@ class Ros2Step:
     def __init__(self, net: NetworkArrays, atm: AtmStatic, batch: int | None = None, mixed: bool = False,
                  max_refine: int = 3, tol: float = 1e-12, assembly: bool = True):
         """``mixed=True``: the mixed-precision step (``vb_ros2_step_mixed``:
-        FP32 row-equilibrated factor, FP64 refinement
-        of both stages, at most ``max_refine`` passes to ``tol``, FP64
-        fallback); ``self.passes`` then holds the passes run per atmosphere.
+        FP32 row-equilibrated factor, FP64 refinement of both stages, at most
+        ``max_refine`` passes to ``tol``, FP64 fallback); ``self.passes`` then
+        holds the passes run per atmosphere. On B200 it is slower than the FP64
+        step: both factors are bound by the same chain of pivot steps.
         ``assembly``: allocate the rate region of the layer-vectorized
         stage 2 (``vb_ros2_assembly_bytes``: nr+1 doubles per layer, none where
         the batch goes by tiles of eight layers per CTA), so the stage-2
